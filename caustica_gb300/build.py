@@ -26,7 +26,7 @@ ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 # the size-specialised passes are split into several units per family (one
 # length group each) so the parallel build finishes in about a minute
 SOURCES = (["cg_kspace.cu", "cg_pennes.cu", "cg_post.cu", "cg_store.cu", "cg_fused_xy.cu", "cg_fast_yx.cu", "cg_fast_z.cu"]
-           + [f"cg_fast_yx_{g}.cu" for g in "abcdef"] + [f"cg_fast_z_{g}.cu" for g in "abcdef"])
+           + [f"cg_fast_yx_{g}.cu" for g in "abcdefghijklmn"] + [f"cg_fast_z_{g}.cu" for g in "abcdefghijklmnopqr"])
 
 
 def nvcc() -> str:
@@ -43,7 +43,7 @@ def _flags(verbose_ptxas: bool = False) -> list[str]:
          f"-I{INCLUDE}", f"-I{CSRC}", "--expt-relaxed-constexpr"]
     if verbose_ptxas:
         f.append("-Xptxas=-v")
-    for var in ("CG_FAST_MINB_Y", "CG_FAST_MINB_X", "CG_FAST_MINB_XG", "CG_FAST_MINB_X20", "CG_FAST_MINB_Z", "CG_YP", "CG_YP20", "CG_XP", "CG_ZP"):
+    for var in ("CG_FAST_MINB_Y", "CG_FAST_MINB_X", "CG_FAST_MINB_XG", "CG_FAST_MINB_X20", "CG_FAST_MINB_Y20", "CG_FAST_MINB_Z", "CG_YP", "CG_YP20", "CG_XP", "CG_XP20"):
         if os.environ.get(var):
             f.append(f"-D{var}={int(os.environ[var])}")
     return f

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 #include <stdio.h>
 
@@ -36,10 +37,32 @@ void cg_set_error(const char* fmt, ...);
 // ---------------------------------------------------------------- complex --
 __host__ __device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __host__ __device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__host__ __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// Products and fused products whose rounding does not depend on the code
+// around them: the compiler may fuse a plain product into a neighbouring sum
+// in one kernel and not in another, and the transforms of different kernels
+// have to agree bit for bit (staging variants, restored states).
+__host__ __device__ __forceinline__ float f_mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
 }
-__host__ __device__ __forceinline__ float2 c_scale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+__host__ __device__ __forceinline__ float f_fma(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  return __fmaf_rn(a, b, c);
+#else
+  return fmaf(a, b, c);
+#endif
+}
+__host__ __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
+  return make_float2(f_fma(a.x, b.x, -f_mul(a.y, b.y)), f_fma(a.x, b.y, f_mul(a.y, b.x)));
+}
+__host__ __device__ __forceinline__ float2 c_scale(float2 a, float s) { return make_float2(f_mul(a.x, s), f_mul(a.y, s)); }
+// a s + b
+__host__ __device__ __forceinline__ float2 c_fma(float2 a, float s, float2 b) {
+  return make_float2(f_fma(a.x, s, b.x), f_fma(a.y, s, b.y));
+}
 __host__ __device__ __forceinline__ float2 c_conj(float2 a) { return make_float2(a.x, -a.y); }
 // i * a
 __host__ __device__ __forceinline__ float2 c_muli(float2 a) { return make_float2(-a.y, a.x); }

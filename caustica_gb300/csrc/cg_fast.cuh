@@ -17,8 +17,6 @@
 // Taylor series of sin and cos (double precision, rounded once to float).
 #pragma once
 
-#include <stdlib.h>
-
 #include <type_traits>
 #include <utility>
 
@@ -89,7 +87,7 @@ __host__ __device__ __forceinline__ float2 twiddle_ct(float2 v) {
   if constexpr (cf == -1.0f && sf == 0.0f) return make_float2(-v.x, -v.y);
   if constexpr (cf == 0.0f && sf == 1.0f) return make_float2(-v.y, v.x);
   if constexpr (cf == 0.0f && sf == -1.0f) return make_float2(v.y, -v.x);
-  return make_float2(v.x * cf - v.y * sf, v.x * sf + v.y * cf);
+  return make_float2(f_fma(v.x, cf, -f_mul(v.y, sf)), f_fma(v.x, sf, f_mul(v.y, cf)));
 }
 
 template <bool INV>
@@ -148,11 +146,11 @@ struct Dft<3, INV> {
     const float h = 0.86602540378443864676f;
     float2 t = c_add(v[1], v[2]);
     float2 d = c_sub(v[1], v[2]);
-    float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
-    float2 r = rot<INV>(c_scale(d, h));
+    float2 m = c_fma(t, -0.5f, v[0]);
+    float2 r = rot<INV>(d);
     v[0] = c_add(v[0], t);
-    v[1] = c_add(m, r);
-    v[2] = c_sub(m, r);
+    v[1] = c_fma(r, h, m);
+    v[2] = c_fma(r, -h, m);
   }
 };
 
@@ -180,10 +178,10 @@ struct Dft<5, INV> {
     float2 t3 = c_sub(v[1], v[4]);
     float2 t4 = c_sub(v[2], v[3]);
     float2 y0 = c_add(v[0], c_add(t1, t2));
-    float2 b1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    float2 b2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    float2 e1 = make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
-    float2 e2 = make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
+    float2 b1 = c_fma(t2, c2, c_fma(t1, c1, v[0]));
+    float2 b2 = c_fma(t2, c1, c_fma(t1, c2, v[0]));
+    float2 e1 = c_fma(t3, s1, c_scale(t4, s2));
+    float2 e2 = c_fma(t3, s2, c_scale(t4, -s1));
     float2 r1 = rot<INV>(e1);
     float2 r2 = rot<INV>(e2);
     v[0] = y0;
@@ -202,16 +200,18 @@ struct Dft<8, INV> {
     float2 o[4] = {v[1], v[3], v[5], v[7]};
     Dft<4, INV>::run(e);
     Dft<4, INV>::run(o);
-    o[1] = INV ? make_float2(r2 * (o[1].x - o[1].y), r2 * (o[1].x + o[1].y))
-               : make_float2(r2 * (o[1].x + o[1].y), r2 * (o[1].y - o[1].x));
+    // o[1] and o[3] without their factor r2, which the last sums apply
+    o[1] = INV ? make_float2(o[1].x - o[1].y, o[1].x + o[1].y) : make_float2(o[1].x + o[1].y, o[1].y - o[1].x);
     o[2] = rot<INV>(o[2]);
-    o[3] = INV ? make_float2(-r2 * (o[3].x + o[3].y), r2 * (o[3].x - o[3].y))
-               : make_float2(r2 * (o[3].y - o[3].x), -r2 * (o[3].x + o[3].y));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = c_add(e[k], o[k]);
-      v[k + 4] = c_sub(e[k], o[k]);
-    }
+    o[3] = INV ? make_float2(-(o[3].x + o[3].y), o[3].x - o[3].y) : make_float2(o[3].y - o[3].x, -(o[3].x + o[3].y));
+    v[0] = c_add(e[0], o[0]);
+    v[4] = c_sub(e[0], o[0]);
+    v[1] = c_fma(o[1], r2, e[1]);
+    v[5] = c_fma(o[1], -r2, e[1]);
+    v[2] = c_add(e[2], o[2]);
+    v[6] = c_sub(e[2], o[2]);
+    v[3] = c_fma(o[3], r2, e[3]);
+    v[7] = c_fma(o[3], -r2, e[3]);
   }
 };
 
@@ -225,23 +225,31 @@ struct Split {
   static constexpr bool ok = (A <= 16);
 };
 
+// The most even split n = a b (a <= b) of a pencil; its smaller factor.
+constexpr int ct_even_split(int n) {
+  int best = 1;
+  for (int a = 1; a * a <= n; ++a)
+    if (n % a == 0) best = a;
+  return best;
+}
+
+// Threads per pencil for a split whose larger factor is m: 8 or 16 (whole
+// pencils per warp), else m rounded up to 4 so that 8 pencils fill whole warps.
+constexpr int ct_tpp(int m) { return m <= 8 ? 8 : (m <= 16 ? 16 : (m + 3) / 4 * 4); }
+
 // Pencil split of the size-specialised passes: (A, B) with B threads
 // holding A values on input and A threads holding B values on output.
-// Lengths 16 x (<= 16) use Split<N> on 16 threads per pencil; 320 = 16 x 20
-// and 400 = 20 x 20 run on 20 threads per pencil, 512 = 32 x 16 (Split<512>)
-// and 640 = 32 x 20 on 32.
+// 16 x (<= 16) where the length allows it (aligned 16-value runs in global
+// memory), else the most even split: no thread holds more than 20 values up
+// to 400 points except on 243, 250, 375 and 384 (27, 25, 25, 24).
 template <int N>
 struct PSplit {
-  static constexpr int A = Split<N>::A, B = Split<N>::B;
-  static constexpr int TPP = A > B ? A : B;  // threads per pencil
+  static constexpr int A = N % 16 == 0 && N / 16 <= 16 ? N / 16 : ct_even_split(N), B = N / A;
+  static constexpr int TPP = ct_tpp(A > B ? A : B);  // threads per pencil
 };
 template <>
-struct PSplit<320> {
-  static constexpr int A = 16, B = 20, TPP = 20;
-};
-template <>
-struct PSplit<400> {
-  static constexpr int A = 20, B = 20, TPP = 20;
+struct PSplit<512> {
+  static constexpr int A = 32, B = 16, TPP = 32;
 };
 template <>
 struct PSplit<640> {
@@ -328,6 +336,14 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
@@ -379,17 +395,9 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const void* map, unsigned
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
-// Launch with programmatic stream serialisation (CG_PDL=0 turns it off).
-inline bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("CG_PDL");
-    on = (e && e[0] == '0') ? 0 : 1;
-  }
-  return on != 0;
-}
+// Launch, with programmatic stream serialisation when `pdl` is set.
 template <typename... KArgs, typename... Args>
-inline void launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline void launch(int pdl, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -397,7 +405,7 @@ inline void launch(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cuda
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, args...);
@@ -413,16 +421,6 @@ inline int sm_count() {
       n = 152;
   }
   return n;
-}
-
-// Persistent grid over `total` equal work items: about `per_sm` CTAs per SM,
-// each a contiguous run of *per_cta items, none empty.
-inline void persistent_grid(long long total, int per_sm, int* grid, int* per_cta) {
-  const long long slots = (long long)sm_count() * per_sm;
-  const long long g0 = total < slots ? total : slots;
-  const long long per = (total + g0 - 1) / g0;
-  *per_cta = (int)per;
-  *grid = (int)((total + per - 1) / per);
 }
 
 }  // namespace cgf

@@ -4,10 +4,10 @@
 // and dispatched by cg_fast_yx.cu.
 //
 // y-pass: rows (x, kz) of length ny, YP rows per CTA; thread (p, s) =
-// (threadIdx / TPP, threadIdx % TPP) owns row p (TPP = threads per pencil:
-// 16, or 20 / 32 for the 320/400 and 512/640 splits). x-pass: CG_XP
-// consecutive (kz, y) columns per CTA; thread (c, s) = (threadIdx % CG_XP,
-// threadIdx / CG_XP) owns column c. Pencil data moves global -> registers -> one exchange per
+// (threadIdx / TPP, threadIdx % TPP) owns row p (TPP = threads per pencil: 8
+// or 16, or 20..32 for the longer splits). x-pass: XP
+// consecutive (kz, y) columns per CTA; thread (c, s) = (threadIdx % XP,
+// threadIdx / XP) owns column c. Pencil data moves global -> registers -> one exchange per
 // transform -> registers -> global (cg_fast.cuh).
 #pragma once
 
@@ -28,11 +28,15 @@
 #ifndef CG_FAST_MINB_XG
 #define CG_FAST_MINB_XG CG_FAST_MINB_X
 #endif
-// and for those modes on the 320-point x axis (20-thread pencils: two CTAs
-// per SM measured 1408 -> 1365 us per 320^3 step; the 400-point axis keeps
-// one, two measured 2464 -> 2675 us per 400^3 step)
+// and of the longer splits (20 and more threads per pencil)
 #ifndef CG_FAST_MINB_X20
-#define CG_FAST_MINB_X20 2
+#define CG_FAST_MINB_X20 3
+#endif
+#ifndef CG_FAST_MINB_Y20
+#define CG_FAST_MINB_Y20 5
+#endif
+#ifndef CG_XP20
+#define CG_XP20 8
 #endif
 // rows per y-CTA and columns per x-CTA (16 threads each)
 #ifndef CG_YP20
@@ -51,21 +55,21 @@ using cgf::RowEx;
 using cgf::fft2;
 using cgf::static_for;
 
-// Threads and resident CTAs per SM of the y- and x-pass CTAs for length N
-// (20-thread pencils get the register budget that avoids spills).
+// Threads and resident CTAs per SM of the y- and x-pass CTAs for length N.
+// Splits with more than 16 threads a pencil take 8 columns per x-CTA, three
+// CTAs to an SM (16 columns, one or two CTAs: 400^3 X_GRAD / X_DIV 353 / 342
+// against 309 / 290 us, 320^3 139 / 198 against 161 / 158).
 template <int N>
 struct YT {
-  static constexpr int TPP = PSplit<N>::TPP, YP = TPP == 20 ? CG_YP20 : CG_YP, THREADS = TPP * YP;
-  static constexpr int MINB = TPP == 16 ? CG_FAST_MINB_Y : 4;
+  static constexpr int TPP = PSplit<N>::TPP, YP = TPP < 16 ? 2 * CG_YP : (TPP > 16 && TPP < 32 ? CG_YP20 : CG_YP);
+  static constexpr int THREADS = TPP * YP;
+  static constexpr int MINB = TPP <= 16 ? CG_FAST_MINB_Y : (TPP < 28 ? CG_FAST_MINB_Y20 : 4);
 };
 template <int N>
 struct XT {
-  static constexpr int TPP = PSplit<N>::TPP, THREADS = TPP * CG_XP;
-  static constexpr int MINB = TPP == 16 ? CG_FAST_MINB_X : 1;
-  // 320-point axis: CG_FAST_MINB_X20 CTAs per SM except for X_DIV (its
-  // parked tile needs the registers of one)
+  static constexpr int TPP = PSplit<N>::TPP, XP = TPP > 16 ? CG_XP20 : CG_XP, THREADS = TPP * XP;
   static constexpr int minb(int mode) {
-    return TPP == 16 ? (mode != X_DIV ? CG_FAST_MINB_XG : MINB) : (N == 320 && mode != X_DIV ? CG_FAST_MINB_X20 : MINB);
+    return TPP <= 16 ? 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X) : (TPP < 28 ? CG_FAST_MINB_X20 : 2);
   }
 };
 
@@ -149,31 +153,31 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
                                                                         float2* __restrict__ S0,
                                                                         float2* __restrict__ S1,
                                                                         float2* __restrict__ S2) {
-  constexpr int A = PSplit<N>::A, B = PSplit<N>::B;
+  constexpr int A = PSplit<N>::A, B = PSplit<N>::B, XP = XT<N>::XP;
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
   float2* tw = sm;       // (A, B) order
   float2* twi = sm + N;  // (B, A) order
   cgf::fill_twt<A, B>(tw, t.twx);
   cgf::fill_twt<B, A>(twi, t.twx);
-  float* kxs = reinterpret_cast<float*>(sm + 2 * N + 2 * N * CG_XP);  // k_x | k_x^2
+  float* kxs = reinterpret_cast<float*>(sm + 2 * N + 2 * N * XP);  // k_x | k_x^2
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     kxs[i] = t.kx[i];
     kxs[N + i] = t.kx2[i];
   }
   cgf::pdl_wait();
-  const int c = threadIdx.x % CG_XP, s = threadIdx.x / CG_XP;
-  const ColEx<A, B, CG_XP> exf{sm + 2 * N + c};
-  const ColEx<B, A, CG_XP> exi{sm + 2 * N + c};
+  const int c = threadIdx.x % XP, s = threadIdx.x / XP;
+  const ColEx<A, B, XP> exf{sm + 2 * N + c};
+  const ColEx<B, A, XP> exi{sm + 2 * N + c};
   const long long ncol = (long long)d.nzh * d.ny;
-  const long long col = (long long)blockIdx.x * CG_XP + c;
+  const long long col = (long long)blockIdx.x * XP + c;
   const bool valid = col < ncol;
   const long long base = (long long)blockIdx.y * d.nspec + col;
   float kyz2 = 0.f;
   {
-    const long long cc = valid ? col : ncol - 1;
-    const int kz = (int)(cc / d.ny);
-    const int ky = (int)(cc - (long long)kz * d.ny);
+    const unsigned cc = (unsigned)(valid ? col : ncol - 1);  // below 2^21: 32-bit division
+    const int kz = (int)(cc / (unsigned)d.ny);
+    const int ky = (int)(cc - (unsigned)kz * (unsigned)d.ny);
     kyz2 = t.ky2[ky] + t.kz2[kz];
   }
   __syncthreads();
@@ -202,39 +206,39 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
   } else if constexpr (MODE == X_GRAD) {
     // S2 <- IFFT(q); S1 <- IFFT(i kx q), q = kappa/N FFT(S0); q waits in shared
     // memory during the first inverse transform instead of in registers
-    float2* qs = sm + 2 * N + N * CG_XP;
+    float2* qs = sm + 2 * N + N * XP;
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
     static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int k = (s < A) ? s + A * b : 0;
       w[b] = c_scale(w[b], kappa(k));
-      if (s < A) qs[(s + A * b) * CG_XP + c] = w[b];
+      if (s < A) qs[(s + A * b) * XP + c] = w[b];
     });
     fft2<B, A, true>(w, z, s, twi, exi);
     store_z(S2);
     static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int k = (s < A) ? s + A * b : 0;
-      w[b] = (s < A) ? c_muli(c_scale(qs[(s + A * b) * CG_XP + c], kxs[k])) : make_float2(0.f, 0.f);
+      w[b] = (s < A) ? c_muli(c_scale(qs[(s + A * b) * XP + c], kxs[k])) : make_float2(0.f, 0.f);
     });
     fft2<B, A, true>(w, z, s, twi, exi);
     store_z(S1);
   } else {
     // X_DIV: S0 <- IFFT(kappa/N (FFT(S0) + i kx FFT(S1))); FFT(S1) waits in shared memory
-    float2* hs = sm + 2 * N + N * CG_XP;
+    float2* hs = sm + 2 * N + N * XP;
     load(S1);
     fft2<A, B, false>(v, w, s, tw, exf);
     if (s < A) static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      hs[(s + A * b) * CG_XP + c] = w[b];
+      hs[(s + A * b) * XP + c] = w[b];
     });
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
     static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int k = (s < A) ? s + A * b : 0;
-      const float2 h = (s < A) ? hs[(s + A * b) * CG_XP + c] : make_float2(0.f, 0.f);
+      const float2 h = (s < A) ? hs[(s + A * b) * XP + c] : make_float2(0.f, 0.f);
       w[b] = c_scale(c_add(w[b], c_muli(c_scale(h, kxs[k]))), kappa(k));
     });
     fft2<B, A, true>(w, z, s, twi, exi);
@@ -249,20 +253,27 @@ static size_t smem_y() {
 }
 template <int N>
 static size_t smem_x() {
-  return sizeof(float2) * (2 * N + 2 * (size_t)N * CG_XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
+  return sizeof(float2) * (2 * N + 2 * (size_t)N * XT<N>::XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
 }
 
 // ------------------------------------------------ per-length launchers --
+// Never a programmatic dependent launch: a y-pass that starts while CTAs of a
+// z- or x-pass are still resident runs on the shared-memory carve-out of that
+// pass, because an SM changes it only when empty, and the y-pass wants the L1
+// for its loads in flight. Per step with all passes / x and z only / none
+// launched programmatically: 64^3 41 / 33 / 42 us, 160x160x192 161 / 162 / 170,
+// 160x160x192 x 2 349 / 311 / 315, 240^3 480 / 438 / 446, 256x256x320
+// 727 / 671 / 675.
 template <int N>
 bool yx_launch_y(int mode, const Dims& d, const Tables& t, float2* S0, float2* S1, float2* S2, int batch,
                  cudaStream_t st) {
   const dim3 grid((unsigned)((d.nx * (long long)d.nzh + YT<N>::YP - 1) / YT<N>::YP), batch);
   const dim3 block(YT<N>::THREADS);
   switch (mode) {
-    case Y_FWD: cgf::launch(kf_ypass<N, Y_FWD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    case Y_INV: cgf::launch(kf_ypass<N, Y_INV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    case Y_INV_GRAD: cgf::launch(kf_ypass<N, Y_INV_GRAD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    default: cgf::launch(kf_ypass<N, Y_FWD_DIV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_FWD: cgf::launch(0, kf_ypass<N, Y_FWD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_INV: cgf::launch(0, kf_ypass<N, Y_INV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_INV_GRAD: cgf::launch(0, kf_ypass<N, Y_INV_GRAD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    default: cgf::launch(0, kf_ypass<N, Y_FWD_DIV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
   }
   return true;
 }
@@ -270,13 +281,13 @@ bool yx_launch_y(int mode, const Dims& d, const Tables& t, float2* S0, float2* S
 template <int N>
 bool yx_launch_x(int mode, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1,
                  float2* S2, int batch, cudaStream_t st) {
-  const dim3 grid((unsigned)(((long long)d.nzh * d.ny + CG_XP - 1) / CG_XP), batch);
+  const dim3 grid((unsigned)(((long long)d.nzh * d.ny + XT<N>::XP - 1) / XT<N>::XP), batch);
   const dim3 block(XT<N>::THREADS);
   switch (mode) {
-    case X_GRAD: cgf::launch(kf_xpass<N, X_GRAD>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
-    case X_DIV: cgf::launch(kf_xpass<N, X_DIV>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
-    case X_FWD: cgf::launch(kf_xpass<N, X_FWD>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
-    default: cgf::launch(kf_xpass<N, X_INV>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
+    case X_GRAD: cgf::launch(d.pdl, kf_xpass<N, X_GRAD>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
+    case X_DIV: cgf::launch(d.pdl, kf_xpass<N, X_DIV>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
+    case X_FWD: cgf::launch(d.pdl, kf_xpass<N, X_FWD>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
+    default: cgf::launch(d.pdl, kf_xpass<N, X_INV>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
   }
   return true;
 }

@@ -15,8 +15,8 @@ void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDe
               const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
               const ZTma* ztma);
 template <int N>
-void zp_run_fwd(const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
-                cudaStream_t st);
+void zp_run_half(bool inverse, const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
+                 cudaStream_t st);
 template <int N>
 int zp_prepare();
 template <int N>
@@ -30,7 +30,7 @@ int zt_prepare();
 
 bool fast_zpass_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
                   int batch, cudaStream_t st, bool persistent) {
-  if ((persistent || !fast_has(d.nz)) && d.ny % 2 == 0) {
+  if (persistent || !fast_has(d.nz)) {
     switch (d.nz) {
 #define CASE(n)                                          \
   case n:                                                \
@@ -54,10 +54,10 @@ bool fast_zpass_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, 
   }
 }
 
-bool fast_zpass_p(int mode, const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src,
-                  const RecordDev& rec, const long long* ctl, int n_local, int record, float* p, float2* S0,
-                  int batch, cudaStream_t st, bool persistent) {
-  if (mode == 1 && (persistent || !fast_has(d.nz)) && d.ny % 2 == 0) {
+bool fast_zpass_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
+                  const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
+                  bool persistent) {
+  if (persistent || !fast_has(d.nz)) {
     switch (d.nz) {
 #define CASE(n)                                                                   \
   case n:                                                                         \
@@ -70,9 +70,9 @@ bool fast_zpass_p(int mode, const Dims& d, const Tables& t, const MediumDev& m, 
     }
   }
   switch (d.nz) {
-#define CASE(n)                                                                         \
-  case n:                                                                               \
-    zt_run_p<n>(mode, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, st);      \
+#define CASE(n)                                                                      \
+  case n:                                                                            \
+    zt_run_p<n>(1, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, st);      \
     return true;
     CG_FAST_SIZES(CASE)
 #undef CASE
@@ -81,27 +81,39 @@ bool fast_zpass_p(int mode, const Dims& d, const Tables& t, const MediumDev& m, 
   }
 }
 
+bool fast_zpass_half(bool inverse, const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0,
+                     int batch, cudaStream_t st) {
+  switch (d.nz) {
+#define CASE(n)                                              \
+  case n:                                                    \
+    zp_run_half<n>(inverse, d, t, m, p, S0, batch, st);      \
+    return true;
+    CG_FAST_ZSIZES(CASE)
+#undef CASE
+    default:
+      return false;
+  }
+}
+
 bool fast_zpass_fwd_step(const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
                          cudaStream_t st, bool persistent) {
-  // the kernel family the step's p-pass runs on this grid (fast_zpass_p, mode 1)
-  if ((persistent || !fast_has(d.nz)) && d.ny % 2 == 0) {
-    switch (d.nz) {
-#define CASE(n)                                      \
-  case n:                                            \
-    zp_run_fwd<n>(d, t, m, p, S0, batch, st);        \
-    return true;
-      CG_FAST_ZSIZES(CASE)
-#undef CASE
-      default:
-        return false;
-    }
-  }
+  // the kernel family the step's p-pass runs on this grid (fast_zpass_p)
+  if (persistent || !fast_has(d.nz)) return fast_zpass_half(false, d, t, m, p, S0, batch, st);
   SourceDev src;
   memset(&src, 0, sizeof(src));
   RecordDev rec;
   memset(&rec, 0, sizeof(rec));
   rec.spp = 1;
-  return fast_zpass_p(0, d, t, m, src, rec, nullptr, 0, 0, p, S0, batch, st, false);
+  switch (d.nz) {
+#define CASE(n)                                                             \
+  case n:                                                                   \
+    zt_run_p<n>(0, d, t, m, src, rec, nullptr, 0, 0, p, S0, batch, st);      \
+    return true;
+    CG_FAST_SIZES(CASE)
+#undef CASE
+    default:
+      return false;
+  }
 }
 
 // ------------------------------------------------ tensor-map staging --

@@ -3,9 +3,10 @@
 // units (a few lengths each, so they compile in parallel) and dispatched by
 // cg_fast_z.cu.
 //
-// Tile = (batch member, x, 32 consecutive y). Real rows y0+2p and y0+2p+1
-// form complex pencil p (p = threadIdx / TPP, TPP = threads per pencil: 16,
-// or 20 / 32 for the 320/400 and 512/640 splits); s = threadIdx % TPP runs
+// Tile = (batch member, x, a run of consecutive y: 32, or 16 where that lets
+// more CTAs share an SM). Real rows y0+2p and y0+2p+1
+// form complex pencil p (p = threadIdx / TPP, TPP = threads per pencil: 8 or
+// 16, or 20..32 for the longer splits); s = threadIdx % TPP runs
 // along the pencil. The inverse (complex-to-real) transform is an (A, B) fft2, the
 // forward one a (B, A) fft2, so the values produced by the inverse arrive in
 // exactly the registers the forward transform reads; the pointwise update
@@ -26,16 +27,21 @@
 #define CG_FAST_MINB CG_FAST_MINB_Z
 
 using cgf::RowEx;
-using cgf::Split;
 using cgf::fft2;
 using cgf::static_for;
 
+// The pencil split with the larger factor first: after the inverse (A, B)
+// transform A threads hold B cells each at n = s + A b, so the pointwise
+// update runs on more lanes and every row access is a run of A floats.
 template <int N>
-using ZSplit = cgf::PSplit<N>;
+struct ZSplit {
+  using P = cgf::PSplit<N>;
+  static constexpr int A = P::A > P::B ? P::A : P::B, B = P::A > P::B ? P::B : P::A, TPP = P::TPP;
+};
 
 template <int N>
 struct ZShape {
-  static constexpr int A = Split<N>::A, B = Split<N>::B, NH = N / 2 + 1;
+  static constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, NH = N / 2 + 1;
   static constexpr int EX_I = RowEx<A, B>::SLAB, EX_F = RowEx<B, A>::SLAB;
   static constexpr int EX = EX_I > EX_F ? EX_I : EX_F;
   static constexpr int STG = (NH * 34 > N * 17) ? NH * 34 : N * 17;  // float2 units
@@ -122,8 +128,8 @@ __device__ __forceinline__ bool z_stage_labels(uint8_t* lab_s, float4* tab_s, co
 // Phase-1 inputs of the inverse transform for thread (p, s): Z_n = A_n + i B_n
 // with the Hermitian extension above N/2, n = s + B a.
 template <int N>
-__device__ __forceinline__ void z_inputs(float2 (&v)[Split<N>::A], const float4* stg4, int p, int s) {
-  constexpr int A = Split<N>::A, B = Split<N>::B;
+__device__ __forceinline__ void z_inputs(float2 (&v)[ZSplit<N>::A], const float4* stg4, int p, int s) {
+  constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B;
   static_for<0, A>([&](auto ai) {
     constexpr int a = decltype(ai)::value;
     const int n = s + B * a;
@@ -138,10 +144,20 @@ __device__ __forceinline__ void z_inputs(float2 (&v)[Split<N>::A], const float4*
   });
 }
 
+// Slot of bin k of pencil p in the split-store buffer: rows of P pencils,
+// permuted within the row so that 16 lanes holding consecutive k of one pencil
+// or consecutive slots touch all banks once.
+template <int P>
+__device__ __forceinline__ int xb_at(int k, int p) {
+  return k * P + (p ^ (P == 8 ? (k >> 1) & 7 : k & 15));
+}
+
 // After the forward transform thread (p, s < B) owns X[s + B a]; put them in
-// xb[k * 17 + p], then split each pencil into its two half spectra and store
-// them to S (x, k, y0 + 2p + {0, 1}), times i*mk[k] when given.
-template <int N>
+// the split-store buffer, then split each of the P pencils into its two half
+// spectra and store them to S (x, k, y0 + 2p + {0, 1}), times i*mk[k] when
+// given. CLOSE: a barrier after the last read of xb, for callers that write
+// it again before their own next barrier.
+template <int N, int P, bool CLOSE>
 __device__ __forceinline__ void z_split_store(float2* xb, const float2 (&X)[ZSplit<N>::A], float2* __restrict__ S,
                                               const Dims& d, int x, int y0, int p, int s, const float* mk) {
   constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, NH = N / 2 + 1;
@@ -150,17 +166,17 @@ __device__ __forceinline__ void z_split_store(float2* xb, const float2 (&X)[ZSpl
   __syncthreads();
   if (s < B) static_for<0, A>([&](auto ai) {
     constexpr int a = decltype(ai)::value;
-    xb[(s + B * a) * 17 + p] = X[a];
+    xb[xb_at<P>(s + B * a, p)] = X[a];
   });
   __syncthreads();
   float2* base = S + (long long)x * NH * d.ny + y0;
   const bool even_ny = (d.ny & 1) == 0;
-  for (int idx = threadIdx.x; idx < NH * CG_TILE; idx += blockDim.x) {
-    const int k = idx >> 4, pp = idx & 15;
+  for (int idx = threadIdx.x; idx < NH * P; idx += blockDim.x) {
+    const int k = idx / P, pp = idx % P;
     const int ya = y0 + 2 * pp;
     if (ya >= d.ny) continue;
-    const float2 zk = xb[k * 17 + pp];
-    const float2 zm = c_conj(xb[((N - k) % N) * 17 + pp]);
+    const float2 zk = xb[xb_at<P>(k, pp)];
+    const float2 zm = c_conj(xb[xb_at<P>(k ? N - k : 0, pp)]);
     float2 a = c_scale(c_add(zk, zm), 0.5f);
     float2 b = c_scale(c_mulmi(c_sub(zk, zm)), 0.5f);
     if (mk) {
@@ -175,7 +191,7 @@ __device__ __forceinline__ void z_split_store(float2* xb, const float2 (&X)[ZSpl
       if (ya + 1 < d.ny) q[1] = b;
     }
   }
-  __syncthreads();
+  if (CLOSE) __syncthreads();
 }
 
 template <int N>
@@ -256,11 +272,11 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_u(Dims d, T
     });
     float2 X[A];
     fft2<B, A, false>(w, X, s, twf, exf);
-    z_split_store<N>(xb, X, S, d, x, y0, p, s, mk);
+    z_split_store<N, CG_TILE, true>(xb, X, S, d, x, y0, p, s, mk);
   }
 }
 
-// MODE 0: forward transform of p only; 2: inverse only into p; 1: full update
+// MODE 0: forward transform of p only; 1: full update
 template <int N, int MODE>
 __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, Tables t, MediumDev m, SourceDev src,
                                                            RecordDev rec, const long long* ctl, int n_local,
@@ -302,7 +318,7 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
   } else {
     float4* tab_s = reinterpret_cast<float4*>(sm + Z::OFF_TAB);
     uint8_t* lab_s = reinterpret_cast<uint8_t*>(tab_s + 256);
-    const bool lab = (MODE == 1) && z_stage_labels<N>(lab_s, tab_s, m, d, x, y0);
+    const bool lab = z_stage_labels<N>(lab_s, tab_s, m, d, x, y0);
     const uint8_t* la = lab_s + (2 * p) * N;
     const uint8_t* lb = la + N;
     z_stage<N>(stg4, S, d, x, y0, nullptr);
@@ -311,22 +327,13 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
     static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int n = s + A * b;
-      pa[b] = (MODE == 1 && s < A && va) ? __ldg(pb + rowa + n) : 0.f;
-      pbv[b] = (MODE == 1 && s < A && vb) ? __ldg(pb + rowb + n) : 0.f;
+      pa[b] = (s < A && va) ? __ldg(pb + rowa + n) : 0.f;
+      pbv[b] = (s < A && vb) ? __ldg(pb + rowb + n) : 0.f;
     });
     __syncthreads();
     float2 v[A];
     z_inputs<N>(v, stg4, p, s);
     fft2<A, B, true>(v, w, s, tw, exi);
-    if constexpr (MODE == 2) {
-      if (s < A) static_for<0, B>([&](auto bi) {
-        constexpr int b = decltype(bi)::value;
-        const int n = s + A * b;
-        if (va) pb[rowa + n] = w[b].x;
-        if (vb) pb[rowb + n] = w[b].y;
-      });
-      return;
-    }
     const long long n_step = ctl[0] + n_local;
     const float spx = t.sx[x];
     const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
@@ -341,14 +348,14 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
         const float po = pa[b];
         float pn = m.nonlinear ? po - (cf.y + cf.w * po) * w[b].x : po - cf.y * w[b].x;
         pn = pn * cf.z;
-        r.x = pn * (spa * sz);
+        r.x = __fmul_rn(pn, spa * sz);  // rounded here: see the persistent p-pass
       }
       if (vb) {
         const float4 cf = lab ? tab_s[lb[n]] : cell_coef(m, rowb + n);
         const float po = pbv[b];
         float pn = m.nonlinear ? po - (cf.y + cf.w * po) * w[b].y : po - cf.y * w[b].y;
         pn = pn * cf.z;
-        r.y = pn * (spb * sz);
+        r.y = __fmul_rn(pn, spb * sz);
       }
       w[b] = r;
     });
@@ -414,94 +421,203 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
       if (per < rec.max_periods) atomicMax(&rec.peaks[(long long)b_idx * rec.max_periods + per], s_peak);
     }
   }
-  if constexpr (MODE != 2) {
-    float2 X[A];
-    fft2<B, A, false>(w, X, s, twf, exf);
-    z_split_store<N>(xb, X, S, d, x, y0, p, s, nullptr);
-  }
+  float2 X[A];
+  fft2<B, A, false>(w, X, s, twf, exf);
+  z_split_store<N, CG_TILE, false>(xb, X, S, d, x, y0, p, s, nullptr);
 }
 
 // ---------------------------------------------------------------------------
-// Persistent, pipelined z-passes (ny a multiple of the tile height). Each CTA
-// walks a contiguous run of tiles -- for the u-pass all three velocity
-// components of a tile in turn, so the tile's labels load once -- and the half
-// spectrum of the next (tile, component) streams into shared memory -- by two
-// tensor-map box copies on an mbarrier (TMA instantiations) or by 16-byte
-// cp.async from every thread -- while the current one is transformed. An
-// item's staging buffer is
-// then reused as its exchange and split-store buffer, so the two buffers cost
-// what the single-item kernel's staging plus exchange cost and two CTAs still
-// fit on an SM.
+// Persistent, pipelined z-passes. Each CTA walks every G-th item -- tiles in
+// the p-pass, (tile, velocity component) pairs in the u-pass -- and the half
+// spectrum and labels of the next item streams into shared memory -- by tensor-map box copies on an
+// mbarrier (TMA instantiations, ny even) or by cp.async from every thread --
+// while the current one is transformed. Both land in the same layout: boxes
+// of 8 pencils by NH k rows of 128 bytes, a pencil's 16 bytes (A_k, B_k) of
+// row k at chunk (p % 8) XOR (k % 8). An item's staging buffer is then reused
+// as its exchange and split-store buffer.
+//
+// Bound: latency (barriers, shared-memory round trips) below about 256^3,
+// HBM above. Resident warps, registers and the L1 that shared memory leaves
+// for loads in flight pull against each other; measured (us, u-pass / p-pass):
+//   8 pencils x 4 CTAs against 16 x 2 (16 threads a pencil): 160x160x192 x 8
+//     378 / 148 against 403 / 156, 256x256x144 111 / 47 against 116 / 53, but
+//     192x192x256 102 / 41 against 97 / 41 and 256^3 172 / 67 against 163 / 66
+//   8 x 2 against 16 x 1 and 8 x 3 (20 threads): 400^3 706 / 289 against
+//     755 / 305 and 817 / 337, 256x256x320 254 / 109 against 263 / 115, 316 / 126
+//   16 x 1 against 8 x 2 (32 threads): 512^3 1786 / 671 against 1847 / 667
+// (one line of spectrum per k row is 8 pencils). Before these tiles, with
+// contiguous runs of 16-pencil tiles per CTA and the smaller split factor
+// first: 400^3 768 / 322, 256x256x320 287 / 125, 160x160x192 x 8 433 / 182,
+// 192x192x256 97 / 43.
+constexpr size_t kSmBytes = 233472;  // shared memory of an SM; each CTA reserves 1 KB of it
+constexpr size_t zp_fit(int ctas) {  // bytes a CTA may use when `ctas` share an SM
+  return (kSmBytes / ctas < 232448 + 1024 ? kSmBytes / ctas : 232448 + 1024) - 1024 - 64;
+}
+
 template <int N>
 struct ZPShape {
   static constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, NH = N / 2 + 1;
-  static constexpr int TPP = ZSplit<N>::TPP;             // threads per pencil
-  static constexpr int THREADS = CG_TILE * TPP;
+  static constexpr int TPP = ZSplit<N>::TPP;           // threads per pencil
+  static constexpr int P = N == 256 || TPP == 32 ? 16 : 8;  // pencils per tile
+  static constexpr int ROWS = 2 * P, THREADS = P * TPP, BOXES = P / 8;
   static constexpr bool WARP = (32 % TPP) == 0;  // a pencil's threads in one warp
-  static constexpr int MINB = TPP == 16 ? CG_FAST_MINB : 1;  // resident CTAs per SM
   // the field values of a thread load before its inverse transform unless
   // the transform's A values per thread leave no registers for them
   static constexpr bool EARLY = A <= 20;
   static constexpr int EX_I = RowEx<A, B>::SLAB, EX_F = RowEx<B, A>::SLAB;
   static constexpr int EX = EX_I > EX_F ? EX_I : EX_F;
-  static constexpr int B_STG = NH * 34, B_EX = CG_TILE * EX, B_XB = N * 17;  // float2 units
-  // tensor-map staging: two 128-byte-wide boxes (8 pencils each) of NH k
-  // rows, each on a 1024-byte boundary (the 128-byte swizzle repeats every 8
-  // rows), plus 1024 bytes to align the first one inside the item buffer
+  // staged boxes, each on a 1024-byte boundary (the 128-byte swizzle repeats
+  // every 8 rows), plus 1024 bytes to align the first one in the item buffer
   static constexpr bool TMA_OK = NH <= 256;
   static constexpr int BOXB = (NH * 128 + 1023) / 1024 * 1024;
-  static constexpr int B_TMA = TMA_OK ? (2 * BOXB + 1024) / 8 : 0;
-  static constexpr int B_MAX0 = B_STG > B_EX ? (B_STG > B_XB ? B_STG : B_XB) : (B_EX > B_XB ? B_EX : B_XB);
-  static constexpr int B_MAX = B_MAX0 > B_TMA ? B_MAX0 : B_TMA;
+  static constexpr int B_STG = (BOXES * BOXB + 1024) / 8, B_EX = P * EX, B_XB = N * P;  // float2 units
+  static constexpr int B_MAX = B_STG > B_EX ? (B_STG > B_XB ? B_STG : B_XB) : (B_EX > B_XB ? B_EX : B_XB);
   static constexpr int BUF = (B_MAX + 1) / 2 * 2;  // even: float4-aligned
-  // without the k_z and sponge tables: they stay in shared memory when
-  // everything fits the 227 KB a CTA may hold, else they are read through L1
-  static constexpr size_t CORE = sizeof(float2) * (2 * N + 2 * (size_t)BUF + 2 * 256) + 2 * (size_t)CG_ZROWS * N;
-  static constexpr size_t LIMIT = 232448 - 64;  // the kernels' static shared variables
-  static constexpr int KZ0 = (NH + 3) / 4 * 2, SZ0 = (N + 3) / 4 * 2;  // float2 units, even
-  static constexpr bool TBL = CORE + sizeof(float2) * (KZ0 + SZ0) <= LIMIT;
-  static constexpr int KZF = TBL ? KZ0 : 0;  // k_z table (floats), float2 units
-  static constexpr int SZF = TBL ? SZ0 : 0;  // z sponge profile (floats), float2 units
-  // twiddles (two orders) | k_z | z sponge | two item buffers | material table | two label tiles
-  static constexpr size_t OFF_KZ = 2 * N, OFF_SZ = OFF_KZ + KZF, OFF_BUF = OFF_SZ + SZF;
-  // per material: float4 (k-space p coefficients) in the p-pass, float2
-  // (dt/rho, absorb) in the u-pass, in the same place
-  static constexpr size_t OFF_TAB = OFF_BUF + 2 * (size_t)BUF;
-  static constexpr size_t OFF_LAB = OFF_TAB + 2 * 256;
-  // then the two staging mbarriers (bytes from the start)
-  static constexpr size_t OFF_BAR = sizeof(float2) * OFF_LAB + 2 * (size_t)CG_ZROWS * N;
-  static constexpr size_t smem = OFF_BAR + 2 * sizeof(unsigned long long);
-  static_assert(smem <= LIMIT, "persistent z-pass tile does not fit shared memory");
 };
 
-// The half spectrum of tile (x, y0) of S into stg4[k * 17 + p], asynchronously
-// (ny even; a ragged last tile stages only its rows below ny).
+// Shared-memory layout of the u-pass (U) or the p-pass:
+// twiddles (two orders, one when A == B) | two item buffers | material table
+// (u: (dt/rho, absorb); p: the four coefficients) | k_z (u) | z sponge | two
+// label tiles | two staging mbarriers. Offsets in float2 units.
+template <int N, bool U>
+struct ZPLayout {
+  using Z = ZPShape<N>;
+  static constexpr int TWF = Z::A == Z::B ? 0 : N;  // twiddles of the forward order
+  static constexpr size_t OFF_BUF = (Z::A == Z::B ? N : 2 * N) + (Z::A == Z::B ? N % 2 : 0);
+  static constexpr size_t OFF_TAB = OFF_BUF + 2 * (size_t)Z::BUF;
+  static constexpr size_t OFF_KZ = OFF_TAB + (U ? 256 : 512);
+  static constexpr size_t LABB = 2 * (size_t)Z::ROWS * N;  // bytes, a multiple of 16
+  static constexpr int KZ0 = U ? (Z::NH + 3) / 4 * 2 : 0, SZ0 = (N + 3) / 4 * 2;
+  static constexpr size_t CORE = sizeof(float2) * OFF_KZ + LABB + 16;
+  // resident CTAs per SM: up to 16 warps (two CTAs of the 20..28-thread
+  // pencils, whose 18..27 values a thread want more than 128 registers), as
+  // far as shared memory allows
+  static constexpr int ctas() {
+    int c = Z::TPP > 16 && Z::TPP < 32 ? 2 : 512 / Z::THREADS;
+    while (c > 1 && CORE > zp_fit(c)) --c;
+    return c;
+  }
+  static constexpr int MINB = ctas();
+  // the k_z and sponge tables stay in shared memory where they cost no
+  // resident CTA, else they are read through L1
+  static constexpr bool TBL = CORE + sizeof(float2) * (KZ0 + SZ0) <= zp_fit(MINB);
+  static constexpr size_t OFF_SZ = OFF_KZ + (TBL ? KZ0 : 0);
+  static constexpr size_t OFF_LAB = OFF_SZ + (TBL ? SZ0 : 0);
+  static constexpr size_t OFF_BAR = sizeof(float2) * OFF_LAB + LABB;  // bytes
+  static constexpr size_t smem = OFF_BAR + 2 * sizeof(unsigned long long);
+  static_assert(smem <= zp_fit(1), "persistent z-pass tile does not fit shared memory");
+};
+
+// An item's place: velocity component comp (radix NC: 3 in the u-pass, 1 in
+// the p-pass), member b, y-tile yt of plane x, the first fastest. CTA i takes
+// items i, i + G, i + 2 G, ...: at any time the resident CTAs work on
+// neighbouring tiles, whose spectrum rows and labels share lines and DRAM
+// pages, and a grid of few tiles still fills the SMs. (A tile's components on
+// three CTAs read its labels three times, once from DRAM; keeping them on one
+// measured 0-3 % slower from 160x160x192 to 400^3.) Stepped by adding the
+// digits of G: a CTA divides once, not once per item.
+template <int NC>
+struct ZCursor {
+  int comp, b, yt, x;
+  int dc, db, dyt, dx;  // digits of the stride
+  __device__ __forceinline__ static void digits(unsigned i, int n_members, int ytiles, int& c, int& b, int& yt,
+                                                int& x) {
+    c = (int)(i % NC);
+    i /= NC;
+    b = (int)(i % (unsigned)n_members);
+    i /= (unsigned)n_members;
+    yt = (int)(i % (unsigned)ytiles);
+    x = (int)(i / (unsigned)ytiles);
+  }
+  __device__ __forceinline__ ZCursor(int n_members, int ytiles) {
+    digits(blockIdx.x, n_members, ytiles, comp, b, yt, x);
+    digits(gridDim.x, n_members, ytiles, dc, db, dyt, dx);
+  }
+  __device__ __forceinline__ void next(int n_members, int ytiles) {
+    comp += dc;
+    b += db;
+    yt += dyt;
+    x += dx;
+    if (comp >= NC) comp -= NC, ++b;
+    if (b >= n_members) b -= n_members, ++yt;
+    if (yt >= ytiles) yt -= ytiles, ++x;
+  }
+};
+
+// First 1024-byte boundary of item buffer j.
+template <int N, class L>
+__device__ __forceinline__ char* zt_stage(float2* sm, int j) {
+  char* b = reinterpret_cast<char*>(sm + L::OFF_BUF + (size_t)j * ZPShape<N>::BUF);
+  const unsigned a = cgf::smem_addr(b);
+  return b + (((a + 1023u) & ~1023u) - a);
+}
+
+// The half spectrum of tile (x, y0) of S into the staging boxes by cp.async
+// (8-byte pieces on an odd ny; the missing second row of a last single row is
+// zero, rows past it are left as they are: nothing of them is stored).
 template <int N>
-__device__ __forceinline__ void z_prefetch(float4* stg4, const float2* __restrict__ S, const Dims& d, int x, int y0) {
-  constexpr int NH = N / 2 + 1;
-  const float2* base = S + (long long)x * NH * d.ny + y0;
-  const int npp = min(CG_TILE, (d.ny - y0) >> 1);
-  for (int idx = threadIdx.x; idx < NH * CG_TILE; idx += blockDim.x) {
-    const int k = idx >> 4, pp = idx & 15;
-    if (pp < npp) cgf::cp_async16(stg4 + k * 17 + pp, base + (long long)k * d.ny + 2 * pp);
+__device__ __forceinline__ void z_prefetch(char* stg, const float2* __restrict__ S, const Dims& d, int x, int y0) {
+  using Z = ZPShape<N>;
+  const float2* base = S + (long long)x * Z::NH * d.ny + y0;
+  const int nyv = min(Z::ROWS, d.ny - y0);
+  const bool even = (d.ny & 1) == 0;
+  for (int idx = threadIdx.x; idx < Z::NH * Z::P; idx += Z::THREADS) {
+    const int k = idx / Z::P, pp = idx % Z::P;
+    char* dst = stg + (pp >> 3) * Z::BOXB + k * 128 + (((pp & 7) ^ (k & 7)) << 4);
+    const float2* src = base + (long long)k * d.ny + 2 * pp;
+    if (2 * pp + 1 < nyv) {
+      if (even) {
+        cgf::cp_async16(dst, src);
+      } else {
+        cgf::cp_async8(dst, src);
+        cgf::cp_async8(dst + 8, src + 1);
+      }
+    } else if (2 * pp < nyv) {
+      cgf::cp_async8(dst, src);
+      *reinterpret_cast<float2*>(dst + 8) = make_float2(0.f, 0.f);
+    }
   }
 }
 
-// The tile's labels (CG_ZROWS rows of N bytes, contiguous), asynchronously.
+// The same by tensor-map box copies, counted on bar; issued by one thread.
+template <int N>
+__device__ __forceinline__ void zt_issue(char* stg, unsigned long long* bar, const CUtensorMap* map, const Dims& d,
+                                         long long b, int x, int y0) {
+  using Z = ZPShape<N>;
+  const int c2 = (int)(b * d.nx + x);
+  cgf::mbar_expect_tx(bar, (unsigned)Z::BOXES * Z::NH * 128u);
+  cgf::tma_load_3d(stg, map, bar, 2 * y0, 0, c2);
+  if constexpr (Z::BOXES == 2) cgf::tma_load_3d(stg + Z::BOXB, map, bar, 2 * y0 + 32, 0, c2);
+}
+
+// The tile's labels (ROWS rows of N bytes, contiguous), asynchronously in the
+// widest pieces the row starts allow (every tile starts a multiple of 16 N
+// bytes into its plane; a plane holds ny N bytes), else by plain byte loads.
 template <int N>
 __device__ __forceinline__ void z_prefetch_labels(uint8_t* lab_s, const uint8_t* __restrict__ labels, const Dims& d,
                                                   int x, int y0) {
+  using Z = ZPShape<N>;
   const uint8_t* src = labels + ((long long)x * d.ny + y0) * N;
-  const int n16 = min(CG_ZROWS, d.ny - y0) * N / 16;
-  for (int i = threadIdx.x; i < n16; i += blockDim.x) cgf::cp_async16(lab_s + 16 * i, src + 16 * i);
+  const int nb = min(Z::ROWS, d.ny - y0) * N;
+  const int plane = d.ny * N;
+  if (plane % 16 == 0) {
+    for (int i = 16 * threadIdx.x; i < nb; i += 16 * Z::THREADS) cgf::cp_async16(lab_s + i, src + i);
+  } else if (plane % 4 == 0) {
+    for (int i = 4 * threadIdx.x; i < nb; i += 4 * Z::THREADS) cgf::cp_async4(lab_s + i, src + i);
+  } else {
+    for (int i = threadIdx.x; i < nb; i += Z::THREADS) lab_s[i] = src[i];
+  }
 }
 
-// z_inputs on a staged tile: times i*mk[k] when mk is given, Im of the
-// self-paired bins dropped, then the Hermitian extension. `row(k)` is the
-// staged float4 (A_k, B_k) of this thread's pencil.
-template <int N, class Row>
-__device__ __forceinline__ void z_inputs_from(float2 (&v)[ZSplit<N>::A], int s, const float* mk, Row row) {
+// Phase-1 inputs of the inverse transform from the staged boxes: times
+// i*mk[k] when mk is given, Im of the self-paired bins dropped, then the
+// Hermitian extension (Z_n = A_n + i B_n, n = s + B a).
+template <int N>
+__device__ __forceinline__ void z_inputs_box(float2 (&v)[ZSplit<N>::A], const char* stg, int p, int s,
+                                             const float* mk) {
   constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B;
+  const char* box = stg + (p >> 3) * ZPShape<N>::BOXB;
+  const int c = p & 7;
   static_for<0, A>([&](auto ai) {
     constexpr int a = decltype(ai)::value;
     const int n = s + B * a;
@@ -509,7 +625,7 @@ __device__ __forceinline__ void z_inputs_from(float2 (&v)[ZSplit<N>::A], int s, 
     if (s < B) {
       const bool hi = 2 * n > N;
       const int k = hi ? N - n : n;
-      const float4 f = row(k);
+      const float4 f = *reinterpret_cast<const float4*>(box + k * 128 + ((c ^ (k & 7)) << 4));
       float2 fa = make_float2(f.x, f.y), fb = make_float2(f.z, f.w);
       if (mk) {
         const float kk = mk[k];
@@ -527,64 +643,28 @@ __device__ __forceinline__ void z_inputs_from(float2 (&v)[ZSplit<N>::A], int s, 
   });
 }
 
-// ... from the padded cp.async staging, stg4[k * 17 + p]
-template <int N>
-__device__ __forceinline__ void z_inputs_raw(float2 (&v)[ZSplit<N>::A], const float4* stg4, int p, int s,
-                                             const float* mk) {
-  z_inputs_from<N>(v, s, mk, [&](int k) { return stg4[k * 17 + p]; });
-}
-
-template <int N, bool UPASS>
+template <int N, bool U>
 __device__ __forceinline__ void zp_tables(float2* sm, const Tables& t, const MediumDev& m) {
+  using L = ZPLayout<N, U>;
   using Z = ZPShape<N>;
   cgf::fill_twt<Z::A, Z::B>(sm, t.twz);
-  cgf::fill_twt<Z::B, Z::A>(sm + N, t.twz);
-  if (Z::TBL) {
-    float* kz_s = reinterpret_cast<float*>(sm + Z::OFF_KZ);
-    for (int i = threadIdx.x; i < Z::NH; i += blockDim.x) kz_s[i] = t.kz[i];
-    float* sz_s = reinterpret_cast<float*>(sm + Z::OFF_SZ);
-    for (int i = threadIdx.x; i < N; i += blockDim.x) sz_s[i] = t.sz[i];
+  if (L::TWF) cgf::fill_twt<Z::B, Z::A>(sm + L::TWF, t.twz);
+  if (L::TBL) {
+    if (U) {
+      float* kz_s = reinterpret_cast<float*>(sm + L::OFF_KZ);
+      for (int i = threadIdx.x; i < Z::NH; i += Z::THREADS) kz_s[i] = t.kz[i];
+    }
+    float* sz_s = reinterpret_cast<float*>(sm + L::OFF_SZ);
+    for (int i = threadIdx.x; i < N; i += Z::THREADS) sz_s[i] = t.sz[i];
   }
   if (m.labels)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+    for (int i = threadIdx.x; i < 256; i += Z::THREADS) {
       const float4 c = m.ltab[i];
-      if (UPASS)
-        sm[Z::OFF_TAB + i] = make_float2(c.x, c.z);
+      if (U)
+        sm[L::OFF_TAB + i] = make_float2(c.x, c.z);
       else
-        reinterpret_cast<float4*>(sm + Z::OFF_TAB)[i] = c;
+        reinterpret_cast<float4*>(sm + L::OFF_TAB)[i] = c;
     }
-}
-
-// Tensor-map staging of item buffer j: its first 1024-byte boundary.
-template <int N>
-__device__ __forceinline__ char* zt_stage(float2* sm, int j) {
-  char* b = reinterpret_cast<char*>(sm + ZPShape<N>::OFF_BUF + (size_t)j * ZPShape<N>::BUF);
-  const unsigned a = cgf::smem_addr(b);
-  return b + (((a + 1023u) & ~1023u) - a);
-}
-
-// The half spectrum of tile (member b, x, y0) into item buffer j by two box
-// copies (pencils 0-7, 8-15), counted on bar; issued by one thread.
-template <int N>
-__device__ __forceinline__ void zt_issue(float2* sm, int j, unsigned long long* bar, const CUtensorMap* map,
-                                         const Dims& d, long long b, int x, int y0) {
-  using Z = ZPShape<N>;
-  char* dst = zt_stage<N>(sm, j);
-  const int c2 = (int)(b * d.nx + x);
-  cgf::mbar_expect_tx(bar, 2u * Z::NH * 128u);
-  cgf::tma_load_3d(dst, map, bar, 2 * y0, 0, c2);
-  cgf::tma_load_3d(dst + Z::BOXB, map, bar, 2 * y0 + 32, 0, c2);
-}
-
-// z_inputs from the tensor-map staging: pencil p's 16 bytes of row k sit in
-// box p / 8 at chunk (p % 8) XOR (k % 8) of the row's 128 bytes.
-template <int N>
-__device__ __forceinline__ void z_inputs_tma(float2 (&v)[ZSplit<N>::A], const char* stg, int p, int s,
-                                             const float* mk) {
-  const char* box = stg + (p >> 3) * ZPShape<N>::BOXB;
-  const int c = p & 7;
-  z_inputs_from<N>(v, s, mk,
-                   [&](int k) { return *reinterpret_cast<const float4*>(box + k * 128 + ((c ^ (k & 7)) << 4)); });
 }
 
 // Waits for item buffer j's staging (tensor-map path); a wait that gives up
@@ -594,137 +674,117 @@ __device__ __forceinline__ void zt_wait(unsigned long long* bars, unsigned& phas
   phase ^= 1u << j;
 }
 
-// TMA: the tile's half spectra arrive by tensor-map box copies on an
-// mbarrier (ztma: the descriptors, by value) instead of per-thread cp.async;
-// the labels keep cp.async. Other instantiations ignore ztma.
+__device__ __forceinline__ void zt_init(unsigned long long* bars) {
+  if (threadIdx.x == 0) {
+    cgf::mbar_init(bars, 1);
+    cgf::mbar_init(bars + 1, 1);
+    cgf::mbar_init_fence();
+  }
+  __syncthreads();
+}
+
+// TMA: the tile's half spectra arrive by tensor-map box copies (ztma: the
+// descriptors, by value) instead of per-thread cp.async; the labels keep
+// cp.async. Other instantiations ignore ztma.
 template <int N, bool TMA = false>
-__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpass_u(Dims d, Tables t, MediumDev m,
-                                                                       float* __restrict__ u, float2* __restrict__ S0,
-                                                                       float2* __restrict__ S1, float2* __restrict__ S2,
-                                                                       int n_members, int tiles_per_cta,
-                                                                       const __grid_constant__ ZTma ztma) {
+__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
+    kfp_zpass_u(Dims d, Tables t, MediumDev m, float* __restrict__ u, float2* __restrict__ S0,
+                float2* __restrict__ S1, float2* __restrict__ S2, int n_members,
+                const __grid_constant__ ZTma ztma) {
   using Z = ZPShape<N>;
+  using L = ZPLayout<N, true>;
   constexpr int A = Z::A, B = Z::B;
   extern __shared__ float2 sm[];
-  const int ytiles = (d.ny + CG_ZROWS - 1) / CG_ZROWS;  // ny even; the last tile may be ragged
-  const long long per_member = (long long)d.nx * ytiles;
-  const long long total = per_member * n_members;
-  const long long t0 = (long long)blockIdx.x * tiles_per_cta;
-  const long long t1 = min(total, t0 + tiles_per_cta);
+  const int ytiles = (d.ny + Z::ROWS - 1) / Z::ROWS;  // the last tile may be ragged
   cgf::pdl_trigger();
-  if (t0 >= t1) return;  // the whole CTA, before any barrier
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(sm) + Z::OFF_BAR);
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(sm) + L::OFF_BAR);
   unsigned phase = 0u;  // bit j: parity of item buffer j's next staging phase
-  if constexpr (TMA) {
-    if (threadIdx.x == 0) {
-      cgf::mbar_init(bars, 1);
-      cgf::mbar_init(bars + 1, 1);
-      cgf::mbar_init_fence();
-    }
-    __syncthreads();
-  }
+  if constexpr (TMA) zt_init(bars);
   zp_tables<N, true>(sm, t, m);
   cgf::pdl_wait();
-  const float* kz_s = Z::TBL ? reinterpret_cast<const float*>(sm + Z::OFF_KZ) : t.kz;
-  const float* sz_s = Z::TBL ? reinterpret_cast<const float*>(sm + Z::OFF_SZ) : t.sz;
-  const float2* tab2_s = sm + Z::OFF_TAB;
-  uint8_t* lab0 = reinterpret_cast<uint8_t*>(sm + Z::OFF_LAB);
+  const float* kz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_KZ) : t.kz;
+  const float* sz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_SZ) : t.sz;
+  const float2* tab2_s = sm + L::OFF_TAB;
+  uint8_t* lab0 = reinterpret_cast<uint8_t*>(sm + L::OFF_LAB);
   const bool lab = m.labels != nullptr;
   const int s = threadIdx.x % Z::TPP, p = threadIdx.x / Z::TPP;
   auto spec = [&](int comp, long long b) { return (comp == 0 ? S1 : (comp == 1 ? S0 : S2)) + b * d.nspec; };
-  // tiles run member-fastest: the members of one (x, y0) follow each other,
-  // so the tile's labels load once for all of them (label slot per group)
-  auto label_slot = [&](long long tile) { return (int)((tile / n_members - t0 / n_members) & 1); };
-  auto prefetch = [&](long long tile, int comp, int j) {
-    const long long b = tile % n_members, r = tile / n_members;
-    const int x = (int)(r / ytiles), y0 = (int)(r - (long long)x * ytiles) * CG_ZROWS;
+  auto prefetch = [&](const ZCursor<3>& c, int j) {
+    const int y0 = c.yt * Z::ROWS;
+    char* stg = zt_stage<N, L>(sm, j);
     if constexpr (TMA) {
-      if (threadIdx.x == 0) zt_issue<N>(sm, j, bars + j, &ztma.map[comp], d, b, x, y0);  // map order = comp order
+      if (threadIdx.x == 0) zt_issue<N>(stg, bars + j, &ztma.map[c.comp], d, c.b, c.x, y0);  // map order = comp order
     } else {
-      z_prefetch<N>(reinterpret_cast<float4*>(sm + Z::OFF_BUF + (size_t)j * Z::BUF), spec(comp, b), d, x, y0);
+      z_prefetch<N>(stg, spec(c.comp, c.b), d, c.x, y0);
     }
-    if (comp == 0 && lab && (tile == t0 || b == 0))
-      z_prefetch_labels<N>(lab0 + label_slot(tile) * CG_ZROWS * N, m.labels, d, x, y0);
+    if (lab) z_prefetch_labels<N>(lab0 + j * Z::ROWS * N, m.labels, d, c.x, y0);
     cgf::cp_async_commit();
   };
-  prefetch(t0, 0, 0);
+  ZCursor<3> cur(n_members, ytiles);
   int j = 0;
-  for (long long tile = t0; tile < t1; ++tile) {
-    const long long b_idx = tile % n_members, r = tile / n_members;
-    const int x = (int)(r / ytiles), y0 = (int)(r - (long long)x * ytiles) * CG_ZROWS;
-    const int ya = y0 + 2 * p, yb = ya + 1;
-    const bool va = ya < d.ny;  // this pencil's rows exist (ny even: yb too)
-    const float spx = t.sx[x];
-    const float spa = va ? spx * t.sy[ya] : 0.f, spb = va ? spx * t.sy[yb] : 0.f;
-    const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
-    const uint8_t* la = lab0 + label_slot(tile) * CG_ZROWS * N + (2 * p) * N;
-    const uint8_t* lb = la + N;
+  prefetch(cur, 0);  // every CTA of the grid has an item
 #pragma unroll 1
-    for (int comp = 0; comp < 3; ++comp, j ^= 1) {
-      float* uc = u + ((long long)comp * n_members + b_idx) * d.ncell;
-      // this thread's velocities load while the staged spectrum is transformed
-      // (after it where A-value registers would not leave room for them)
-      float ua[B], ub[B];
-      auto load_u = [&]() {
-        static_for<0, B>([&](auto bi) {
-          constexpr int b = decltype(bi)::value;
-          const int n = s + A * b;
-          ua[b] = (s < A && va) ? __ldg(uc + rowa + n) : 0.f;
-          ub[b] = (s < A && va) ? __ldg(uc + rowb + n) : 0.f;
-        });
-      };
-      if (Z::EARLY) load_u();
-      // (tensor-map path) this thread's generic accesses to the buffer the
-      // next copy fills are ordered before that copy
-      if constexpr (TMA) cgf::fence_proxy_async();
-      cgf::cp_async_wait0();
-      __syncthreads();
-      {
-        long long nt = tile;
-        int nc = comp + 1;
-        if (nc == 3) {
-          nc = 0;
-          ++nt;
-        }
-        if (nt < t1) prefetch(nt, nc, j ^ 1);
-      }
-      float2* bufj = sm + Z::OFF_BUF + (size_t)j * Z::BUF;
-      float2 v[A], w[B];
-      if constexpr (TMA) {
-        zt_wait(bars, phase, j, ztma.err);
-        z_inputs_tma<N>(v, zt_stage<N>(sm, j), p, s, comp == 2 ? kz_s : nullptr);
-      } else {
-        z_inputs_raw<N>(v, reinterpret_cast<const float4*>(bufj), p, s, comp == 2 ? kz_s : nullptr);
-      }
-      __syncthreads();  // the staging is read: the buffer becomes the exchange
-      const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
-      const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
-      fft2<A, B, true>(v, w, s, sm, exi);
-      if (!Z::EARLY) load_u();
-      // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
-      if (s < A) static_for<0, B>([&](auto bi) {
+  for (; cur.x < d.nx; j ^= 1) {
+    const int comp = cur.comp;
+    const long long b_idx = cur.b;
+    const int x = cur.x, y0 = cur.yt * Z::ROWS;
+    const uint8_t* la = lab0 + j * Z::ROWS * N + (2 * p) * N;
+    const uint8_t* lb = la + N;
+    const int ya = y0 + 2 * p, yb = ya + 1;
+    const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist
+    const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
+    float* uc = u + ((long long)comp * n_members + b_idx) * d.ncell;
+    // this thread's velocities load while the staged spectrum is transformed
+    // (after it where A-value registers would not leave room for them)
+    float ua[B], ub[B];
+    auto load_u = [&]() {
+      static_for<0, B>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
         const int n = s + A * b;
-        const float sz = sz_s[n];
-        // (dt/rho, absorb) of the two cells
-        const float2 ca = lab ? tab2_s[la[n]] : (va ? make_float2(m.dtr[rowa + n], m.ab[rowa + n]) : make_float2(0.f, 0.f));
-        const float2 cb = lab ? tab2_s[lb[n]] : (va ? make_float2(m.dtr[rowb + n], m.ab[rowb + n]) : make_float2(0.f, 0.f));
-        float una = ua[b] - ca.x * w[b].x;
-        una = una * ca.y;
-        una = una * (spa * sz);
-        float unb = ub[b] - cb.x * w[b].y;
-        unb = unb * cb.y;
-        unb = unb * (spb * sz);
-        if (va) {
-          uc[rowa + n] = una;
-          uc[rowb + n] = unb;
-        }
-        w[b] = make_float2(una, unb);
+        ua[b] = (s < A && va) ? __ldg(uc + rowa + n) : 0.f;
+        ub[b] = (s < A && vb) ? __ldg(uc + rowb + n) : 0.f;
       });
-      float2 X[A];
-      fft2<B, A, false>(w, X, s, sm + N, exf);
-      z_split_store<N>(bufj, X, spec(comp, b_idx), d, x, y0, p, s, comp == 2 ? kz_s : nullptr);
-    }
+    };
+    if (Z::EARLY) load_u();
+    // (tensor-map path) this thread's generic accesses to the buffer the
+    // next copy fills are ordered before that copy
+    if constexpr (TMA) cgf::fence_proxy_async();
+    cgf::cp_async_wait0();
+    __syncthreads();
+    cur.next(n_members, ytiles);
+    if (cur.x < d.nx) prefetch(cur, j ^ 1);
+    float2* bufj = sm + L::OFF_BUF + (size_t)j * Z::BUF;
+    float2 v[A], w[B];
+    if constexpr (TMA) zt_wait(bars, phase, j, ztma.err);
+    z_inputs_box<N>(v, zt_stage<N, L>(sm, j), p, s, comp == 2 ? kz_s : nullptr);
+    __syncthreads();  // the staging is read: the buffer becomes the exchange
+    const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
+    const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
+    fft2<A, B, true>(v, w, s, sm, exi);
+    if (!Z::EARLY) load_u();
+    const float spx = t.sx[x];
+    const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
+    // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
+    if (s < A) static_for<0, B>([&](auto bi) {
+      constexpr int b = decltype(bi)::value;
+      const int n = s + A * b;
+      const float sz = sz_s[n];
+      // (dt/rho, absorb) of the two cells
+      const float2 ca = lab ? tab2_s[la[n]] : (va ? make_float2(m.dtr[rowa + n], m.ab[rowa + n]) : make_float2(0.f, 0.f));
+      const float2 cb = lab ? tab2_s[lb[n]] : (vb ? make_float2(m.dtr[rowb + n], m.ab[rowb + n]) : make_float2(0.f, 0.f));
+      float una = ua[b] - ca.x * w[b].x;
+      una = una * ca.y;
+      una = una * (spa * sz);
+      float unb = ub[b] - cb.x * w[b].y;
+      unb = unb * cb.y;
+      unb = unb * (spb * sz);
+      if (va) uc[rowa + n] = una;
+      if (vb) uc[rowb + n] = unb;
+      w[b] = make_float2(una, vb ? unb : 0.f);
+    });
+    float2 X[A];
+    fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+    z_split_store<N, Z::P, false>(bufj, X, spec(comp, b_idx), d, x, y0, p, s, comp == 2 ? kz_s : nullptr);
   }
 }
 
@@ -733,86 +793,78 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpa
 // FWD: only the closing forward transform, of the pressure as it is -- the
 // spectrum a step leaves behind, rebuilt from a restored pressure field by
 // the very code the step runs, so a restored run continues bit for bit.
+// INV: only the opening inverse transform, its values to the pressure.
 // TMA: the half spectra arrive by tensor-map box copies (as in the u-pass).
-template <int N, bool REC, bool FWD = false, bool TMA = false>
-__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpass_p(Dims d, Tables t, MediumDev m,
-                                                                       SourceDev src, RecordDev rec,
-                                                                       const long long* ctl, int n_local, int record,
-                                                                       float* __restrict__ p_all,
-                                                                       float2* __restrict__ S0, int n_members,
-                                                                       int tiles_per_cta,
-                                                                       const __grid_constant__ ZTma ztma) {
+template <int N, bool REC, bool FWD = false, bool TMA = false, bool INV = false>
+__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
+    kfp_zpass_p(Dims d, Tables t, MediumDev m, SourceDev src, RecordDev rec, const long long* ctl, int n_local,
+                int record, float* __restrict__ p_all, float2* __restrict__ S0, int n_members,
+                const __grid_constant__ ZTma ztma) {
   using Z = ZPShape<N>;
+  using L = ZPLayout<N, false>;
   constexpr int A = Z::A, B = Z::B;
-  static_assert(!(FWD && TMA), "the forward-only pass stages no spectrum");
+  static_assert(!(FWD && (TMA || INV)), "the forward-only pass stages no spectrum");
   extern __shared__ float2 sm[];
-  const int ytiles = (d.ny + CG_ZROWS - 1) / CG_ZROWS;  // ny even; the last tile may be ragged
-  const long long per_member = (long long)d.nx * ytiles;
-  const long long total = per_member * n_members;
-  const long long t0 = (long long)blockIdx.x * tiles_per_cta;
-  const long long t1 = min(total, t0 + tiles_per_cta);
+  const int ytiles = (d.ny + Z::ROWS - 1) / Z::ROWS;  // the last tile may be ragged
   cgf::pdl_trigger();
-  if (t0 >= t1) return;  // the whole CTA, before any barrier
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(sm) + Z::OFF_BAR);
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(sm) + L::OFF_BAR);
   unsigned phase = 0u;  // bit j: parity of item buffer j's next staging phase
-  if constexpr (TMA) {
-    if (threadIdx.x == 0) {
-      cgf::mbar_init(bars, 1);
-      cgf::mbar_init(bars + 1, 1);
-      cgf::mbar_init_fence();
-    }
+  if constexpr (TMA) zt_init(bars);
+  if constexpr (FWD) {
+    cgf::fill_twt<Z::B, Z::A>(sm + L::TWF, t.twz);
     __syncthreads();
+  } else if constexpr (INV) {
+    cgf::fill_twt<Z::A, Z::B>(sm, t.twz);
+  } else {
+    zp_tables<N, false>(sm, t, m);
   }
-  zp_tables<N, false>(sm, t, m);
   cgf::pdl_wait();
-  const float* sz_s = Z::TBL ? reinterpret_cast<const float*>(sm + Z::OFF_SZ) : t.sz;
-  const float4* tab_s = reinterpret_cast<const float4*>(sm + Z::OFF_TAB);
-  uint8_t* lab0 = reinterpret_cast<uint8_t*>(sm + Z::OFF_LAB);
-  const bool lab = m.labels != nullptr;
+  const float* sz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_SZ) : t.sz;
+  const float4* tab_s = reinterpret_cast<const float4*>(sm + L::OFF_TAB);
+  uint8_t* lab0 = reinterpret_cast<uint8_t*>(sm + L::OFF_LAB);
+  const bool lab = !INV && m.labels != nullptr;
   const int s = threadIdx.x % Z::TPP, p = threadIdx.x / Z::TPP;
-  // tiles run member-fastest: the members of one (x, y0) follow each other,
-  // so the tile's labels load once for all of them (label slot per group)
-  auto label_slot = [&](long long tile) { return (int)((tile / n_members - t0 / n_members) & 1); };
-  auto prefetch = [&](long long tile, int j) {
-    const long long b = tile % n_members, r = tile / n_members;
-    const int x = (int)(r / ytiles), y0 = (int)(r - (long long)x * ytiles) * CG_ZROWS;
+  auto prefetch = [&](const ZCursor<1>& c, int j) {
+    const int y0 = c.yt * Z::ROWS;
+    char* stg = zt_stage<N, L>(sm, j);
     if constexpr (TMA) {
-      if (threadIdx.x == 0) zt_issue<N>(sm, j, bars + j, &ztma.map[1], d, b, x, y0);  // map[1]: S0
+      if (threadIdx.x == 0) zt_issue<N>(stg, bars + j, &ztma.map[1], d, c.b, c.x, y0);  // map[1]: S0
     } else {
-      z_prefetch<N>(reinterpret_cast<float4*>(sm + Z::OFF_BUF + (size_t)j * Z::BUF), S0 + b * d.nspec, d, x, y0);
+      z_prefetch<N>(stg, S0 + c.b * d.nspec, d, c.x, y0);
     }
-    if (lab && (tile == t0 || b == 0)) z_prefetch_labels<N>(lab0 + label_slot(tile) * CG_ZROWS * N, m.labels, d, x, y0);
+    if (lab) z_prefetch_labels<N>(lab0 + j * Z::ROWS * N, m.labels, d, c.x, y0);
     cgf::cp_async_commit();
   };
+  ZCursor<1> cur(n_members, ytiles);
   if constexpr (FWD) {
     int jf = 0;
-    for (long long tile = t0; tile < t1; ++tile, jf ^= 1) {
-      const long long b_idx = tile % n_members, r = tile / n_members;
-      const int x = (int)(r / ytiles), y0 = (int)(r - (long long)x * ytiles) * CG_ZROWS;
+    for (; cur.x < d.nx; jf ^= 1, cur.next(n_members, ytiles)) {
+      const long long b_idx = cur.b;
+      const int x = cur.x, y0 = cur.yt * Z::ROWS;
       const int ya = y0 + 2 * p;
-      const bool va = ya < d.ny;  // ny even: row ya + 1 too
+      const bool va = ya < d.ny, vb = ya + 1 < d.ny;
       const float* pb = p_all + b_idx * d.ncell;
       const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
       float2 w[B];
       if (s < A) static_for<0, B>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
         const int n = s + A * b;
-        w[b] = make_float2(va ? __ldg(pb + rowa + n) : 0.f, va ? __ldg(pb + rowb + n) : 0.f);
+        w[b] = make_float2(va ? __ldg(pb + rowa + n) : 0.f, vb ? __ldg(pb + rowb + n) : 0.f);
       });
-      float2* bufj = sm + Z::OFF_BUF + (size_t)jf * Z::BUF;
+      float2* bufj = sm + L::OFF_BUF + (size_t)jf * Z::BUF;
       const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
       float2 X[A];
-      fft2<B, A, false>(w, X, s, sm + N, exf);
-      z_split_store<N>(bufj, X, S0 + b_idx * d.nspec, d, x, y0, p, s, nullptr);
+      fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+      z_split_store<N, Z::P, false>(bufj, X, S0 + b_idx * d.nspec, d, x, y0, p, s, nullptr);
     }
     return;
   }
-  prefetch(t0, 0);
-  const long long n_step = ctl[0] + n_local;
+  prefetch(cur, 0);
+  const long long n_step = INV ? 0 : ctl[0] + n_local;
   const int m_bin = (int)(n_step % rec.spp);
   const long long per_log = n_step / rec.spp;
   unsigned int wpeak = 0u;
-  long long wmember = -1;
+  int wmember = -1;
   const long long Ry = rec.hi[1] - rec.lo[1], Rz = rec.hi[2] - rec.lo[2];
   const bool drive_on = src.S > 0 && n_step < src.n_drive;
   const float4 dr = drive_on ? src.drive[n_step] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -825,11 +877,14 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpa
     if (n >= rec.lo[2] && n < rec.hi[2]) zrec |= 1u << b;
   });
   int j = 0;
-  for (long long tile = t0; tile < t1; ++tile, j ^= 1) {
-    const long long b_idx = tile % n_members, r = tile / n_members;
-    const int x = (int)(r / ytiles), y0 = (int)(r - (long long)x * ytiles) * CG_ZROWS;
+#pragma unroll 1
+  for (; cur.x < d.nx; j ^= 1) {
+    const long long b_idx = cur.b;
+    const int x = cur.x, y0 = cur.yt * Z::ROWS;
+    const uint8_t* la = lab0 + j * Z::ROWS * N + (2 * p) * N;
+    const uint8_t* lb = la + N;
     const int ya = y0 + 2 * p, yb = ya + 1;
-    const bool va = ya < d.ny;  // this pencil's rows exist (ny even: yb too)
+    const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist
     float* pb = p_all + b_idx * d.ncell;
     float2* S = S0 + b_idx * d.nspec;
     const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
@@ -841,49 +896,55 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpa
         constexpr int b = decltype(bi)::value;
         const int n = s + A * b;
         pa[b] = (s < A && va) ? __ldg(pb + rowa + n) : 0.f;
-        pbv[b] = (s < A && va) ? __ldg(pb + rowb + n) : 0.f;
+        pbv[b] = (s < A && vb) ? __ldg(pb + rowb + n) : 0.f;
       });
     };
-    if (Z::EARLY) load_p();
+    if (Z::EARLY && !INV) load_p();
     if constexpr (TMA) cgf::fence_proxy_async();  // see the u-pass
     cgf::cp_async_wait0();
     __syncthreads();
-    if (tile + 1 < t1) prefetch(tile + 1, j ^ 1);
-    float2* bufj = sm + Z::OFF_BUF + (size_t)j * Z::BUF;
-    const uint8_t* la = lab0 + label_slot(tile) * CG_ZROWS * N + (2 * p) * N;
-    const uint8_t* lb = la + N;
+    cur.next(n_members, ytiles);
+    if (cur.x < d.nx) prefetch(cur, j ^ 1);
+    float2* bufj = sm + L::OFF_BUF + (size_t)j * Z::BUF;
     float2 v[A], w[B];
-    if constexpr (TMA) {
-      zt_wait(bars, phase, j, ztma.err);
-      z_inputs_tma<N>(v, zt_stage<N>(sm, j), p, s, nullptr);
-    } else {
-      z_inputs_raw<N>(v, reinterpret_cast<const float4*>(bufj), p, s, nullptr);
-    }
+    if constexpr (TMA) zt_wait(bars, phase, j, ztma.err);
+    z_inputs_box<N>(v, zt_stage<N, L>(sm, j), p, s, nullptr);
     __syncthreads();  // the staging is read: the buffer becomes the exchange
     const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
     const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
     fft2<A, B, true>(v, w, s, sm, exi);
+    if constexpr (INV) {
+      if (s < A) static_for<0, B>([&](auto bi) {
+        constexpr int b = decltype(bi)::value;
+        const int n = s + A * b;
+        if (va) pb[rowa + n] = w[b].x;
+        if (vb) pb[rowb + n] = w[b].y;
+      });
+        continue;
+    }
     if (!Z::EARLY) load_p();
     const float spx = t.sx[x];
-    const float spa = va ? spx * t.sy[ya] : 0.f, spb = va ? spx * t.sy[yb] : 0.f;
+    const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
     // p <- (p - (rho c^2 dt [+ 2 beta dt p]) div u) * absorb * sponge   (engine.py:470-477)
     if (s < A) static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int n = s + A * b;
       const float sz = sz_s[n];
       const float4 ca = lab ? tab_s[la[n]] : (va ? cell_coef(m, rowa + n) : make_float4(0.f, 0.f, 0.f, 0.f));
-      const float4 cb = lab ? tab_s[lb[n]] : (va ? cell_coef(m, rowb + n) : make_float4(0.f, 0.f, 0.f, 0.f));
+      const float4 cb = lab ? tab_s[lb[n]] : (vb ? cell_coef(m, rowb + n) : make_float4(0.f, 0.f, 0.f, 0.f));
       const float poa = pa[b], pob = pbv[b];
       float pna = m.nonlinear ? poa - (ca.y + ca.w * poa) * w[b].x : poa - ca.y * w[b].x;
       float pnb = m.nonlinear ? pob - (cb.y + cb.w * pob) * w[b].y : pob - cb.y * w[b].y;
       pna = pna * ca.z;
       pnb = pnb * cb.z;
-      w[b] = make_float2(pna * (spa * sz), pnb * (spb * sz));
+      // rounded here: the transform below takes the stored value, so that the
+      // forward-only pass rebuilds the same spectrum from it bit for bit
+      w[b] = make_float2(__fmul_rn(pna, spa * sz), vb ? __fmul_rn(pnb, spb * sz) : 0.f);
     });
     // source (engine.py:478-482): entries of rows ya, yb owned by this thread
     if (drive_on && s < A && va) {
       const int ra = x * d.ny + ya;
-      const int e0 = src.row_ptr[ra], e1 = src.row_ptr[ra + 1], e2 = src.row_ptr[ra + 2];
+      const int e0 = src.row_ptr[ra], e1 = src.row_ptr[ra + 1], e2 = vb ? src.row_ptr[ra + 2] : e1;
       for (int e = e0; e < e2; ++e) {
         const int zz = src.zidx[e];
         if (zz % A != s) continue;
@@ -904,20 +965,18 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpa
     // write p, convergence peak, record window (z-range membership of this
     // thread's cells is a per-kernel bit mask, the y/x membership per tile)
     unsigned int lpeak = 0u;
-    const bool x_conv = va && x >= rec.clo[0] && x < rec.chi[0];
-    const bool x_rec = REC && va && record && x >= rec.lo[0] && x < rec.hi[0];
-    const bool conv_a = x_conv && ya >= rec.clo[1] && ya < rec.chi[1];
-    const bool conv_b = x_conv && yb >= rec.clo[1] && yb < rec.chi[1];
-    const bool rec_a = x_rec && ya >= rec.lo[1] && ya < rec.hi[1];
-    const bool rec_b = x_rec && yb >= rec.lo[1] && yb < rec.hi[1];
+    const bool x_conv = x >= rec.clo[0] && x < rec.chi[0];
+    const bool x_rec = REC && record && x >= rec.lo[0] && x < rec.hi[0];
+    const bool conv_a = x_conv && va && ya >= rec.clo[1] && ya < rec.chi[1];
+    const bool conv_b = x_conv && vb && yb >= rec.clo[1] && yb < rec.chi[1];
+    const bool rec_a = x_rec && va && ya >= rec.lo[1] && ya < rec.hi[1];
+    const bool rec_b = x_rec && vb && yb >= rec.lo[1] && yb < rec.hi[1];
     if (s < A) static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int n = s + A * b;
       const float pna = w[b].x, pnb = w[b].y;
-      if (va) {
-        pb[rowa + n] = pna;
-        pb[rowb + n] = pnb;
-      }
+      if (va) pb[rowa + n] = pna;
+      if (vb) pb[rowb + n] = pnb;
       if ((zconv >> b) & 1u) {
         if (conv_a) lpeak = max(lpeak, __float_as_uint(fabsf(pna)));
         if (conv_b) lpeak = max(lpeak, __float_as_uint(fabsf(pnb)));
@@ -934,8 +993,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpa
         float* __restrict__ pmax = rec.pmax + b_idx * rec.nrec;
         const long long ra = ((long long)(x - rec.lo[0]) * Ry + (ya - rec.lo[1])) * Rz - rec.lo[2];
         const long long rb = ra + Rz;  // row yb = ya + 1
-        constexpr int RC = 4;
-        static_assert(B % RC == 0, "record chunks split the thread's cells evenly");
+        constexpr int RC = B % 4 == 0 ? 4 : (B % 5 == 0 ? 5 : (B % 3 == 0 ? 3 : (B % 2 == 0 ? 2 : 1)));
         static_for<0, B / RC>([&](auto ci) {
           constexpr int c0 = decltype(ci)::value * RC;
           float sv[2 * RC], cm[2 * RC], pm[2 * RC];
@@ -975,94 +1033,106 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPShape<N>::MINB) kfp_zpa
     lpeak = __reduce_max_sync(0xffffffffu, lpeak);
     if (b_idx != wmember) {
       if ((threadIdx.x & 31) == 0 && wpeak && per_log < rec.max_periods)
-        atomicMax(&rec.peaks[wmember * rec.max_periods + per_log], wpeak);
+        atomicMax(&rec.peaks[(long long)wmember * rec.max_periods + per_log], wpeak);
       wpeak = 0u;
-      wmember = b_idx;
+      wmember = (int)b_idx;
     }
     wpeak = max(wpeak, lpeak);
     float2 X[A];
-    fft2<B, A, false>(w, X, s, sm + N, exf);
-    z_split_store<N>(bufj, X, S, d, x, y0, p, s, nullptr);
+    fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+    z_split_store<N, Z::P, false>(bufj, X, S, d, x, y0, p, s, nullptr);
   }
   if ((threadIdx.x & 31) == 0 && wpeak && wmember >= 0 && per_log < rec.max_periods)
-    atomicMax(&rec.peaks[wmember * rec.max_periods + per_log], wpeak);
+    atomicMax(&rec.peaks[(long long)wmember * rec.max_periods + per_log], wpeak);
 }
 
 // ------------------------------------------------ per-length launchers --
-// persistent z-passes (any N of CG_FAST_ZSIZES, ny even); ztma (encoded
-// descriptors, host memory) selects the tensor-map staging where the length
-// allows it
+// persistent z-passes (any N of CG_FAST_ZSIZES); ztma (encoded descriptors,
+// host memory) selects the tensor-map staging where the length allows it
 static const ZTma kNoZTma = {};
+// one CTA per item up to `per_sm` resident CTAs on every SM
+static int zp_grid(long long items, int per_sm) {
+  const long long slots = (long long)cgf::sm_count() * per_sm;
+  return (int)(items < slots ? items : slots);
+}
+template <int N>
+static long long zp_tiles(const Dims& d, int batch) {
+  return (long long)d.nx * ((d.ny + ZPShape<N>::ROWS - 1) / ZPShape<N>::ROWS) * batch;
+}
 template <int N>
 void zp_run_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
               int batch, cudaStream_t st, const ZTma* ztma) {
-  int g = 0, per = 0;
-  cgf::persistent_grid((long long)d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS) * batch, ZPShape<N>::MINB, &g, &per);
+  using L = ZPLayout<N, true>;
+  const int g = zp_grid(3 * zp_tiles<N>(d, batch), L::MINB);
   if constexpr (ZPShape<N>::TMA_OK) {
     if (ztma) {
-      cgf::launch(kfp_zpass_u<N, true>, dim3(g), dim3(ZPShape<N>::THREADS), ZPShape<N>::smem, st, d, t, m, u, S0, S1,
-                  S2, batch, per, *ztma);
+      cgf::launch(d.pdl, kfp_zpass_u<N, true>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
+                  *ztma);
       return;
     }
   }
-  cgf::launch(kfp_zpass_u<N>, dim3(g), dim3(ZPShape<N>::THREADS), ZPShape<N>::smem, st, d, t, m, u, S0, S1, S2,
-              batch, per, kNoZTma);
+  cgf::launch(d.pdl, kfp_zpass_u<N>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
+              kNoZTma);
 }
 
 template <int N>
 void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
               const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
               const ZTma* ztma) {
-  int g = 0, per = 0;
-  cgf::persistent_grid((long long)d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS) * batch, ZPShape<N>::MINB, &g, &per);
+  using L = ZPLayout<N, false>;
+  const int g = zp_grid(zp_tiles<N>(d, batch), L::MINB);
   const dim3 grid(g), block(ZPShape<N>::THREADS);
-  const size_t sm = ZPShape<N>::smem;
+  const size_t sm = L::smem;
   if constexpr (ZPShape<N>::TMA_OK) {
     if (ztma) {
       if (record)
-        cgf::launch(kfp_zpass_p<N, true, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p,
-                    S0, batch, per, *ztma);
+        cgf::launch(d.pdl, kfp_zpass_p<N, true, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p,
+                    S0, batch, *ztma);
       else
-        cgf::launch(kfp_zpass_p<N, false, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record,
-                    p, S0, batch, per, *ztma);
+        cgf::launch(d.pdl, kfp_zpass_p<N, false, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record,
+                    p, S0, batch, *ztma);
       return;
     }
   }
   if (record)
-    cgf::launch(kfp_zpass_p<N, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, per,
-                kNoZTma);
+    cgf::launch(d.pdl, kfp_zpass_p<N, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, kNoZTma);
   else
-    cgf::launch(kfp_zpass_p<N, false>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch,
-                per, kNoZTma);
+    cgf::launch(d.pdl, kfp_zpass_p<N, false>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, kNoZTma);
 }
 
+// p -> S0 (forward) or S0 -> p (inverse) alone
 template <int N>
-void zp_run_fwd(const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
-                cudaStream_t st) {
-  int g = 0, per = 0;
-  cgf::persistent_grid((long long)d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS) * batch, ZPShape<N>::MINB, &g, &per);
+void zp_run_half(bool inverse, const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
+                 cudaStream_t st) {
+  using L = ZPLayout<N, false>;
+  const int g = zp_grid(zp_tiles<N>(d, batch), L::MINB);
   SourceDev src;
   memset(&src, 0, sizeof(src));
   RecordDev rec;
   memset(&rec, 0, sizeof(rec));
   rec.spp = 1;
-  cgf::launch(kfp_zpass_p<N, false, true>, dim3(g), dim3(ZPShape<N>::THREADS), ZPShape<N>::smem, st, d, t, m, src,
-              rec, (const long long*)nullptr, 0, 0, p, S0, batch, per, kNoZTma);
+  if (inverse)
+    cgf::launch(d.pdl, kfp_zpass_p<N, false, false, false, true>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m,
+                src, rec, (const long long*)nullptr, 0, 0, p, S0, batch, kNoZTma);
+  else
+    cgf::launch(d.pdl, kfp_zpass_p<N, false, true>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, src, rec,
+                (const long long*)nullptr, 0, 0, p, S0, batch, kNoZTma);
 }
 
 template <typename K>
-static bool zp_allow(K kernel, int bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+static bool zp_allow(K kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
 
 template <int N>
 int zp_prepare() {
-  const int sm = (int)ZPShape<N>::smem;
-  bool ok = zp_allow(kfp_zpass_u<N>, sm) && zp_allow(kfp_zpass_p<N, false, true>, sm) &&
-            zp_allow(kfp_zpass_p<N, true>, sm) && zp_allow(kfp_zpass_p<N, false>, sm);
+  constexpr size_t su = ZPLayout<N, true>::smem, sp = ZPLayout<N, false>::smem;
+  bool ok = zp_allow(kfp_zpass_u<N>, su) && zp_allow(kfp_zpass_p<N, false, true>, sp) &&
+            zp_allow(kfp_zpass_p<N, false, false, false, true>, sp) && zp_allow(kfp_zpass_p<N, true>, sp) &&
+            zp_allow(kfp_zpass_p<N, false>, sp);
   if constexpr (ZPShape<N>::TMA_OK)
-    ok = ok && zp_allow(kfp_zpass_u<N, true>, sm) && zp_allow(kfp_zpass_p<N, true, false, true>, sm) &&
-         zp_allow(kfp_zpass_p<N, false, false, true>, sm);
+    ok = ok && zp_allow(kfp_zpass_u<N, true>, su) && zp_allow(kfp_zpass_p<N, true, false, true>, sp) &&
+         zp_allow(kfp_zpass_p<N, false, false, true>, sp);
   return ok ? 0 : -1;
 }
 
@@ -1071,7 +1141,7 @@ template <int N>
 void zt_run_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
               int batch, cudaStream_t st) {
   const dim3 grid((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), batch);
-  cgf::launch(kf_zpass_u<N>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, u, S0, S1, S2);
+  cgf::launch(d.pdl, kf_zpass_u<N>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, u, S0, S1, S2);
 }
 
 template <int N>
@@ -1079,13 +1149,10 @@ void zt_run_p(int mode, const Dims& d, const Tables& t, const MediumDev& m, cons
               const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st) {
   const dim3 grid((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), batch);
   if (mode == 0)
-    cgf::launch(kf_zpass_p<N, 0>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, src, rec, ctl, n_local,
-                record, p, S0);
-  else if (mode == 1)
-    cgf::launch(kf_zpass_p<N, 1>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, src, rec, ctl, n_local,
+    cgf::launch(d.pdl, kf_zpass_p<N, 0>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, src, rec, ctl, n_local,
                 record, p, S0);
   else
-    cgf::launch(kf_zpass_p<N, 2>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, src, rec, ctl, n_local,
+    cgf::launch(d.pdl, kf_zpass_p<N, 1>, grid, dim3(CG_THREADS), ZShape<N>::smem, st, d, t, m, src, rec, ctl, n_local,
                 record, p, S0);
 }
 
@@ -1094,8 +1161,7 @@ int zt_prepare() {
   const int sm = (int)ZShape<N>::smem;
   return (cudaFuncSetAttribute(kf_zpass_u<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess ||
           cudaFuncSetAttribute(kf_zpass_p<N, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess ||
-          cudaFuncSetAttribute(kf_zpass_p<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess ||
-          cudaFuncSetAttribute(kf_zpass_p<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
+          cudaFuncSetAttribute(kf_zpass_p<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm) != cudaSuccess)
              ? -1
              : 0;
 }
@@ -1105,7 +1171,8 @@ int zt_prepare() {
                             cudaStream_t, const ZTma*);                                                            \
   template void zp_run_p<n>(const Dims&, const Tables&, const MediumDev&, const SourceDev&, const RecordDev&,     \
                             const long long*, int, int, float*, float2*, int, cudaStream_t, const ZTma*);         \
-  template void zp_run_fwd<n>(const Dims&, const Tables&, const MediumDev&, float*, float2*, int, cudaStream_t); \
+  template void zp_run_half<n>(bool, const Dims&, const Tables&, const MediumDev&, float*, float2*, int,            \
+                               cudaStream_t);                                                                      \
   template int zp_prepare<n>();
 #define CG_ZT_INSTANTIATE(n)                                                                                       \
   template void zt_run_u<n>(const Dims&, const Tables&, const MediumDev&, float*, float2*, float2*, float2*, int,  \

@@ -729,6 +729,13 @@ static size_t smem_zpass(int nz) {
   return sizeof(float2) * ((size_t)nz + a + (a > st ? a : st));
 }
 
+// Programmatic dependent launch of the x- and z-passes unless CG_PDL=0 (the
+// y-passes never take it, yx_launch_y).
+static int pdl_default() {
+  const char* e = getenv("CG_PDL");
+  return (e && e[0] == '0') ? 0 : 1;
+}
+
 extern "C" int cg_solver_create(const cg_solver_config* cfg, cg_solver** out) {
   CG_REQUIRE(cfg && out, "null argument");
   *out = nullptr;
@@ -748,6 +755,7 @@ extern "C" int cg_solver_create(const cg_solver_config* cfg, cg_solver** out) {
   s->d.nzh = cfg->nz / 2 + 1;
   s->d.ncell = (long long)cfg->nx * cfg->ny * cfg->nz;
   s->d.nspec = (long long)cfg->nx * s->d.nzh * cfg->ny;
+  s->d.pdl = pdl_default();
   s->B = cfg->batch;
   if (cg_make_plan(cfg->nx, &s->px) || cg_make_plan(cfg->ny, &s->py) || cg_make_plan(cfg->nz, &s->pz)) {
     cg_set_error("grid %dx%dx%d: every axis must be 2/3/5-smooth and <= %d", cfg->nx, cfg->ny, cfg->nz, CG_MAX_N);
@@ -1136,7 +1144,7 @@ static int launch_step_slabs(cg_solver* s, int n_local, int record, EvLog* log) 
     mark(6);
     ok = ok && fast_ypass(Y_INV, sl.d, sl.t, sl.S0, sl.S1, sl.S2, B, st);
     mark(7);
-    ok = ok && fast_zpass_p(1, sl.d, sl.t, sl.m, sl.src, sl.rec, s->ctl, n_local, record, sl.p, sl.S0, B, st, true);
+    ok = ok && fast_zpass_p(sl.d, sl.t, sl.m, sl.src, sl.rec, s->ctl, n_local, record, sl.p, sl.S0, B, st, true);
     mark(0);
     ok = ok && fast_ypass(Y_FWD, sl.d, sl.t, sl.S0, sl.S1, sl.S2, B, st);
   }
@@ -1207,7 +1215,7 @@ static int launch_step(cg_solver* s, int n_local, int record, EvLog* log = nullp
   mark(7);
   if (!(zt && fast_zpass_p_tma(d, t, m, make_source(s), make_record(s), s->ctl, n_local, record, s->p, s->S0, B,
                                st, s->ztma_host)) &&
-      !fast_zpass_p(1, d, t, m, make_source(s), make_record(s), s->ctl, n_local, record, s->p, s->S0, B, st,
+      !fast_zpass_p(d, t, m, make_source(s), make_record(s), s->ctl, n_local, record, s->p, s->S0, B, st,
                     s->zpers != 0))
     k_zpass_p<<<gz, CG_THREADS, s->smem_z, st>>>(1, d, s->pz, t, m, make_source(s), make_record(s), s->ctl, n_local,
                                                  record, s->p, s->S0);
@@ -1483,7 +1491,7 @@ extern "C" int cg_solver_autotune(cg_solver* s, int n_steps, int* out4) {
   const bool fx_ok = !(fenv && fenv[0] == '0') && !slab_pinned && fused_xy_supported(s->d);
   const int fx_lo = (fx_ok && fenv && fenv[0] == '1') ? 1 : 0;
   // the per-tile z-passes exist for the lengths of CG_FAST_SIZES only
-  const bool zp_choice = (s->d.ny % 2 == 0) && fast_has(s->d.nz) && !slab_pinned;
+  const bool zp_choice = fast_has(s->d.nz) && !slab_pinned;
   invalidate_graphs(s);
   cudaEvent_t a, b;
   CG_CUDA_TRY(cudaEventCreate(&a));
@@ -1518,13 +1526,16 @@ extern "C" int cg_solver_autotune(cg_solver* s, int n_steps, int* out4) {
       for (int i = 0; i < nk; ++i) cand[nc++] = {0, 1, ks[i], 0};
     }
   }
+  auto use = [&](const TuneChoice& c) {
+    s->fused_xy = c.fused;
+    s->zpers = c.zpers;
+    s->slabs = c.slabs;
+    s->ztma = c.ztma;
+  };
   for (int c = 0; c < nc; ++c) cand_ms[c] = 1e30f;
   for (int r = 0; r < kRounds; ++r)
     for (int c = 0; c < nc; ++c) {
-      s->fused_xy = cand[c].fused;
-      s->zpers = cand[c].zpers;
-      s->slabs = cand[c].slabs;
-      s->ztma = cand[c].ztma;
+      use(cand[c]);
       int rc = CG_OK;
       for (int k = 0; k < (r == 0 ? 2 : 1) && rc == CG_OK; ++k) rc = launch_step(s, k % s->spp, 0);
       CG_CUDA_TRY(cudaEventRecord(a, s->stream));
@@ -1549,10 +1560,7 @@ extern "C" int cg_solver_autotune(cg_solver* s, int n_steps, int* out4) {
     }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
-  s->fused_xy = best.fused;
-  s->zpers = best.zpers;
-  s->slabs = best.slabs;
-  s->ztma = best.ztma;
+  use(best);
   int rc = ztma_check(s);
   if (rc != CG_OK) return rc;
   rc = cg_solver_reset(s);
@@ -1676,6 +1684,7 @@ extern "C" int cg_fft3d_create(int nx, int ny, int nz, int batch, cg_fft3d** out
   f->d.nx = nx; f->d.ny = ny; f->d.nz = nz; f->d.nzh = nz / 2 + 1;
   f->d.ncell = (long long)nx * ny * nz;
   f->d.nspec = (long long)nx * f->d.nzh * ny;
+  f->d.pdl = pdl_default();
   f->B = batch;
   if (cg_make_plan(nx, &f->px) || cg_make_plan(ny, &f->py) || cg_make_plan(nz, &f->pz)) {
     cg_set_error("FFT shape %dx%dx%d: every axis must be 2/3/5-smooth and <= %d", nx, ny, nz, CG_MAX_N);
@@ -1752,7 +1761,7 @@ extern "C" int cg_fft3d_forward(cg_fft3d* f, const float* in, float* out_spec) {
   const dim3 gy((unsigned)((d.nx * (long long)d.nzh + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gx((unsigned)(((long long)d.nzh * d.ny + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gz((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), f->B);
-  if (!fast_zpass_p(0, d, t, m, sd, rd, nullptr, 0, 0, f->real, f->spec, f->B, f->stream))
+  if (!fast_zpass_half(false, d, t, m, f->real, f->spec, f->B, f->stream))
     k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(0, d, f->pz, t, m, sd, rd, nullptr, 0, 0, f->real, f->spec);
   if (!fast_ypass(Y_FWD, d, t, f->spec, nullptr, nullptr, f->B, f->stream))
     k_ypass<<<gy, CG_THREADS, f->smem_y, f->stream>>>(Y_FWD, d, f->py, t, f->spec, nullptr, nullptr);
@@ -1783,7 +1792,7 @@ extern "C" int cg_fft3d_inverse(cg_fft3d* f, const float* in_spec, float* out) {
     k_xpass<<<gx, CG_THREADS, f->smem_x, f->stream>>>(X_INV, d, f->px, t, 0.f, 1.f, f->spec, nullptr, nullptr);
   if (!fast_ypass(Y_INV, d, t, f->spec, nullptr, nullptr, f->B, f->stream))
     k_ypass<<<gy, CG_THREADS, f->smem_y, f->stream>>>(Y_INV, d, f->py, t, f->spec, nullptr, nullptr);
-  if (!fast_zpass_p(2, d, t, m, sd, rd, nullptr, 0, 0, f->real, f->spec, f->B, f->stream))
+  if (!fast_zpass_half(true, d, t, m, f->real, f->spec, f->B, f->stream))
     k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(2, d, f->pz, t, m, sd, rd, nullptr, 0, 0, f->real, f->spec);
   CG_CUDA_TRY(cudaGetLastError());
   CG_CUDA_TRY(cudaMemcpyAsync(out, f->real, sizeof(float) * f->B * d.ncell, cudaMemcpyDefault, f->stream));

@@ -20,6 +20,7 @@ struct Dims {
   int nx, ny, nz, nzh;
   long long ncell;  // nx*ny*nz
   long long nspec;  // nx*nzh*ny
+  int pdl = 0;      // host: launch the x- and z-passes with programmatic stream serialisation
 };
 
 struct Tables {
@@ -121,9 +122,12 @@ bool fast_xpass(int mode, const Dims& d, const Tables& t, float kcoef, float inv
 // persistent = false keeps the one-tile-per-CTA z kernels (autotuner choice)
 bool fast_zpass_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
                   int batch, cudaStream_t st, bool persistent = true);
-bool fast_zpass_p(int mode, const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src,
-                  const RecordDev& rec, const long long* ctl, int n_local, int record, float* p, float2* S0,
-                  int batch, cudaStream_t st, bool persistent = true);
+bool fast_zpass_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
+                  const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
+                  bool persistent = true);
+// the z-transform alone: p -> S0, or S0 -> p (unnormalised)
+bool fast_zpass_half(bool inverse, const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0,
+                     int batch, cudaStream_t st);
 
 // Tensor-map (TMA) staging of the persistent z-tiles: one descriptor per
 // spectrum in the u-pass's component order (S1, S0, S2; the p-pass reads
@@ -155,10 +159,16 @@ bool fast_zpass_p_tma(const Dims& d, const Tables& t, const MediumDev& m, const 
 bool fast_zpass_fwd_step(const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
                          cudaStream_t st, bool persistent);
 
-// Axis lengths with a size-specialised kernel.
+// Axis lengths with a one-tile-per-CTA z-pass (the autotuner's alternative to
+// the persistent ones).
 #define CG_FAST_SIZES(X) X(8) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(160) X(192) X(256)
-// lengths of the x/y passes and of the persistent z-passes (ny even): the
-// above, 320 and 400 (20 threads per pencil), 512 and 640 (32 threads per
-// pencil)
-#define CG_FAST_ZSIZES(X) CG_FAST_SIZES(X) X(320) X(400) X(512) X(640)
+// Axis lengths of the size-specialised x-, y- and persistent z-passes: the
+// above, every other 2/3/5-smooth length from 36 to 400 (a grid of any size is
+// padded to such lengths), 512 and 640. The remaining ones run the
+// runtime-plan passes.
+#define CG_FAST_ZSIZES(X)                                                                                         \
+  CG_FAST_SIZES(X)                                                                                                \
+  X(36) X(40) X(45) X(50) X(54) X(60) X(72) X(75) X(80) X(81) X(90) X(100) X(108) X(120) X(125) X(135) X(144)      \
+  X(150) X(162) X(180) X(200) X(216) X(225) X(240) X(243) X(250) X(270) X(288) X(300) X(320) X(324) X(360) X(375) \
+  X(384) X(400) X(512) X(640)
 #define CG_FAST_XYSIZES(X) CG_FAST_ZSIZES(X)
