@@ -388,6 +388,13 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const void* map, unsigned
       : "memory");
 }
 
+// A value that this pass reads once, kept out of the L1 and in program order.
+__device__ __forceinline__ float2 ld_once(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
+}
+
 // Programmatic dependent launch: a pass lets the next one launch as soon as
 // all of its own CTAs are running (pdl_trigger), and waits for the previous
 // pass to complete and its writes to be visible (pdl_wait) before its first

@@ -185,7 +185,16 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
   auto load = [&](const float2* __restrict__ src) {
     static_for<0, A>([&](auto ai) {
       constexpr int a = decltype(ai)::value;
-      v[a] = (valid && s < B) ? src[base + (long long)(s + B * a) * ncol] : make_float2(0.f, 0.f);
+      const float2* g = src + (base + (long long)(s + B * a) * ncol);
+      // in program order: the compiler otherwise starts the divergence pass's
+      // second tile under the first transform and spills (X_GRAD / X_DIV us,
+      // plain against ordered: 192x192x256 41 / 41 -> 39 / 39, 240^3 58 / 70 ->
+      // 55 / 59, 384^3 269 / 304 -> 267 / 282; 20 threads a pencil have the
+      // registers for it: 400^3 309 / 290 -> 309 / 298)
+      if constexpr (PSplit<N>::TPP == 20)
+        v[a] = (valid && s < B) ? *g : make_float2(0.f, 0.f);
+      else
+        v[a] = (valid && s < B) ? cgf::ld_once(g) : make_float2(0.f, 0.f);
     });
   };
   // after an inverse (B, A) transform thread s < B owns z[a] = element s + B a
@@ -257,23 +266,31 @@ static size_t smem_x() {
 }
 
 // ------------------------------------------------ per-length launchers --
-// Never a programmatic dependent launch: a y-pass that starts while CTAs of a
-// z- or x-pass are still resident runs on the shared-memory carve-out of that
-// pass, because an SM changes it only when empty, and the y-pass wants the L1
-// for its loads in flight. Per step with all passes / x and z only / none
-// launched programmatically: 64^3 41 / 33 / 42 us, 160x160x192 161 / 162 / 170,
-// 160x160x192 x 2 349 / 311 / 315, 240^3 480 / 438 / 446, 256x256x320
-// 727 / 671 / 675.
+// Programmatic dependent launch of the y-passes. Not after a z-pass: a y-pass
+// that starts while CTAs of a z-pass are still resident runs on the
+// shared-memory carve-out of that pass, because an SM changes it only when
+// empty, and the y-pass wants the L1 for its loads in flight. Per step with all
+// passes / x and z only / none launched programmatically: 64^3 41 / 33 / 42 us,
+// 160x160x192 161 / 162 / 170, 160x160x192 x 2 349 / 311 / 315, 240^3
+// 480 / 438 / 446, 256x256x320 727 / 671 / 675. After an x-pass (the inverse
+// y-passes) where 16-thread x-CTAs leave 64 KB of L1 (nx <= 192) and the grid
+// is not so small that waiting CTAs delay the x-pass: with / without, 192x192x256
+// 279 / 282 us, 128x128x160 96 / 100, 96x96x128 54 / 54, 64^3 36 / 33, 240^3
+// 471 / 444, 300^3 1126 / 1114.
+static inline int y_pdl(int mode, const Dims& d) {
+  return d.pdl && (mode == Y_INV || mode == Y_INV_GRAD) && d.nx <= 192 && d.ncell >= (1 << 20);
+}
+
 template <int N>
 bool yx_launch_y(int mode, const Dims& d, const Tables& t, float2* S0, float2* S1, float2* S2, int batch,
                  cudaStream_t st) {
   const dim3 grid((unsigned)((d.nx * (long long)d.nzh + YT<N>::YP - 1) / YT<N>::YP), batch);
   const dim3 block(YT<N>::THREADS);
   switch (mode) {
-    case Y_FWD: cgf::launch(0, kf_ypass<N, Y_FWD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    case Y_INV: cgf::launch(0, kf_ypass<N, Y_INV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    case Y_INV_GRAD: cgf::launch(0, kf_ypass<N, Y_INV_GRAD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    default: cgf::launch(0, kf_ypass<N, Y_FWD_DIV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_FWD: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_FWD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_INV: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_INV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_INV_GRAD: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_INV_GRAD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    default: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_FWD_DIV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
   }
   return true;
 }
