@@ -516,44 +516,109 @@ __global__ void __launch_bounds__(CG_THREADS) k_zpass_p(int mode, Dims d, AxisPl
   z_store_forward(S, f, d, x, y0, nyv, nullptr);
 }
 
-// Final phasors in FP64: P_h = 2/K sum_m (s_m - c_m) exp(+2 pi i h m / spp)
-// (engine.py:538-552: buffers[h] += p exp(+i h w t); *= 2/rec_steps).
-// The nh x spp unit phasors are formed once per block in shared memory (FP64
-// sincospi is slow on GB300); every bin is read once and feeds all
-// harmonics, each summed over m in increasing order.
-__global__ void k_finalize(RecordDev rec, int B, int nh, const int* harm, int K, float2* out) {
-  extern __shared__ double2 uph[];  // [nh][spp] (cos, sin)
-  for (int i = threadIdx.x; i < nh * rec.spp; i += blockDim.x) {
+// Final phasors P_h = sum_m (s_m - c_m) u_hm, u_hm = 2/K exp(+2 pi i h m / spp)
+// (engine.py:538-552: buffers[h] += p exp(+i h w t); *= 2/rec_steps). The nh x
+// spp factors are formed in FP64 once per block, in shared memory; every bin is
+// read once and feeds all harmonics, each summed over m in increasing order.
+//
+// Bound: HBM, 8 spp bytes read and 8 nh written per voxel. FP64 arithmetic is
+// slow on GB300 and took 4.9 ms for three harmonics of 192x192x256 (13 bins,
+// 1.2 GB of traffic) where the traffic takes 0.2 ms, so the products and sums run on unevaluated
+// pairs of floats (Dekker's two-sum and the fused two-product: relative error
+// below 2^-44 of the largest term, far inside the final rounding to float32).
+// That needs the error terms to be representable: a voxel whose bins are not
+// all zero and not all within [2^-60, 2^120] takes the FP64 sum. u carries the factor 2/K
+// from the start, so no partial sum exceeds twice the largest pressure.
+constexpr float kPairLo = 8.6736174e-19f, kPairHi = 1.3292280e36f;  // 2^-60, 2^120
+
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float t = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+}
+
+template <int NH>
+__global__ void __launch_bounds__(256) k_finalize(RecordDev rec, int B, const int* harm, int K, float2* out) {
+  extern __shared__ float4 upf[];  // [NH][spp] float pairs (re hi, re lo, im hi, im lo)
+  const double sc = 2.0 / K;
+  for (int i = threadIdx.x; i < NH * rec.spp; i += blockDim.x) {
     const int h = i / rec.spp, mm = i - h * rec.spp;
     double sn, cs;
     sincospi(2.0 * (double)((harm[h] * (long long)mm) % rec.spp) / rec.spp, &sn, &cs);
-    uph[i] = make_double2(cs, sn);
+    const double re = cs * sc, im = sn * sc;
+    const float rh = (float)re, ih = (float)im;
+    upf[i] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
   }
   __syncthreads();
   const long long total = (long long)B * rec.nrec;
-  const double sc = 2.0 / K;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long b = i / rec.nrec;
     const long long r = i - b * rec.nrec;
-    double re[CG_MAX_H], im[CG_MAX_H];
+    const float* bins = rec.bins + b * rec.spp * rec.nrec + r;
+    const float* comp = rec.comp + b * rec.spp * rec.nrec + r;
+    float re[NH], ree[NH], im[NH], ime[NH];  // sums and their error terms
 #pragma unroll
-    for (int h = 0; h < CG_MAX_H; ++h) re[h] = im[h] = 0.0;
-    for (int mm = 0; mm < rec.spp; ++mm) {
-      const long long o = (b * rec.spp + mm) * rec.nrec + r;
-      const double v = (double)rec.bins[o] - (double)rec.comp[o];
+    for (int h = 0; h < NH; ++h) re[h] = ree[h] = im[h] = ime[h] = 0.f;
+    bool exact = true;
+    constexpr int U = 4;  // bins loaded ahead of their use
+    for (int m0 = 0; m0 < rec.spp; m0 += U) {
+      float sv[U], cv[U];
 #pragma unroll
-      for (int h = 0; h < CG_MAX_H; ++h)
-        if (h < nh) {
-          const double2 u = uph[h * rec.spp + mm];
-          re[h] += v * u.x;
-          im[h] += v * u.y;
+      for (int j = 0; j < U; ++j) {
+        const bool in = m0 + j < rec.spp;
+        sv[j] = in ? __ldcs(bins + (m0 + j) * rec.nrec) : 0.f;
+        cv[j] = in ? __ldcs(comp + (m0 + j) * rec.nrec) : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        if (m0 + j >= rec.spp) break;
+        float v, w;  // s - c as an exact pair
+        two_sum(sv[j], -cv[j], v, w);
+        const float av = fabsf(v);
+        exact = exact && (av == 0.f || (av >= kPairLo && av <= kPairHi));
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+          const float4 u = upf[h * rec.spp + m0 + j];
+          float p = __fmul_rn(v, u.x), e;
+          float t = __fmaf_rn(w, u.x, __fmaf_rn(v, u.y, __fmaf_rn(v, u.x, -p)));
+          two_sum(re[h], p, re[h], e);
+          ree[h] = __fadd_rn(ree[h], __fadd_rn(e, t));
+          p = __fmul_rn(v, u.z);
+          t = __fmaf_rn(w, u.z, __fmaf_rn(v, u.w, __fmaf_rn(v, u.z, -p)));
+          two_sum(im[h], p, im[h], e);
+          ime[h] = __fadd_rn(ime[h], __fadd_rn(e, t));
         }
+      }
     }
+    if (exact) {
 #pragma unroll
-    for (int h = 0; h < CG_MAX_H; ++h)
-      if (h < nh) out[(b * nh + h) * rec.nrec + r] = make_float2((float)(re[h] * sc), (float)(im[h] * sc));
+      for (int h = 0; h < NH; ++h)
+        out[(b * NH + h) * rec.nrec + r] = make_float2(__fadd_rn(re[h], ree[h]), __fadd_rn(im[h], ime[h]));
+    } else {
+#pragma unroll 1
+      for (int h = 0; h < NH; ++h) {
+        double dr = 0.0, di = 0.0;
+        for (int mm = 0; mm < rec.spp; ++mm) {
+          const double v = (double)bins[mm * rec.nrec] - (double)comp[mm * rec.nrec];
+          const float4 u = upf[h * rec.spp + mm];
+          dr += v * ((double)u.x + (double)u.y);
+          di += v * ((double)u.z + (double)u.w);
+        }
+        out[(b * NH + h) * rec.nrec + r] = make_float2((float)dr, (float)di);
+      }
+    }
   }
+}
+
+static size_t smem_finalize(int nh, int spp) { return sizeof(float4) * (size_t)nh * spp; }
+
+static const void* finalize_kernel(int nh) {
+  static const void* const k[CG_MAX_H] = {(const void*)k_finalize<1>, (const void*)k_finalize<2>,
+                                          (const void*)k_finalize<3>, (const void*)k_finalize<4>,
+                                          (const void*)k_finalize<5>, (const void*)k_finalize<6>,
+                                          (const void*)k_finalize<7>, (const void*)k_finalize<8>};
+  return k[nh - 1];
 }
 
 // ------------------------------------------------------------ set-up ----
@@ -872,7 +937,7 @@ extern "C" int cg_solver_create(const cg_solver_config* cfg, cg_solver** out) {
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_xpass);
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_zpass_u);
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_zpass_p);
-  if (e == cudaSuccess) e = allow_max_smem((const void*)k_finalize);
+  if (e == cudaSuccess) e = allow_max_smem(finalize_kernel(s->nh));
   if (e == cudaSuccess && fast_prepare() != 0) e = cudaErrorInvalidValue;
   if (e != cudaSuccess) {
     cg_set_error("solver set-up: %s", cudaGetErrorString(e));
@@ -1316,9 +1381,11 @@ extern "C" int cg_solver_finalize(cg_solver* s, int n_record_steps, float* phaso
     int rc = dev_alloc(&s->ph, (size_t)s->B * s->nh * s->nrec);
     if (rc != CG_OK) return rc;
   }
-  k_finalize<<<1024, 256, sizeof(double2) * (size_t)s->nh * s->spp, s->stream>>>(make_record(s), s->B, s->nh,
-                                                                                  s->harm_dev, n_record_steps, s->ph);
-  cudaError_t e = cudaGetLastError();
+  RecordDev rec = make_record(s);
+  void* args[] = {&rec, &s->B, &s->harm_dev, &n_record_steps, &s->ph};
+  const long long blocks = ((long long)s->B * s->nrec + 255) / 256, most = 152LL * 8 * 4;  // four waves
+  cudaError_t e = cudaLaunchKernel(finalize_kernel(s->nh), dim3((unsigned)(blocks < most ? blocks : most)), dim3(256),
+                                   args, smem_finalize(s->nh, s->spp), s->stream);
   if (e == cudaSuccess && phasors)
     e = cudaMemcpyAsync(phasors, s->ph, sizeof(float2) * (size_t)s->B * s->nh * s->nrec, cudaMemcpyDefault,
                         s->stream);
