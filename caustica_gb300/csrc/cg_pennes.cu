@@ -57,117 +57,132 @@ __device__ __forceinline__ float cem43_rate_dev(float T) {
   return (T > 43.0f) ? exp2f(-e) : exp2f(-2.0f * e);
 }
 
-// One cell of the sub-step; (x, y, z) its coordinates, i its linear index.
-__device__ __forceinline__ void pennes_cell(const PennesDev& P, const float* __restrict__ th, float* __restrict__ thn,
-                                            float* thmax, float* dose, float* dcomp, const float4* tab,
-                                            const float* ft, long long i, int x, int y, int z) {
-  const long long sx = (long long)P.ny * P.nz, sy = P.nz;
-  const float t0 = th[i];
-  const bool lab = P.labels != nullptr;
-  const int lme = lab ? P.labels[i] : 0;
-  const float4 me = lab ? tab[lme] : make_float4(0.f, 0.f, 0.f, 0.f);
-  // face conductance between lower-index material a and upper-index b
-  auto fk = [&](int a, int b) {
-    return ft ? ft[a * P.nlab + b] : face_k(tab[a].x, tab[b].x, P.inv_dx2);
+// One sub-step on dense per-cell coefficient maps, streaming along x: block
+// (32, PD_Y) owns a z-y tile and walks xs consecutive x planes; a warp is one
+// z row. A thread keeps its x-1 / x / x+1 temperatures and the x face below it
+// in registers, takes its z neighbours and lower z face from the next lanes,
+// and reads the y neighbours through L1 (the next warps' rows), so no barrier
+// is needed. Every load of plane x + 1 is issued before plane x is computed,
+// none behind a branch on another's value.
+//
+// Bound: HBM (57 bytes per cell with dose) on large grids, latency below L2
+// size. 101x117x143 with dose and walls: 24 us a sub-step, 256x256x320 with dose
+// 220 us (5.3 TB/s); 43 us with one row per warp, six neighbour and six face
+// loads per cell in branches of their own.
+#define PD_Y 8
+template <bool DOSE, bool DIR>
+__global__ void __launch_bounds__(32 * PD_Y) k_pennes_dense(PennesDev P, int xs, const float* __restrict__ th,
+                                                            float* __restrict__ thn, float* __restrict__ thmax,
+                                                            float* __restrict__ dose, float* __restrict__ dcomp) {
+  cgf::pdl_trigger();
+  const int lane = threadIdx.x;
+  const unsigned ztiles = ((unsigned)P.nz + 31) / 32, yt = blockIdx.x / ztiles;
+  const int z = (int)(blockIdx.x - yt * ztiles) * 32 + lane, y = (int)yt * PD_Y + threadIdx.y;
+  const int x0 = blockIdx.y * xs, x1 = min(P.nx, x0 + xs);
+  const bool in = z < P.nz && y < P.ny;
+  const bool yhi = in && y + 1 < P.ny, ylo = in && y > 0, zhi = in && z + 1 < P.nz, zlo = in && z > 0;
+  // the lane whose z neighbour is in another warp's row piece loads it
+  const bool hlo = zlo && lane == 0, hhi = zhi && lane == 31;
+  const long long sx = (long long)P.ny * P.nz, sky = (long long)(P.ny - 1) * P.nz, skz = (long long)P.ny * (P.nz - 1);
+  const int c0 = y * P.nz + z;                 // (y, z) inside a plane of cells or x faces
+  const int cy = c0, cz = y * (P.nz - 1) + z;  // ... of y faces, of z faces
+  struct Plane {
+    float tyh, tyl, hz, kxh, kyh, kyl, kzh, kzl, q, pf, po, cf, tm, d, c;
+    float wxl, wxh, wyl, wyh, wzl, wzh;
   };
-  float w = 0.0f;
-  // axis x: face above (x, x+1) then face below (x-1, x)
-  if (x + 1 < P.nx) {
-    const float kf = lab ? fk(lme, P.labels[i + sx]) : P.kfx[((long long)x * P.ny + y) * P.nz + z];
-    w = __fadd_rn(w, __fmul_rn(__fsub_rn(th[i + sx], t0), kf));
-  }
-  if (x > 0) {
-    const float kf = lab ? fk(P.labels[i - sx], lme) : P.kfx[((long long)(x - 1) * P.ny + y) * P.nz + z];
-    w = __fsub_rn(w, __fmul_rn(__fsub_rn(t0, th[i - sx]), kf));
-  }
-  if (y + 1 < P.ny) {
-    const float kf = lab ? fk(lme, P.labels[i + sy]) : P.kfy[((long long)x * (P.ny - 1) + y) * P.nz + z];
-    w = __fadd_rn(w, __fmul_rn(__fsub_rn(th[i + sy], t0), kf));
-  }
-  if (y > 0) {
-    const float kf = lab ? fk(P.labels[i - sy], lme) : P.kfy[((long long)x * (P.ny - 1) + (y - 1)) * P.nz + z];
-    w = __fsub_rn(w, __fmul_rn(__fsub_rn(t0, th[i - sy]), kf));
-  }
-  if (z + 1 < P.nz) {
-    const float kf = lab ? fk(lme, P.labels[i + 1]) : P.kfz[((long long)x * P.ny + y) * (P.nz - 1) + z];
-    w = __fadd_rn(w, __fmul_rn(__fsub_rn(th[i + 1], t0), kf));
-  }
-  if (z > 0) {
-    const float kf = lab ? fk(P.labels[i - 1], lme) : P.kfz[((long long)x * P.ny + y) * (P.nz - 1) + (z - 1)];
-    w = __fsub_rn(w, __fmul_rn(__fsub_rn(t0, th[i - 1]), kf));
-  }
-  if (P.dirichlet) {
-    const long long pyz = (long long)P.ny * P.nz, pxz = (long long)P.nx * P.nz, pxy = (long long)P.nx * P.ny;
-    const float* W = P.walls;
-    const float dwall = __fsub_rn(P.theta_wall, t0);
-    // 2 k_edge / dx^2 (pennes.py:414-426); label mode: walls only on the grid's own axes
-    const float wk = lab ? __fmul_rn(__fmul_rn(2.0f, me.x), P.inv_dx2) : 0.f;
-    const bool wx = !lab || (P.wall_axes & 1), wy = !lab || (P.wall_axes & 2), wz = !lab || (P.wall_axes & 4);
-    if (wx && x == 0) w = __fadd_rn(w, __fmul_rn(lab ? wk : W[(long long)y * P.nz + z], dwall));
-    if (wx && x == P.nx - 1) w = __fadd_rn(w, __fmul_rn(lab ? wk : W[pyz + (long long)y * P.nz + z], dwall));
-    if (!lab) W += 2 * pyz;
-    if (wy && y == 0) w = __fadd_rn(w, __fmul_rn(lab ? wk : W[(long long)x * P.nz + z], dwall));
-    if (wy && y == P.ny - 1) w = __fadd_rn(w, __fmul_rn(lab ? wk : W[pxz + (long long)x * P.nz + z], dwall));
-    if (!lab) W += 2 * pxz;
-    if (wz && z == 0) w = __fadd_rn(w, __fmul_rn(lab ? wk : W[(long long)x * P.ny + y], dwall));
-    if (wz && z == P.nz - 1) w = __fadd_rn(w, __fmul_rn(lab ? wk : W[pxy + (long long)x * P.ny + y], dwall));
-  }
-  if (P.q) w = __fadd_rn(w, P.q[i]);
-  if (lab) {
-    if (me.z != 0.0f || P.has_poff) {
-      w = __fsub_rn(w, __fmul_rn(me.z, t0));
-      if (P.has_poff) w = __fsub_rn(w, me.w);
+  // wall planes 2 k_edge / dx^2 (pennes.py:414-426): x lo, x hi, y lo, y hi, z lo, z hi
+  const float* const Wy = P.walls + 2 * sx;
+  const float* const Wz = Wy + 2 * (long long)P.nx * P.nz;
+  auto load = [&](int x) {
+    Plane v;
+    const long long o = (long long)x * sx;
+    const float* t_ = th + o;
+    v.tyh = yhi ? t_[c0 + P.nz] : 0.f;
+    v.tyl = ylo ? t_[c0 - P.nz] : 0.f;
+    v.hz = hlo ? t_[c0 - 1] : (hhi ? t_[c0 + 1] : 0.f);
+    v.kxh = in && x + 1 < P.nx ? (P.kfx + o)[c0] : 0.f;
+    const float* ky = P.kfy + (long long)x * sky;
+    v.kyh = yhi ? ky[cy] : 0.f;
+    v.kyl = ylo ? ky[cy - P.nz] : 0.f;
+    const float* kz = P.kfz + (long long)x * skz;
+    v.kzh = zhi ? kz[cz] : 0.f;
+    v.kzl = hlo ? kz[cz - 1] : 0.f;  // the other lanes take it from the lane below
+    v.q = in && P.q ? (P.q + o)[c0] : 0.f;
+    v.pf = in && P.perf ? (P.perf + o)[c0] : 0.f;
+    v.po = in && P.poff ? (P.poff + o)[c0] : 0.f;
+    v.cf = in ? (P.coeff + o)[c0] : 0.f;
+    v.tm = in ? (thmax + o)[c0] : 0.f;
+    v.d = DOSE && in ? (dose + o)[c0] : 0.f;
+    v.c = DOSE && in ? (dcomp + o)[c0] : 0.f;
+    if (DIR) {
+      const long long oy = (long long)x * P.nz + z, oz = (long long)x * P.ny + y;
+      v.wxl = in && x == 0 ? P.walls[c0] : 0.f;
+      v.wxh = in && x == P.nx - 1 ? P.walls[sx + c0] : 0.f;
+      v.wyl = in && !ylo ? Wy[oy] : 0.f;
+      v.wyh = in && !yhi ? Wy[(long long)P.nx * P.nz + oy] : 0.f;
+      v.wzl = in && !zlo ? Wz[oz] : 0.f;
+      v.wzh = in && !zhi ? Wz[(long long)P.nx * P.ny + oz] : 0.f;
     }
-    w = __fmul_rn(w, me.y);
-  } else {
-    if (P.perf) {
-      w = __fsub_rn(w, __fmul_rn(P.perf[i], t0));
-      if (P.poff) w = __fsub_rn(w, P.poff[i]);
+    return v;
+  };
+  float tp = 0.f, tc = 0.f, tn = 0.f, kxl = 0.f;
+  cgf::pdl_wait();
+  if (in) {
+    const float* t_ = th + (long long)x0 * sx;
+    tc = t_[c0];
+    if (x0 > 0) tp = (t_ - sx)[c0], kxl = (P.kfx + (long long)(x0 - 1) * sx)[c0];
+    if (x0 + 1 < P.nx) tn = (t_ + sx)[c0];
+  }
+  Plane v = load(x0);
+  for (int x = x0; x < x1; ++x) {
+    const long long o = (long long)x * sx;
+    Plane nv = {};
+    float tnn = 0.f;
+    if (x + 1 < x1) {
+      nv = load(x + 1);
+      if (in && x + 2 < P.nx) tnn = (th + (o + 2 * sx))[c0];
     }
-    w = __fmul_rn(w, P.coeff[i]);
-  }
-  const float t1 = __fadd_rn(t0, w);
-  thn[i] = t1;
-  const float tm = thmax[i];
-  thmax[i] = (t1 > tm || t1 != t1) ? t1 : tm;
-  if (P.dose) {
-    const float r_new = cem43_rate_dev(__fadd_rn(t1, P.t_ref));
-    const float r_old = cem43_rate_dev(__fadd_rn(t0, P.t_ref));
-    const float inc = __fmul_rn(__fadd_rn(r_new, r_old), P.half_dt_min);
-    // Kahan: true dose = s - c
-    const float sd = dose[i], c = dcomp[i];
-    const float yk = __fsub_rn(inc, c);
-    const float tk = __fadd_rn(sd, yk);
-    dcomp[i] = __fsub_rn(__fsub_rn(tk, sd), yk);
-    dose[i] = tk;
-  }
-}
-
-// One sub-step on dense per-cell coefficient maps (label media take the
-// streaming kernels below). Block (32, PENNES_ROWS): each warp walks one
-// (x, y) row along z, so accesses along z are coalesced and the coordinates
-// need no 64-bit division; the rows of a block are consecutive in y, so the
-// y-neighbours of most cells are already in L1.
-#define PENNES_ROWS 8
-__global__ void __launch_bounds__(32 * PENNES_ROWS) k_pennes_step(PennesDev P, const float* __restrict__ th,
-                                                                  float* __restrict__ thn, float* thmax, float* dose,
-                                                                  float* dcomp) {
-  __shared__ float4 tab[256];
-  __shared__ float ft_s[CG_PENNES_FTAB * CG_PENNES_FTAB];
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  if (P.labels)
-    for (int i = tid; i < 256; i += 32 * PENNES_ROWS) tab[i] = P.ltab[i];
-  if (P.ftab)
-    for (int i = tid; i < P.nlab * P.nlab; i += 32 * PENNES_ROWS) ft_s[i] = P.ftab[i];
-  __syncthreads();
-  const float* ft = P.ftab ? ft_s : nullptr;
-  const long long nrows = (long long)P.nx * P.ny;
-  for (long long row = (long long)blockIdx.x * PENNES_ROWS + threadIdx.y; row < nrows;
-       row += (long long)gridDim.x * PENNES_ROWS) {
-    const int x = (int)(row / P.ny), y = (int)(row - (long long)x * P.ny);
-    const long long base = row * P.nz;
-    for (int z = threadIdx.x; z < P.nz; z += 32)
-      pennes_cell(P, th, thn, thmax, dose, dcomp, tab, ft, base + z, x, y, z);
+    const float su = __shfl_down_sync(0xffffffffu, tc, 1), sd = __shfl_up_sync(0xffffffffu, tc, 1);
+    const float ku = __shfl_up_sync(0xffffffffu, v.kzh, 1);
+    if (in) {
+      const float t0 = tc, tzh = lane == 31 ? v.hz : su, tzl = lane == 0 ? v.hz : sd, kzl = lane == 0 ? v.kzl : ku;
+      float w = 0.0f;
+      if (x + 1 < P.nx) w = __fadd_rn(w, __fmul_rn(__fsub_rn(tn, t0), v.kxh));
+      if (x > 0) w = __fsub_rn(w, __fmul_rn(__fsub_rn(t0, tp), kxl));
+      if (yhi) w = __fadd_rn(w, __fmul_rn(__fsub_rn(v.tyh, t0), v.kyh));
+      if (ylo) w = __fsub_rn(w, __fmul_rn(__fsub_rn(t0, v.tyl), v.kyl));
+      if (zhi) w = __fadd_rn(w, __fmul_rn(__fsub_rn(tzh, t0), v.kzh));
+      if (zlo) w = __fsub_rn(w, __fmul_rn(__fsub_rn(t0, tzl), kzl));
+      if (DIR) {
+        const float dwall = __fsub_rn(P.theta_wall, t0);
+        if (x == 0) w = __fadd_rn(w, __fmul_rn(v.wxl, dwall));
+        if (x == P.nx - 1) w = __fadd_rn(w, __fmul_rn(v.wxh, dwall));
+        if (!ylo) w = __fadd_rn(w, __fmul_rn(v.wyl, dwall));
+        if (!yhi) w = __fadd_rn(w, __fmul_rn(v.wyh, dwall));
+        if (!zlo) w = __fadd_rn(w, __fmul_rn(v.wzl, dwall));
+        if (!zhi) w = __fadd_rn(w, __fmul_rn(v.wzh, dwall));
+      }
+      if (P.q) w = __fadd_rn(w, v.q);
+      if (P.perf) {
+        w = __fsub_rn(w, __fmul_rn(v.pf, t0));
+        if (P.poff) w = __fsub_rn(w, v.po);
+      }
+      w = __fmul_rn(w, v.cf);
+      const float t1 = __fadd_rn(t0, w);
+      (thn + o)[c0] = t1;
+      (thmax + o)[c0] = (t1 > v.tm || t1 != t1) ? t1 : v.tm;
+      if (DOSE) {
+        const float r_new = cem43_rate_dev(__fadd_rn(t1, P.t_ref));
+        const float r_old = cem43_rate_dev(__fadd_rn(t0, P.t_ref));
+        const float inc = __fmul_rn(__fadd_rn(r_new, r_old), P.half_dt_min);
+        // Kahan: true dose = d - c
+        const float yk = __fsub_rn(inc, v.c);
+        const float tk = __fadd_rn(v.d, yk);
+        (dcomp + o)[c0] = __fsub_rn(__fsub_rn(tk, v.d), yk);
+        (dose + o)[c0] = tk;
+      }
+    }
+    tp = tc, tc = tn, tn = tnn, kxl = v.kxh, v = nv;
   }
 }
 
@@ -190,7 +205,7 @@ __device__ __forceinline__ float cem43_rate_fast(float T) {
 // dose and its compensation for plane x + 1, and temperature/label of plane
 // x + 2 are issued before plane x is computed). FT: face conductances from
 // the material-pair table; DOSE: CEM43 accumulation; DIR: Dirichlet walls.
-// The temperature arithmetic is pennes_cell's, in the same order.
+// The temperature arithmetic is the dense kernel's, in the same order.
 #define PS_Z 32
 #define PS_Y 8
 template <bool FT, bool DOSE, bool DIR>
@@ -202,6 +217,7 @@ __global__ void __launch_bounds__(PS_Z * PS_Y) k_pennes_stream(PennesDev P, int 
   constexpr int TW = PS_Z + 2, TS = (PS_Y + 2) * TW;  // plane tile row width and size
   __shared__ float tpl[2 * TS];
   __shared__ uint8_t lpl[2 * TS];
+  cgf::pdl_trigger();
   const int tz = threadIdx.x, ty = threadIdx.y, tid = ty * PS_Z + tz;
   for (int i = tid; i < 256; i += PS_Z * PS_Y) tab[i] = P.ltab[i];
   if (FT)
@@ -227,6 +243,7 @@ __global__ void __launch_bounds__(PS_Z * PS_Y) k_pennes_stream(PennesDev P, int 
   // registers of plane x: own x-1 / x / x+1 values, halo, per-cell state
   float tp = 0.f, tc = 0.f, tn = 0.f, hyt = 0.f, hzt = 0.f, aq = 0.f, am = 0.f, ad = 0.f, ac = 0.f;
   int lp = 0, lc = 0, ln = 0, hyl = 0, hzl = 0;
+  cgf::pdl_wait();
   if (in) {
     const long long o = x0 * sx;
     const float* t_ = th + o;
@@ -318,7 +335,7 @@ __global__ void __launch_bounds__(PS_Z * PS_Y) k_pennes_stream(PennesDev P, int 
 // z-neighbour inside the pair is a register. Block (PP_Z, PP_Y) covers 2 PP_Z
 // z by PP_Y y; the shared plane tile keeps the pair columns 8-byte aligned
 // (interior from column 2, halo columns 1 and 2 PP_Z + 2). Per cell the
-// arithmetic is pennes_cell's, in the same order.
+// arithmetic is the dense kernel's, in the same order.
 #define PP_Z 16
 #define PP_Y 16
 template <bool FT, bool DOSE, bool DIR>
@@ -330,6 +347,7 @@ __global__ void __launch_bounds__(PP_Z * PP_Y) k_pennes_stream2(PennesDev P, int
   constexpr int TW = 2 * PP_Z + 4, TS = (PP_Y + 2) * TW;  // plane tile row width and size
   __shared__ __align__(16) float tpl[2 * TS];
   __shared__ __align__(16) uint8_t lpl[2 * TS];
+  cgf::pdl_trigger();
   const int tz = threadIdx.x, ty = threadIdx.y, tid = ty * PP_Z + tz;
   for (int i = tid; i < 256; i += PP_Z * PP_Y) tab[i] = P.ltab[i];
   if (FT)
@@ -358,6 +376,7 @@ __global__ void __launch_bounds__(PP_Z * PP_Y) k_pennes_stream2(PennesDev P, int
          ad = {0.f, 0.f}, ac = {0.f, 0.f};
   float hzt = 0.f;
   int lp = 0, lc = 0, ln = 0, hyl = 0, hzl = 0;  // label pairs: low byte = cell z
+  cgf::pdl_wait();
   if (in) {
     const long long o = x0 * sx;
     const float* t_ = th + o;
@@ -469,9 +488,9 @@ template <bool FT, bool DOSE, bool DIR>
 static void launch_stream_k(bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs, const float* th,
                             float* thn, float* thmax, float* dose, float* dcomp) {
   if (pair)
-    k_pennes_stream2<FT, DOSE, DIR><<<g, b, 0, st>>>(P, xs, th, thn, thmax, dose, dcomp);
+    cgf::launch(1, k_pennes_stream2<FT, DOSE, DIR>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
   else
-    k_pennes_stream<FT, DOSE, DIR><<<g, b, 0, st>>>(P, xs, th, thn, thmax, dose, dcomp);
+    cgf::launch(1, k_pennes_stream<FT, DOSE, DIR>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
 }
 
 template <bool FT, bool DOSE>
@@ -495,6 +514,21 @@ static void launch_stream(bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStr
       launch_stream_dir<false, true>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
     else
       launch_stream_dir<false, false>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+  }
+}
+
+static void launch_dense(const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs, const float* th, float* thn,
+                         float* thmax, float* dose, float* dcomp) {
+  if (P.dose) {
+    if (P.dirichlet)
+      cgf::launch(1, k_pennes_dense<true, true>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+    else
+      cgf::launch(1, k_pennes_dense<true, false>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+  } else {
+    if (P.dirichlet)
+      cgf::launch(1, k_pennes_dense<false, true>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+    else
+      cgf::launch(1, k_pennes_dense<false, false>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
   }
 }
 
@@ -722,17 +756,28 @@ static PennesDev make_dev(const cg_pennes* h) {
   return P;
 }
 
+// x planes per block: 8, or 4, or 2 where more would leave an SM with fewer
+// than 3.5 blocks. Sub-step (us) at 2 / 4 / 8 planes: labels 48^3 4.2 / 4.3 /
+// 6.5, 64^3 4.5 / 7.2 / 6.4, 96x96x128 8.6 / 8.3 / 11.9, 128^3 14.2 / 13.4 /
+// 15.0, 256x256x320 155 / 142 / 141; dense 96x96x128 13.8 / 13.4 / 13.9,
+// 101x117x143 20.7 / 19.8 / 19.1, 256x256x320 259 / 231 / 220 (16 planes:
+// 96x96x128 14.4, 256x256x320 149 and 221). Before (8 or 16 planes, plain
+// launches): labels 48^3 9.1, 96x96x128 12.3, 256x256x320 149.
+static int pennes_planes(long long tiles, int nx) {
+  int xs = 8;
+  while (xs > 2 && tiles * ((nx + xs - 1) / xs) * 2 < 7LL * cgf::sm_count()) xs /= 2;
+  return xs;
+}
+
 extern "C" int cg_pennes_run(cg_pennes* h, int n_sub) {
   CG_REQUIRE(h, "null handle");
   CG_REQUIRE(h->has_coef && h->has_state, "set coefficients and state before running");
   CG_REQUIRE(n_sub >= 0, "n_sub must be >= 0");
   const PennesDev P = make_dev(h);
-  const dim3 block(32, PENNES_ROWS);
-  long long blocks = ((long long)h->cfg.nx * h->cfg.ny + PENNES_ROWS - 1) / PENNES_ROWS;
-  if (blocks > 152 * 64) blocks = 152 * 64;
-  // label mode streams along x; z-pairs when nz is even (CG_PENNES_PAIR=0
-  // keeps single cells). x planes per block: 16, or 8 when 16 leaves fewer
-  // than four waves of 4 resident blocks on every SM (CG_PENNES_XS pins it).
+  // Both modes stream along x; label media take z-pairs when nz is even
+  // (CG_PENNES_PAIR=0 keeps single cells). x planes per block (CG_PENNES_XS
+  // pins it): pennes_planes. Each sub-step is launched programmatically: its
+  // blocks fill their tables while the step before drains.
   static const int xs_pin = [] {
     const char* e = getenv("CG_PENNES_XS");
     return e ? atoi(e) : 0;
@@ -741,19 +786,22 @@ extern "C" int cg_pennes_run(cg_pennes* h, int n_sub) {
     const char* e = getenv("CG_PENNES_PAIR");
     return !(e && atoi(e) == 0);
   }();
-  const bool pair = pair_ok && h->cfg.nz % 2 == 0;
-  const int tzc = pair ? 2 * PP_Z : PS_Z, tyc = pair ? PP_Y : PS_Y;
-  const dim3 sblock(pair ? PP_Z : PS_Z, tyc);
+  const bool pair = P.labels && pair_ok && h->cfg.nz % 2 == 0;
+  const int tzc = pair ? 2 * PP_Z : (P.labels ? PS_Z : 32), tyc = pair ? PP_Y : (P.labels ? PS_Y : PD_Y);
+  const dim3 sblock(pair ? PP_Z : tzc, tyc);
   const long long tiles_zy = (long long)((h->cfg.nz + tzc - 1) / tzc) * ((h->cfg.ny + tyc - 1) / tyc);
-  const int xs = xs_pin > 0 ? xs_pin : (tiles_zy * ((h->cfg.nx + 15) / 16) >= 4LL * 4 * cgf::sm_count() ? 16 : 8);
+  const int xs = xs_pin > 0 ? xs_pin : pennes_planes(tiles_zy, h->cfg.nx);
   const dim3 sgrid((unsigned)((h->cfg.nz + tzc - 1) / tzc), (unsigned)((h->cfg.ny + tyc - 1) / tyc),
                    (unsigned)((h->cfg.nx + xs - 1) / xs));
+  // dense maps: z-y tiles along one grid dimension (any ny), as many x planes
+  // a block as keep the other within its limit
+  const int xd = xs > (h->cfg.nx + 65534) / 65535 ? xs : (h->cfg.nx + 65534) / 65535;
+  const dim3 dgrid((unsigned)tiles_zy, (unsigned)((h->cfg.nx + xd - 1) / xd));
   for (int i = 0; i < n_sub; ++i) {
     if (P.labels)
       launch_stream(pair, P, sgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
     else
-      k_pennes_step<<<(unsigned)blocks, block, 0, h->stream>>>(P, h->th[h->cur], h->th[1 - h->cur], h->thmax,
-                                                               h->dose, h->dcomp);
+      launch_dense(P, dgrid, sblock, h->stream, xd, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
     h->cur = 1 - h->cur;
   }
   CG_CUDA_TRY(cudaGetLastError());
