@@ -39,12 +39,16 @@ bool fast_xpass(int mode, const Dims& d, const Tables& t, float kcoef, float inv
   }
 }
 
-int fast_prepare_yx() {
-#define SET(n) \
-  if (yx_prepare<n>()) return -1;
-  CG_FAST_XYSIZES(SET)
-#undef SET
-  return 0;
+int fast_prepare_yx(int n) {
+  switch (n) {
+#define CASE(k) \
+  case k:       \
+    return yx_prepare<k>();
+    CG_FAST_XYSIZES(CASE)
+#undef CASE
+    default:
+      return 0;
+  }
 }
 
 bool fast_xy_has(int n) {

@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
     });
   };
   auto kappa = [&](int k) { return sinc_a2(kcoef * (kxs[N + k] + kyz2)) * invN; };
-  if constexpr (MODE == X_FWD || MODE == X_INV) {
-    load(S0);
+  if constexpr (MODE == X_FWD || MODE == X_INV) {  // S0 <- (I)FFT(S1); S1 may be S0
+    load(S1);
     fft2<A, B, MODE == X_INV>(v, w, s, tw, exf);
     if (valid && s < A) static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;

@@ -203,19 +203,29 @@ bool fast_zpass_p_tma(const Dims& d, const Tables& t, const MediumDev& m, const 
   }
 }
 
-int fast_prepare_z() {
-#define SET(n) \
-  if (zt_prepare<n>()) return -1;
-  CG_FAST_SIZES(SET)
-#undef SET
-#define SETP(n) \
-  if (zp_prepare<n>()) return -1;
-  CG_FAST_ZSIZES(SETP)
-#undef SETP
-  return 0;
+static int fast_prepare_z(int n) {
+  switch (n) {
+#define CASE(k) \
+  case k:       \
+    if (zt_prepare<k>()) return -1; \
+    break;
+    CG_FAST_SIZES(CASE)
+#undef CASE
+    default:
+      break;
+  }
+  switch (n) {
+#define CASE(k) \
+  case k:       \
+    return zp_prepare<k>();
+    CG_FAST_ZSIZES(CASE)
+#undef CASE
+    default:
+      return 0;
+  }
 }
 
-int fast_prepare_yx();
+int fast_prepare_yx(int n);
 
 bool fast_has(int n) {
   switch (n) {
@@ -228,4 +238,6 @@ bool fast_has(int n) {
   }
 }
 
-int fast_prepare() { return (fast_prepare_yx() == 0 && fast_prepare_z() == 0) ? 0 : -1; }
+int fast_prepare(const Dims& d) {
+  return (fast_prepare_yx(d.nx) == 0 && fast_prepare_yx(d.ny) == 0 && fast_prepare_z(d.nz) == 0) ? 0 : -1;
+}

@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(CG_THREADS) k_xpass(int mode, Dims d, AxisPlan
     int ky = (int)(col - (long long)kz * d.ny);
     kyz2 = t.ky2[ky] + t.kz2[kz];
   }
-  if (mode == X_FWD || mode == X_INV) {
-    x_load(b0, S0, col0, ncols, ncol, N);
+  if (mode == X_FWD || mode == X_INV) {  // S0 <- (I)FFT(S1); S1 may be S0
+    x_load(b0, S1, col0, ncols, ncol, N);
     __syncthreads();
     float2* r = (mode == X_FWD) ? tile_fft<false>(b0, b1, XLD, tw, pl, c, g, G) : tile_fft<true>(b0, b1, XLD, tw, pl, c, g, G);
     x_store(S0, r, col0, ncols, ncol, N);
@@ -938,7 +938,7 @@ extern "C" int cg_solver_create(const cg_solver_config* cfg, cg_solver** out) {
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_zpass_u);
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_zpass_p);
   if (e == cudaSuccess) e = allow_max_smem(finalize_kernel(s->nh));
-  if (e == cudaSuccess && fast_prepare() != 0) e = cudaErrorInvalidValue;
+  if (e == cudaSuccess && fast_prepare(s->d) != 0) e = cudaErrorInvalidValue;
   if (e != cudaSuccess) {
     cg_set_error("solver set-up: %s", cudaGetErrorString(e));
     solver_free(s);
@@ -1787,7 +1787,7 @@ extern "C" int cg_fft3d_create(int nx, int ny, int nz, int batch, cg_fft3d** out
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_ypass);
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_xpass);
   if (e == cudaSuccess) e = allow_max_smem((const void*)k_zpass_p);
-  if (e == cudaSuccess && fast_prepare() != 0) e = cudaErrorInvalidValue;
+  if (e == cudaSuccess && fast_prepare(f->d) != 0) e = cudaErrorInvalidValue;
   if (e == cudaSuccess) e = cudaStreamSynchronize(f->stream);
   if (e != cudaSuccess) {
     cg_set_error("fft set-up: %s", cudaGetErrorString(e));
@@ -1813,6 +1813,20 @@ static Tables fft_tables(const cg_fft3d* f) {
   return t;
 }
 
+// Whether a transform can work on the caller's buffer itself: memory of the
+// current device, aligned for the passes' accesses. Host buffers and others go
+// through the handle's staging arrays.
+static bool direct(const void* p, size_t align) {
+  int dev = 0;
+  cudaPointerAttributes at;
+  if (((uintptr_t)p & (align - 1)) != 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return (at.type == cudaMemoryTypeDevice && at.device == dev) || at.type == cudaMemoryTypeManaged;
+}
+
 extern "C" int cg_fft3d_forward(cg_fft3d* f, const float* in, float* out_spec) {
   CG_REQUIRE(f && in && out_spec, "null argument");
   const Dims d = f->d;
@@ -1824,18 +1838,26 @@ extern "C" int cg_fft3d_forward(cg_fft3d* f, const float* in, float* out_spec) {
   RecordDev rd;
   memset(&rd, 0, sizeof(rd));
   rd.spp = 1;
-  CG_CUDA_TRY(cudaMemcpyAsync(f->real, in, sizeof(float) * f->B * d.ncell, cudaMemcpyDefault, f->stream));
+  const size_t in_bytes = sizeof(float) * f->B * d.ncell, out_bytes = sizeof(float2) * f->B * d.nspec;
+  // the z-pass reads the real rows while it writes the spectrum: buffers that
+  // overlap are staged
+  const uintptr_t ia = (uintptr_t)in, oa = (uintptr_t)out_spec;
+  const bool apart = ia + in_bytes <= oa || oa + out_bytes <= ia;
+  const bool in_ok = apart && direct(in, 4), out_ok = direct(out_spec, 16);
+  float* real = in_ok ? const_cast<float*>(in) : f->real;
+  float2* spec = out_ok ? (float2*)out_spec : f->spec;
+  if (!in_ok) CG_CUDA_TRY(cudaMemcpyAsync(real, in, in_bytes, cudaMemcpyDefault, f->stream));
   const dim3 gy((unsigned)((d.nx * (long long)d.nzh + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gx((unsigned)(((long long)d.nzh * d.ny + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gz((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), f->B);
-  if (!fast_zpass_half(false, d, t, m, f->real, f->spec, f->B, f->stream))
-    k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(0, d, f->pz, t, m, sd, rd, nullptr, 0, 0, f->real, f->spec);
-  if (!fast_ypass(Y_FWD, d, t, f->spec, nullptr, nullptr, f->B, f->stream))
-    k_ypass<<<gy, CG_THREADS, f->smem_y, f->stream>>>(Y_FWD, d, f->py, t, f->spec, nullptr, nullptr);
-  if (!fast_xpass(X_FWD, d, t, 0.f, 1.f, f->spec, nullptr, nullptr, f->B, f->stream))
-    k_xpass<<<gx, CG_THREADS, f->smem_x, f->stream>>>(X_FWD, d, f->px, t, 0.f, 1.f, f->spec, nullptr, nullptr);
+  if (!fast_zpass_half(false, d, t, m, real, spec, f->B, f->stream))
+    k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(0, d, f->pz, t, m, sd, rd, nullptr, 0, 0, real, spec);
+  if (!fast_ypass(Y_FWD, d, t, spec, nullptr, nullptr, f->B, f->stream))
+    k_ypass<<<gy, CG_THREADS, f->smem_y, f->stream>>>(Y_FWD, d, f->py, t, spec, nullptr, nullptr);
+  if (!fast_xpass(X_FWD, d, t, 0.f, 1.f, spec, spec, nullptr, f->B, f->stream))
+    k_xpass<<<gx, CG_THREADS, f->smem_x, f->stream>>>(X_FWD, d, f->px, t, 0.f, 1.f, spec, spec, nullptr);
   CG_CUDA_TRY(cudaGetLastError());
-  CG_CUDA_TRY(cudaMemcpyAsync(out_spec, f->spec, sizeof(float2) * f->B * d.nspec, cudaMemcpyDefault, f->stream));
+  if (!out_ok) CG_CUDA_TRY(cudaMemcpyAsync(out_spec, spec, out_bytes, cudaMemcpyDefault, f->stream));
   CG_CUDA_TRY(cudaStreamSynchronize(f->stream));
   return CG_OK;
 }
@@ -1851,18 +1873,25 @@ extern "C" int cg_fft3d_inverse(cg_fft3d* f, const float* in_spec, float* out) {
   RecordDev rd;
   memset(&rd, 0, sizeof(rd));
   rd.spp = 1;
-  CG_CUDA_TRY(cudaMemcpyAsync(f->spec, in_spec, sizeof(float2) * f->B * d.nspec, cudaMemcpyDefault, f->stream));
+  // the x-pass takes the caller's spectrum to the handle's (which it leaves as
+  // it is), the z-pass writes the caller's rows; by then the spectrum is read
+  const bool in_ok = direct(in_spec, 8), out_ok = direct(out, 4);
+  float2* src = in_ok ? (float2*)const_cast<float*>(in_spec) : f->spec;
+  float* real = out_ok ? out : f->real;
+  if (!in_ok)
+    CG_CUDA_TRY(cudaMemcpyAsync(src, in_spec, sizeof(float2) * f->B * d.nspec, cudaMemcpyDefault, f->stream));
   const dim3 gy((unsigned)((d.nx * (long long)d.nzh + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gx((unsigned)(((long long)d.nzh * d.ny + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gz((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), f->B);
-  if (!fast_xpass(X_INV, d, t, 0.f, 1.f, f->spec, nullptr, nullptr, f->B, f->stream))
-    k_xpass<<<gx, CG_THREADS, f->smem_x, f->stream>>>(X_INV, d, f->px, t, 0.f, 1.f, f->spec, nullptr, nullptr);
+  if (!fast_xpass(X_INV, d, t, 0.f, 1.f, f->spec, src, nullptr, f->B, f->stream))
+    k_xpass<<<gx, CG_THREADS, f->smem_x, f->stream>>>(X_INV, d, f->px, t, 0.f, 1.f, f->spec, src, nullptr);
   if (!fast_ypass(Y_INV, d, t, f->spec, nullptr, nullptr, f->B, f->stream))
     k_ypass<<<gy, CG_THREADS, f->smem_y, f->stream>>>(Y_INV, d, f->py, t, f->spec, nullptr, nullptr);
-  if (!fast_zpass_half(true, d, t, m, f->real, f->spec, f->B, f->stream))
-    k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(2, d, f->pz, t, m, sd, rd, nullptr, 0, 0, f->real, f->spec);
+  if (!fast_zpass_half(true, d, t, m, real, f->spec, f->B, f->stream))
+    k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(2, d, f->pz, t, m, sd, rd, nullptr, 0, 0, real, f->spec);
   CG_CUDA_TRY(cudaGetLastError());
-  CG_CUDA_TRY(cudaMemcpyAsync(out, f->real, sizeof(float) * f->B * d.ncell, cudaMemcpyDefault, f->stream));
+  if (!out_ok)
+    CG_CUDA_TRY(cudaMemcpyAsync(out, real, sizeof(float) * f->B * d.ncell, cudaMemcpyDefault, f->stream));
   CG_CUDA_TRY(cudaStreamSynchronize(f->stream));
   return CG_OK;
 }
@@ -1958,7 +1987,7 @@ extern "C" int cg_fft3d_forward_noalloc(int nx, int ny, int nz, int batch, const
   const dim3 gz((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), batch);
   k_zpass_p<<<gz, CG_THREADS, sz, st>>>(0, d, pz, t, m, sd, rd, nullptr, 0, 0, (float*)in_dev, spec);
   k_ypass<<<gy, CG_THREADS, sy, st>>>(Y_FWD, d, py, t, spec, nullptr, nullptr);
-  k_xpass<<<gx, CG_THREADS, sx, st>>>(X_FWD, d, px, t, 0.f, 1.f, spec, nullptr, nullptr);
+  k_xpass<<<gx, CG_THREADS, sx, st>>>(X_FWD, d, px, t, 0.f, 1.f, spec, spec, nullptr);
   CG_CUDA_TRY(cudaGetLastError());
   return CG_OK;
 }

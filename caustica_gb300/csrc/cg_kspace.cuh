@@ -110,7 +110,9 @@ __device__ __forceinline__ float4 cell_coef(const MediumDev& m, long long i) {
 // (returns false otherwise; the caller then uses the generic kernel).
 bool fast_has(int n);
 bool fast_xy_has(int n);  // n in CG_FAST_XYSIZES
-int fast_prepare();  // lift the dynamic shared-memory limits (once per device)
+// lift the dynamic shared-memory limits of the grid's own kernels (setting one
+// loads the kernel, so not of every length)
+int fast_prepare(const Dims& d);
 // fused transverse passes (cg_fused_xy.cu): 1 when they apply to the grid
 int fused_xy_supported(const Dims& d);
 bool fused_xy(bool grad, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1,
