@@ -238,13 +238,15 @@ constexpr int ct_even_split(int n) {
 constexpr int ct_tpp(int m) { return m <= 8 ? 8 : (m <= 16 ? 16 : (m + 3) / 4 * 4); }
 
 // Pencil split of the size-specialised passes: (A, B) with B threads
-// holding A values on input and A threads holding B values on output.
-// 16 x (<= 16) where the length allows it (aligned 16-value runs in global
-// memory), else the most even split: no thread holds more than 20 values up
-// to 400 points except on 243, 250, 375 and 384 (27, 25, 25, 24).
+// holding A values on input and A threads holding B values on output. The
+// most even split: fewest instructions for the warp that waits on its
+// longest codelet, and up to 400 points no thread holds more than 20 values
+// except on 243, 250, 375 and 384 (27, 25, 25, 24). Against 16 x (N / 16)
+// for the multiples of 16: 64^3 33 -> 29 us a step, 96x96x128 54 -> 52,
+// 32^3 25 -> 20.
 template <int N>
 struct PSplit {
-  static constexpr int A = N % 16 == 0 && N / 16 <= 16 ? N / 16 : ct_even_split(N), B = N / A;
+  static constexpr int A = ct_even_split(N), B = N / A;
   static constexpr int TPP = ct_tpp(A > B ? A : B);  // threads per pencil
 };
 template <>
@@ -254,6 +256,16 @@ struct PSplit<512> {
 template <>
 struct PSplit<640> {
   static constexpr int A = 32, B = 20, TPP = 32;
+};
+
+// The split of the y-passes, whose threads read and write runs of a row: 16 x
+// (N / 16) from 80 points on, for whole lines (Y_INV_GRAD on 96x96x128 9.8 us
+// against 11.9 for 8 x 12), the most even one below (32^3 6.4 against 7.8).
+template <int N>
+struct YSplit {
+  static constexpr bool LINES = N % 16 == 0 && N > 64 && N <= 256;
+  static constexpr int A = LINES ? N / 16 : PSplit<N>::A, B = N / A;
+  static constexpr int TPP = ct_tpp(A > B ? A : B);
 };
 
 // Odd leading dimension >= n (bank-conflict-free strided access).

@@ -51,6 +51,7 @@
 
 using cgf::ColEx;
 using cgf::PSplit;
+using cgf::YSplit;
 using cgf::RowEx;
 using cgf::fft2;
 using cgf::static_for;
@@ -61,7 +62,7 @@ using cgf::static_for;
 // against 309 / 290 us, 320^3 139 / 198 against 161 / 158).
 template <int N>
 struct YT {
-  static constexpr int TPP = PSplit<N>::TPP, YP = TPP < 16 ? 2 * CG_YP : (TPP > 16 && TPP < 32 ? CG_YP20 : CG_YP);
+  static constexpr int TPP = YSplit<N>::TPP, YP = TPP < 16 ? 2 * CG_YP : (TPP > 16 && TPP < 32 ? CG_YP20 : CG_YP);
   static constexpr int THREADS = TPP * YP;
   static constexpr int MINB = TPP <= 16 ? CG_FAST_MINB_Y : (TPP < 28 ? CG_FAST_MINB_Y20 : 4);
 };
@@ -81,7 +82,7 @@ template <int N, int MODE>
 __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, Tables t, float2* __restrict__ S0,
                                                                         float2* __restrict__ S1,
                                                                         float2* __restrict__ S2) {
-  constexpr int A = PSplit<N>::A, B = PSplit<N>::B, TPP = PSplit<N>::TPP;
+  constexpr int A = YSplit<N>::A, B = YSplit<N>::B, TPP = YSplit<N>::TPP;
   using Ex = RowEx<A, B, (32 % TPP == 0)>;  // pencil-local exchange: warp barriers
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
 // twiddles | exchange | (x: a parked spectrum tile, k_x, k_x^2)
 template <int N>
 static size_t smem_y() {
-  return sizeof(float2) * (N + YT<N>::YP * RowEx<PSplit<N>::A, PSplit<N>::B>::SLAB);
+  return sizeof(float2) * (N + YT<N>::YP * RowEx<YSplit<N>::A, YSplit<N>::B>::SLAB);
 }
 template <int N>
 static size_t smem_x() {
