@@ -53,6 +53,7 @@ struct cg_solver {
   int* ztma_err = nullptr;
   int ztma = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one period, record off/on
+  int plain[2] = {0, 0};  // a short run went out as plain launches before there was a graph
   // phasors of the last finalize, [B][nh][nrec], kept for device post-processing
   float2* ph = nullptr;
   int ph_valid = 0;
