@@ -11,7 +11,24 @@ template <int N>
 bool yx_launch_x(int mode, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1,
                  float2* S2, int batch, cudaStream_t st);
 template <int N>
+bool plane_launch(bool div, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1,
+                  float2* S2, int batch, cudaStream_t st);
+template <int N>
 int yx_prepare();
+
+bool fast_plane(bool div, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1, float2* S2,
+                int batch, cudaStream_t st) {
+  if (d.nx != 1) return false;
+  switch (d.ny) {
+#define CASE(n) \
+  case n:       \
+    return plane_launch<n>(div, d, t, kcoef, invN, S0, S1, S2, batch, st);
+    CG_FAST_XYSIZES(CASE)
+#undef CASE
+    default:
+      return false;
+  }
+}
 
 bool fast_ypass(int mode, const Dims& d, const Tables& t, float2* S0, float2* S1, float2* S2, int batch,
                 cudaStream_t st) {

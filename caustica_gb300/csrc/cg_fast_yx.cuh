@@ -149,6 +149,99 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
   }
 }
 
+// The transverse chain of a grid of one x plane (2-D), where the x-transforms
+// are the identity and k_x = 0: Y_FWD, X_GRAD, Y_INV_GRAD in one kernel
+// (DIV = false: S0 <- IFFT(i ky q), S2 <- IFFT(q), S1 <- 0 q, q = kappa/N
+// FFT(S0)) or Y_FWD_DIV, X_DIV, Y_INV (S0 <- IFFT(kappa/N (i ky FFT(S0) +
+// FFT(S2 + 0 S1)))). The zero multiples carry a non-finite u_x or p over, as
+// the products with k_x = 0 do. Bound: launch latency (a 135x192 step takes
+// 34 us in eight launches, the arithmetic of one fits in two); four launches a
+// step take 17 us. Rows as in the y-pass.
+template <int N, bool DIV>
+__global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, float kcoef, float invN,
+                                                              float2* __restrict__ S0, float2* __restrict__ S1,
+                                                              float2* __restrict__ S2) {
+  constexpr int A = YSplit<N>::A, B = YSplit<N>::B, TPP = YSplit<N>::TPP;
+  using ExF = RowEx<A, B, (32 % TPP == 0)>;
+  using ExI = RowEx<B, A, (32 % TPP == 0)>;
+  constexpr int SLAB = ExF::SLAB > ExI::SLAB ? ExF::SLAB : ExI::SLAB;
+  extern __shared__ float2 sm[];
+  cgf::pdl_trigger();
+  float2* tw = sm;       // (A, B) order
+  float2* twi = sm + N;  // (B, A) order
+  cgf::fill_twt<A, B>(tw, t.twy);
+  cgf::fill_twt<B, A>(twi, t.twy);
+  cgf::pdl_wait();
+  const int s = threadIdx.x % TPP, p = threadIdx.x / TPP;
+  const ExF exf{sm + 2 * N + p * SLAB};
+  const ExI exi{sm + 2 * N + p * SLAB};
+  const int row = blockIdx.x * YT<N>::YP + p;  // kz
+  const bool valid = row < d.nzh;
+  const long long off = (long long)blockIdx.y * d.nspec + (long long)row * N;
+  const float kz2 = valid ? t.kz2[row] : 0.f;
+  __syncthreads();
+  float2 v[A], w[B], z[A];
+  auto load = [&](const float2* src) {
+    static_for<0, A>([&](auto ai) {
+      constexpr int a = decltype(ai)::value;
+      v[a] = (valid && s < B) ? src[off + s + B * a] : make_float2(0.f, 0.f);
+    });
+  };
+  auto store_z = [&](float2* dst) {
+    if (valid && s < B) static_for<0, A>([&](auto ai) {
+      constexpr int a = decltype(ai)::value;
+      dst[off + s + B * a] = z[a];
+    });
+  };
+  auto kappa = [&](int k) { return sinc_a2(kcoef * (t.ky2[k] + kz2)) * invN; };
+  if constexpr (!DIV) {
+    load(S0);
+    fft2<A, B, false>(v, w, s, tw, exf);
+    float2 g[B];
+    static_for<0, B>([&](auto bi) {
+      constexpr int b = decltype(bi)::value;
+      const int k = (s < A) ? s + A * b : 0;
+      w[b] = c_scale(w[b], kappa(k));
+      g[b] = c_muli(c_scale(w[b], t.ky[k]));
+    });
+    fft2<B, A, true>(g, z, s, twi, exi);
+    store_z(S0);
+    fft2<B, A, true>(w, z, s, twi, exi);
+    store_z(S2);
+    static_for<0, A>([&](auto ai) { z[decltype(ai)::value] = c_scale(z[decltype(ai)::value], 0.f); });
+    store_z(S1);
+  } else {
+    load(S0);
+    fft2<A, B, false>(v, w, s, tw, exf);
+    float2 h[B];
+    static_for<0, B>([&](auto bi) {
+      constexpr int b = decltype(bi)::value;
+      const int k = (s < A) ? s + A * b : 0;
+      h[b] = c_muli(c_scale(w[b], t.ky[k]));
+    });
+    load(S2);
+    static_for<0, A>([&](auto ai) {
+      constexpr int a = decltype(ai)::value;
+      if (valid && s < B) v[a] = c_add(v[a], c_scale(S1[off + s + B * a], 0.f));
+    });
+    fft2<A, B, false>(v, w, s, tw, exf);
+    static_for<0, B>([&](auto bi) {
+      constexpr int b = decltype(bi)::value;
+      const int k = (s < A) ? s + A * b : 0;
+      w[b] = c_scale(c_add(w[b], h[b]), kappa(k));
+    });
+    fft2<B, A, true>(w, z, s, twi, exi);
+    store_z(S0);
+  }
+}
+
+template <int N>
+static size_t smem_plane() {
+  using F = RowEx<YSplit<N>::A, YSplit<N>::B>;
+  using I = RowEx<YSplit<N>::B, YSplit<N>::A>;
+  return sizeof(float2) * (2 * N + YT<N>::YP * (F::SLAB > I::SLAB ? F::SLAB : I::SLAB));
+}
+
 template <int N, int MODE>
 __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Dims d, Tables t, float kcoef, float invN,
                                                                         float2* __restrict__ S0,
@@ -310,6 +403,17 @@ bool yx_launch_x(int mode, const Dims& d, const Tables& t, float kcoef, float in
   return true;
 }
 
+template <int N>
+bool plane_launch(bool div, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1,
+                  float2* S2, int batch, cudaStream_t st) {
+  const dim3 grid((unsigned)((d.nzh + YT<N>::YP - 1) / YT<N>::YP), batch);
+  if (div)
+    cgf::launch(d.pdl, kf_plane<N, true>, grid, dim3(YT<N>::THREADS), smem_plane<N>(), st, d, t, kcoef, invN, S0, S1, S2);
+  else
+    cgf::launch(d.pdl, kf_plane<N, false>, grid, dim3(YT<N>::THREADS), smem_plane<N>(), st, d, t, kcoef, invN, S0, S1, S2);
+  return true;
+}
+
 template <int N, int M>
 static int allow_yx() {
   const int sy = (int)smem_y<N>(), sx = (int)smem_x<N>();
@@ -321,6 +425,10 @@ static int allow_yx() {
 // Y_* and X_* modes are both 0..3
 template <int N>
 int yx_prepare() {
+  const int sp = (int)smem_plane<N>();
+  if (cudaFuncSetAttribute(kf_plane<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp) != cudaSuccess ||
+      cudaFuncSetAttribute(kf_plane<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp) != cudaSuccess)
+    return -1;
   return (allow_yx<N, 0>() || allow_yx<N, 1>() || allow_yx<N, 2>() || allow_yx<N, 3>()) ? -1 : 0;
 }
 
@@ -328,4 +436,6 @@ int yx_prepare() {
   template bool yx_launch_y<n>(int, const Dims&, const Tables&, float2*, float2*, float2*, int, cudaStream_t); \
   template bool yx_launch_x<n>(int, const Dims&, const Tables&, float, float, float2*, float2*, float2*, int,   \
                                cudaStream_t);                                                                  \
+  template bool plane_launch<n>(bool, const Dims&, const Tables&, float, float, float2*, float2*, float2*, int,   \
+                                cudaStream_t);                                                                 \
   template int yx_prepare<n>();

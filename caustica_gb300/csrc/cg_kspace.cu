@@ -1238,14 +1238,15 @@ static int launch_step(cg_solver* s, int n_local, int record, EvLog* log = nullp
     if (log) log->mark(sl, st);
   };
   const bool fx = s->fused_xy != 0;
-  if (fx) {
-    mark(0);
+  mark(0);
+  if (fast_plane(false, d, t, (float)s->kcoef, s->invN, s->S0, s->S1, s->S2, B, st)) {
+    // a grid of one x plane: the whole chain in that launch
+  } else if (fx) {
     if (!fused_xy(true, d, t, (float)s->kcoef, s->invN, s->S0, s->S1, s->S2, B, st)) {
       cg_set_error("fused transverse pass launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       return CG_ERR_CUDA;
     }
   } else {
-    mark(0);
     if (!fast_ypass(Y_FWD, d, t, s->S0, s->S1, s->S2, B, st))
       k_ypass<<<gy, CG_THREADS, s->smem_y, st>>>(Y_FWD, d, s->py, t, s->S0, s->S1, s->S2);
     mark(1);
@@ -1260,14 +1261,14 @@ static int launch_step(cg_solver* s, int n_local, int record, EvLog* log = nullp
   if (!(zt && fast_zpass_u_tma(d, t, m, s->u, s->S0, s->S1, s->S2, B, st, s->ztma_host)) &&
       !fast_zpass_u(d, t, m, s->u, s->S0, s->S1, s->S2, B, st, s->zpers != 0))
     k_zpass_u<<<gz, CG_THREADS, s->smem_z, st>>>(d, s->pz, t, m, s->u, s->S0, s->S1, s->S2);
-  if (fx) {
-    mark(4);
+  mark(4);
+  if (fast_plane(true, d, t, (float)s->kcoef, s->invN, s->S0, s->S1, s->S2, B, st)) {
+  } else if (fx) {
     if (!fused_xy(false, d, t, (float)s->kcoef, s->invN, s->S0, s->S1, s->S2, B, st)) {
       cg_set_error("fused transverse pass launch failed: %s", cudaGetErrorString(cudaGetLastError()));
       return CG_ERR_CUDA;
     }
   } else {
-    mark(4);
     if (!fast_ypass(Y_FWD_DIV, d, t, s->S0, s->S1, s->S2, B, st))
       k_ypass<<<gy, CG_THREADS, s->smem_y, st>>>(Y_FWD_DIV, d, s->py, t, s->S0, s->S1, s->S2);
     mark(5);
@@ -1475,7 +1476,7 @@ extern "C" int cg_solver_info(const cg_solver* s, long long* out /* 8 */) {
   out[4] = (long long)s->smem_x;
   out[5] = (long long)s->smem_z;
   out[6] = s->B;
-  out[7] = s->slabs > 1 ? 2 + 6 * s->slabs : (s->fused_xy ? 4 : 8);  // kernel launches per step
+  out[7] = s->slabs > 1 ? 2 + 6 * s->slabs : (s->fused_xy ? 4 : 8);  // passes per step
   return CG_OK;
 }
 

@@ -121,6 +121,10 @@ bool fast_ypass(int mode, const Dims& d, const Tables& t, float2* S0, float2* S1
                 cudaStream_t st);
 bool fast_xpass(int mode, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1,
                 float2* S2, int batch, cudaStream_t st);
+// the gradient or divergence transverse chain of a grid of one x plane in one
+// launch; false when nx > 1 or ny has no size-specialised kernel
+bool fast_plane(bool div, const Dims& d, const Tables& t, float kcoef, float invN, float2* S0, float2* S1, float2* S2,
+                int batch, cudaStream_t st);
 // persistent = false keeps the one-tile-per-CTA z kernels (autotuner choice)
 bool fast_zpass_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
                   int batch, cudaStream_t st, bool persistent = true);
