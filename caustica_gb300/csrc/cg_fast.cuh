@@ -400,6 +400,25 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const void* map, unsigned
       : "memory");
 }
 
+// Contiguous copies between global and shared memory (16-byte aligned, sizes a
+// multiple of 16): a load counted on bar, a store as one bulk group of the
+// issuing thread, and the waits for its groups to have read shared memory or
+// to be complete.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, unsigned bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(smem_addr(src)),
+               "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
 // A value that this pass reads once, kept out of the L1 and in program order.
 __device__ __forceinline__ float2 ld_once(const float2* p) {
   float2 v;

@@ -28,13 +28,6 @@
 #ifndef CG_FAST_MINB_XG
 #define CG_FAST_MINB_XG CG_FAST_MINB_X
 #endif
-// and of the longer splits (20 and more threads per pencil)
-#ifndef CG_FAST_MINB_X20
-#define CG_FAST_MINB_X20 3
-#endif
-#ifndef CG_FAST_MINB_Y20
-#define CG_FAST_MINB_Y20 5
-#endif
 #ifndef CG_XP20
 #define CG_XP20 8
 #endif
@@ -58,19 +51,24 @@ using cgf::static_for;
 
 // Threads and resident CTAs per SM of the y- and x-pass CTAs for length N.
 // Splits with more than 16 threads a pencil take 8 columns per x-CTA, three
-// CTAs to an SM (16 columns, one or two CTAs: 400^3 X_GRAD / X_DIV 353 / 342
-// against 309 / 290 us, 320^3 139 / 198 against 161 / 158).
+// CTAs to an SM, or four where no thread holds more than 16 and 20 values
+// (X_GRAD / X_DIV us with four / three: 216^3 57 / 55 against 66 / 64, 320^3
+// 155 / 166 against 176 / 166, 400^3 323 / 333 against 297 / 302; with two,
+// 400^3 348 / 345), and five y-CTAs, or six up to 34 values (Y_INV_GRAD /
+// Y_FWD_DIV with six / five: 288^3 106 / 109 against 107 / 129, 320^3 146 / 144
+// against 129 / 133).
 template <int N>
 struct YT {
   static constexpr int TPP = YSplit<N>::TPP, YP = TPP < 16 ? 2 * CG_YP : (TPP > 16 && TPP < 32 ? CG_YP20 : CG_YP);
   static constexpr int THREADS = TPP * YP;
-  static constexpr int MINB = TPP <= 16 ? CG_FAST_MINB_Y : (TPP < 28 ? CG_FAST_MINB_Y20 : 4);
+  static constexpr int SUM = YSplit<N>::A + YSplit<N>::B;
+  static constexpr int MINB = TPP <= 16 ? CG_FAST_MINB_Y : (TPP < 28 ? (SUM <= 34 ? 6 : 5) : 4);
 };
 template <int N>
 struct XT {
   static constexpr int TPP = PSplit<N>::TPP, XP = TPP > 16 ? CG_XP20 : CG_XP, THREADS = TPP * XP;
   static constexpr int minb(int mode) {
-    return TPP <= 16 ? 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X) : (TPP < 28 ? CG_FAST_MINB_X20 : 2);
+    return TPP <= 16 ? 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X) : (TPP < 28 ? (PSplit<N>::A <= 16 && TPP == 20 ? 4 : 3) : 2);
   }
 };
 

@@ -473,22 +473,33 @@ struct ZPShape {
   static constexpr int B_STG = (BOXES * BOXB + 1024) / 8, B_EX = P * EX, B_XB = N * P;  // float2 units
   static constexpr int B_MAX = B_STG > B_EX ? (B_STG > B_XB ? B_STG : B_XB) : (B_EX > B_XB ? B_EX : B_XB);
   static constexpr int BUF = (B_MAX + 1) / 2 * 2;  // even: float4-aligned
+  // tensor-map instantiations of more than 16 threads a pencil move the tile's
+  // field rows (contiguous) through shared memory by bulk copies instead of the
+  // threads' loads and stores: runs of 18..25 floats straddle sectors, and the
+  // registers that held the early loads are what these lengths lack. u- / p-pass
+  // us, threads' loads -> bulk: 300^3 397 / 146 -> 357 / 142, 384^3 669 / 274 ->
+  // 634 / 250, 400^3 705 / 278 -> 697 / 266, 256x256x200 222 / 92 -> 211 / 88;
+  // with 16 threads 192x192x256 97 / 41 -> 99 / 43, 160x160x192 x 8 379 / 149 ->
+  // 380 / 148.
+  static constexpr bool BULK = N % 2 == 0 && TMA_OK && TPP > 16;
 };
 
 // Shared-memory layout of the u-pass (U) or the p-pass:
 // twiddles (two orders, one when A == B) | two item buffers | material table
 // (u: (dt/rho, absorb); p: the four coefficients) | k_z (u) | z sponge | two
-// label tiles | two staging mbarriers. Offsets in float2 units.
-template <int N, bool U>
+// label tiles | field rows (bulk copies) | mbarriers. Offsets in float2 units.
+template <int N, bool U, bool TMA>
 struct ZPLayout {
   using Z = ZPShape<N>;
+  static constexpr bool BULK = TMA && Z::BULK;
   static constexpr int TWF = Z::A == Z::B ? 0 : N;  // twiddles of the forward order
   static constexpr size_t OFF_BUF = (Z::A == Z::B ? N : 2 * N) + (Z::A == Z::B ? N % 2 : 0);
   static constexpr size_t OFF_TAB = OFF_BUF + 2 * (size_t)Z::BUF;
   static constexpr size_t OFF_KZ = OFF_TAB + (U ? 256 : 512);
-  static constexpr size_t LABB = 2 * (size_t)Z::ROWS * N;  // bytes, a multiple of 16
+  static constexpr size_t LABB = 2 * ((size_t)Z::ROWS * N + 16);  // bytes, slots on multiples of 16
   static constexpr int KZ0 = U ? (Z::NH + 3) / 4 * 2 : 0, SZ0 = (N + 3) / 4 * 2;
-  static constexpr size_t CORE = sizeof(float2) * OFF_KZ + LABB + 16;
+  static constexpr size_t FLDB = BULK ? sizeof(float) * (size_t)Z::ROWS * N : 0;  // a multiple of 16
+  static constexpr size_t CORE = sizeof(float2) * OFF_KZ + LABB + FLDB + 32;
   // resident CTAs per SM: up to 16 warps (two CTAs of the 20..28-thread
   // pencils, whose 18..27 values a thread want more than 128 registers), as
   // far as shared memory allows
@@ -503,8 +514,9 @@ struct ZPLayout {
   static constexpr bool TBL = CORE + sizeof(float2) * (KZ0 + SZ0) <= zp_fit(MINB);
   static constexpr size_t OFF_SZ = OFF_KZ + (TBL ? KZ0 : 0);
   static constexpr size_t OFF_LAB = OFF_SZ + (TBL ? SZ0 : 0);
-  static constexpr size_t OFF_BAR = sizeof(float2) * OFF_LAB + LABB;  // bytes
-  static constexpr size_t smem = OFF_BAR + 2 * sizeof(unsigned long long);
+  static constexpr size_t OFF_FLD = sizeof(float2) * OFF_LAB + LABB;  // bytes
+  static constexpr size_t OFF_BAR = OFF_FLD + FLDB;                   // bytes
+  static constexpr size_t smem = OFF_BAR + 4 * sizeof(unsigned long long);
   static_assert(smem <= zp_fit(1), "persistent z-pass tile does not fit shared memory");
 };
 
@@ -590,22 +602,33 @@ __device__ __forceinline__ void zt_issue(char* stg, unsigned long long* bar, con
   if constexpr (Z::BOXES == 2) cgf::tma_load_3d(stg + Z::BOXB, map, bar, 2 * y0 + 32, 0, c2);
 }
 
-// The tile's labels (ROWS rows of N bytes, contiguous), asynchronously in the
-// widest pieces the row starts allow (every tile starts a multiple of 16 N
-// bytes into its plane; a plane holds ny N bytes), else by plain byte loads.
+// The tile's labels (ROWS rows of N bytes, contiguous) into lab_s +
+// label_shift, asynchronously: 16 bytes at a time where every plane of ny N
+// bytes starts on 16 (a tile starts a multiple of 16 N bytes into its plane),
+// else the 4-byte words that hold them; the last word of the volume, if it is
+// not whole, byte by byte.
+template <int N>
+__device__ __forceinline__ int label_shift(const Dims& d, int x) {
+  return (int)(((unsigned)x * (unsigned)(d.ny * N)) & 3u);
+}
 template <int N>
 __device__ __forceinline__ void z_prefetch_labels(uint8_t* lab_s, const uint8_t* __restrict__ labels, const Dims& d,
                                                   int x, int y0) {
   using Z = ZPShape<N>;
-  const uint8_t* src = labels + ((long long)x * d.ny + y0) * N;
+  const long long first = ((long long)x * d.ny + y0) * N;
   const int nb = min(Z::ROWS, d.ny - y0) * N;
-  const int plane = d.ny * N;
-  if (plane % 16 == 0) {
-    for (int i = 16 * threadIdx.x; i < nb; i += 16 * Z::THREADS) cgf::cp_async16(lab_s + i, src + i);
-  } else if (plane % 4 == 0) {
-    for (int i = 4 * threadIdx.x; i < nb; i += 4 * Z::THREADS) cgf::cp_async4(lab_s + i, src + i);
+  if ((d.ny * N) % 16 == 0) {
+    for (int i = 16 * threadIdx.x; i < nb; i += 16 * Z::THREADS) cgf::cp_async16(lab_s + i, labels + first + i);
   } else {
-    for (int i = threadIdx.x; i < nb; i += Z::THREADS) lab_s[i] = src[i];
+    const int mis = label_shift<N>(d, x);
+    const uint8_t* src = labels + first - mis;  // the volume starts on a multiple of 256
+    const long long avail = d.ncell - (first - mis);
+    for (int i = 4 * threadIdx.x; i < nb + mis; i += 4 * Z::THREADS) {
+      if (i + 4 <= avail)
+        cgf::cp_async4(lab_s + i, src + i);
+      else
+        for (int k = i; k < avail; ++k) lab_s[k] = src[k];
+    }
   }
 }
 
@@ -643,9 +666,9 @@ __device__ __forceinline__ void z_inputs_box(float2 (&v)[ZSplit<N>::A], const ch
   });
 }
 
-template <int N, bool U>
+template <int N, bool U, bool TMA>
 __device__ __forceinline__ void zp_tables(float2* sm, const Tables& t, const MediumDev& m) {
-  using L = ZPLayout<N, U>;
+  using L = ZPLayout<N, U, TMA>;
   using Z = ZPShape<N>;
   cgf::fill_twt<Z::A, Z::B>(sm, t.twz);
   if (L::TWF) cgf::fill_twt<Z::B, Z::A>(sm + L::TWF, t.twz);
@@ -678,6 +701,7 @@ __device__ __forceinline__ void zt_init(unsigned long long* bars) {
   if (threadIdx.x == 0) {
     cgf::mbar_init(bars, 1);
     cgf::mbar_init(bars + 1, 1);
+    cgf::mbar_init(bars + 2, 1);
     cgf::mbar_init_fence();
   }
   __syncthreads();
@@ -687,12 +711,12 @@ __device__ __forceinline__ void zt_init(unsigned long long* bars) {
 // descriptors, by value) instead of per-thread cp.async; the labels keep
 // cp.async. Other instantiations ignore ztma.
 template <int N, bool TMA = false>
-__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
+__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::MINB)
     kfp_zpass_u(Dims d, Tables t, MediumDev m, float* __restrict__ u, float2* __restrict__ S0,
                 float2* __restrict__ S1, float2* __restrict__ S2, int n_members,
                 const __grid_constant__ ZTma ztma) {
   using Z = ZPShape<N>;
-  using L = ZPLayout<N, true>;
+  using L = ZPLayout<N, true, TMA>;
   constexpr int A = Z::A, B = Z::B;
   extern __shared__ float2 sm[];
   const int ytiles = (d.ny + Z::ROWS - 1) / Z::ROWS;  // the last tile may be ragged
@@ -700,7 +724,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(sm) + L::OFF_BAR);
   unsigned phase = 0u;  // bit j: parity of item buffer j's next staging phase
   if constexpr (TMA) zt_init(bars);
-  zp_tables<N, true>(sm, t, m);
+  zp_tables<N, true, TMA>(sm, t, m);
   cgf::pdl_wait();
   const float* kz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_KZ) : t.kz;
   const float* sz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_SZ) : t.sz;
@@ -717,18 +741,30 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
     } else {
       z_prefetch<N>(stg, spec(c.comp, c.b), d, c.x, y0);
     }
-    if (lab) z_prefetch_labels<N>(lab0 + j * Z::ROWS * N, m.labels, d, c.x, y0);
+    if (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
     cgf::cp_async_commit();
   };
   ZCursor<3> cur(n_members, ytiles);
   int j = 0;
+  // the item's velocity rows (BULK)
+  float* fld = reinterpret_cast<float*>(reinterpret_cast<char*>(sm) + L::OFF_FLD);
+  auto rows_of = [&](const ZCursor<3>& c) {
+    return u + ((long long)c.comp * n_members + c.b) * d.ncell + ((long long)c.x * d.ny + c.yt * Z::ROWS) * N;
+  };
+  auto rows_bytes = [&](const ZCursor<3>& c) { return 4u * (unsigned)min(Z::ROWS, d.ny - c.yt * Z::ROWS) * N; };
+  auto load_rows = [&](const ZCursor<3>& c) {
+    if (threadIdx.x != 0) return;
+    cgf::mbar_expect_tx(bars + 2, rows_bytes(c));
+    cgf::bulk_load(fld, rows_of(c), rows_bytes(c), bars + 2);
+  };
   prefetch(cur, 0);  // every CTA of the grid has an item
+  if constexpr (L::BULK) load_rows(cur);
 #pragma unroll 1
   for (; cur.x < d.nx; j ^= 1) {
     const int comp = cur.comp;
     const long long b_idx = cur.b;
     const int x = cur.x, y0 = cur.yt * Z::ROWS;
-    const uint8_t* la = lab0 + j * Z::ROWS * N + (2 * p) * N;
+    const uint8_t* la = lab0 + j * (Z::ROWS * N + 16) + label_shift<N>(d, x) + (2 * p) * N;
     const uint8_t* lb = la + N;
     const int ya = y0 + 2 * p, yb = ya + 1;
     const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist
@@ -745,7 +781,9 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
         ub[b] = (s < A && vb) ? __ldg(uc + rowb + n) : 0.f;
       });
     };
-    if (Z::EARLY) load_u();
+    float* const rows = rows_of(cur);
+    const unsigned bytes = rows_bytes(cur);
+    if (Z::EARLY && !L::BULK) load_u();
     // (tensor-map path) this thread's generic accesses to the buffer the
     // next copy fills are ordered before that copy
     if constexpr (TMA) cgf::fence_proxy_async();
@@ -761,7 +799,15 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
     const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
     const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
     fft2<A, B, true>(v, w, s, sm, exi);
-    if (!Z::EARLY) load_u();
+    if (!Z::EARLY && !L::BULK) load_u();
+    if constexpr (L::BULK) {
+      zt_wait(bars, phase, 2, ztma.err);
+      static_for<0, B>([&](auto bi) {
+        constexpr int b = decltype(bi)::value;
+        ua[b] = (s < A) ? fld[2 * p * N + s + A * b] : 0.f;
+        ub[b] = (s < A) ? fld[(2 * p + 1) * N + s + A * b] : 0.f;
+      });
+    }
     const float spx = t.sx[x];
     const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
     // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
@@ -778,14 +824,31 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
       float unb = ub[b] - cb.x * w[b].y;
       unb = unb * cb.y;
       unb = unb * (spb * sz);
-      if (va) uc[rowa + n] = una;
-      if (vb) uc[rowb + n] = unb;
+      if constexpr (L::BULK) {
+        fld[2 * p * N + n] = una;
+        fld[(2 * p + 1) * N + n] = unb;
+      } else {
+        if (va) uc[rowa + n] = una;
+        if (vb) uc[rowb + n] = unb;
+      }
       w[b] = make_float2(una, vb ? unb : 0.f);
     });
+    if constexpr (L::BULK) {
+      cgf::fence_proxy_async();
+      __syncthreads();
+      if (threadIdx.x == 0) cgf::bulk_store(rows, fld, bytes);
+    }
     float2 X[A];
     fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+    if constexpr (L::BULK)
+      if (threadIdx.x == 0 && cur.x < d.nx) {  // cur: the next item
+        cgf::bulk_wait_read();
+        load_rows(cur);
+      }
     z_split_store<N, Z::P, false>(bufj, X, spec(comp, b_idx), d, x, y0, p, s, comp == 2 ? kz_s : nullptr);
   }
+  if constexpr (L::BULK)
+    if (threadIdx.x == 0) cgf::bulk_wait();
 }
 
 // REC: the step records into the phase bins (an instantiation without the
@@ -796,12 +859,12 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true>::MINB)
 // INV: only the opening inverse transform, its values to the pressure.
 // TMA: the half spectra arrive by tensor-map box copies (as in the u-pass).
 template <int N, bool REC, bool FWD = false, bool TMA = false, bool INV = false>
-__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
+__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::MINB)
     kfp_zpass_p(Dims d, Tables t, MediumDev m, SourceDev src, RecordDev rec, const long long* ctl, int n_local,
                 int record, float* __restrict__ p_all, float2* __restrict__ S0, int n_members,
                 const __grid_constant__ ZTma ztma) {
   using Z = ZPShape<N>;
-  using L = ZPLayout<N, false>;
+  using L = ZPLayout<N, false, TMA>;
   constexpr int A = Z::A, B = Z::B;
   static_assert(!(FWD && (TMA || INV)), "the forward-only pass stages no spectrum");
   extern __shared__ float2 sm[];
@@ -816,7 +879,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
   } else if constexpr (INV) {
     cgf::fill_twt<Z::A, Z::B>(sm, t.twz);
   } else {
-    zp_tables<N, false>(sm, t, m);
+    zp_tables<N, false, TMA>(sm, t, m);
   }
   cgf::pdl_wait();
   const float* sz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_SZ) : t.sz;
@@ -832,7 +895,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
     } else {
       z_prefetch<N>(stg, S0 + c.b * d.nspec, d, c.x, y0);
     }
-    if (lab) z_prefetch_labels<N>(lab0 + j * Z::ROWS * N, m.labels, d, c.x, y0);
+    if (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
     cgf::cp_async_commit();
   };
   ZCursor<1> cur(n_members, ytiles);
@@ -859,7 +922,19 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
     }
     return;
   }
+  // the tile's pressure rows (BULK)
+  float* fld = reinterpret_cast<float*>(reinterpret_cast<char*>(sm) + L::OFF_FLD);
+  auto rows_of = [&](const ZCursor<1>& c) {
+    return p_all + c.b * d.ncell + ((long long)c.x * d.ny + c.yt * Z::ROWS) * N;
+  };
+  auto rows_bytes = [&](const ZCursor<1>& c) { return 4u * (unsigned)min(Z::ROWS, d.ny - c.yt * Z::ROWS) * N; };
+  auto load_rows = [&](const ZCursor<1>& c) {
+    if (threadIdx.x != 0) return;
+    cgf::mbar_expect_tx(bars + 2, rows_bytes(c));
+    cgf::bulk_load(fld, rows_of(c), rows_bytes(c), bars + 2);
+  };
   prefetch(cur, 0);
+  if constexpr (L::BULK) load_rows(cur);
   const long long n_step = INV ? 0 : ctl[0] + n_local;
   const int m_bin = (int)(n_step % rec.spp);
   const long long per_log = n_step / rec.spp;
@@ -881,7 +956,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
   for (; cur.x < d.nx; j ^= 1) {
     const long long b_idx = cur.b;
     const int x = cur.x, y0 = cur.yt * Z::ROWS;
-    const uint8_t* la = lab0 + j * Z::ROWS * N + (2 * p) * N;
+    const uint8_t* la = lab0 + j * (Z::ROWS * N + 16) + label_shift<N>(d, x) + (2 * p) * N;
     const uint8_t* lb = la + N;
     const int ya = y0 + 2 * p, yb = ya + 1;
     const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist
@@ -899,7 +974,9 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
         pbv[b] = (s < A && vb) ? __ldg(pb + rowb + n) : 0.f;
       });
     };
-    if (Z::EARLY && !INV) load_p();
+    float* const rows = rows_of(cur);
+    const unsigned bytes = rows_bytes(cur);
+    if (Z::EARLY && !INV && !L::BULK) load_p();
     if constexpr (TMA) cgf::fence_proxy_async();  // see the u-pass
     cgf::cp_async_wait0();
     __syncthreads();
@@ -922,7 +999,15 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
       });
         continue;
     }
-    if (!Z::EARLY) load_p();
+    if (!Z::EARLY && !L::BULK) load_p();
+    if constexpr (L::BULK) {
+      zt_wait(bars, phase, 2, ztma.err);
+      static_for<0, B>([&](auto bi) {
+        constexpr int b = decltype(bi)::value;
+        pa[b] = (s < A) ? fld[2 * p * N + s + A * b] : 0.f;
+        pbv[b] = (s < A) ? fld[(2 * p + 1) * N + s + A * b] : 0.f;
+      });
+    }
     const float spx = t.sx[x];
     const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
     // p <- (p - (rho c^2 dt [+ 2 beta dt p]) div u) * absorb * sponge   (engine.py:470-477)
@@ -975,8 +1060,13 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
       constexpr int b = decltype(bi)::value;
       const int n = s + A * b;
       const float pna = w[b].x, pnb = w[b].y;
-      if (va) pb[rowa + n] = pna;
-      if (vb) pb[rowb + n] = pnb;
+      if constexpr (L::BULK) {
+        fld[2 * p * N + n] = pna;
+        fld[(2 * p + 1) * N + n] = pnb;
+      } else {
+        if (va) pb[rowa + n] = pna;
+        if (vb) pb[rowb + n] = pnb;
+      }
       if ((zconv >> b) & 1u) {
         if (conv_a) lpeak = max(lpeak, __float_as_uint(fabsf(pna)));
         if (conv_b) lpeak = max(lpeak, __float_as_uint(fabsf(pnb)));
@@ -1038,10 +1128,22 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false>::MINB)
       wmember = (int)b_idx;
     }
     wpeak = max(wpeak, lpeak);
+    if constexpr (L::BULK) {
+      cgf::fence_proxy_async();
+      __syncthreads();
+      if (threadIdx.x == 0) cgf::bulk_store(rows, fld, bytes);
+    }
     float2 X[A];
     fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+    if constexpr (L::BULK)
+      if (threadIdx.x == 0 && cur.x < d.nx) {  // cur: the next tile
+        cgf::bulk_wait_read();
+        load_rows(cur);
+      }
     z_split_store<N, Z::P, false>(bufj, X, S, d, x, y0, p, s, nullptr);
   }
+  if constexpr (L::BULK)
+    if (threadIdx.x == 0) cgf::bulk_wait();
   if ((threadIdx.x & 31) == 0 && wpeak && wmember >= 0 && per_log < rec.max_periods)
     atomicMax(&rec.peaks[(long long)wmember * rec.max_periods + per_log], wpeak);
 }
@@ -1062,16 +1164,17 @@ static long long zp_tiles(const Dims& d, int batch) {
 template <int N>
 void zp_run_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
               int batch, cudaStream_t st, const ZTma* ztma) {
-  using L = ZPLayout<N, true>;
-  const int g = zp_grid(3 * zp_tiles<N>(d, batch), L::MINB);
+  const long long items = 3 * zp_tiles<N>(d, batch);
   if constexpr (ZPShape<N>::TMA_OK) {
     if (ztma) {
-      cgf::launch(d.pdl, kfp_zpass_u<N, true>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
+      using L = ZPLayout<N, true, true>;
+      cgf::launch(d.pdl, kfp_zpass_u<N, true>, dim3(zp_grid(items, L::MINB)), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
                   *ztma);
       return;
     }
   }
-  cgf::launch(d.pdl, kfp_zpass_u<N>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
+  using L = ZPLayout<N, true, false>;
+  cgf::launch(d.pdl, kfp_zpass_u<N>, dim3(zp_grid(items, L::MINB)), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
               kNoZTma);
 }
 
@@ -1079,12 +1182,12 @@ template <int N>
 void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
               const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
               const ZTma* ztma) {
-  using L = ZPLayout<N, false>;
-  const int g = zp_grid(zp_tiles<N>(d, batch), L::MINB);
-  const dim3 grid(g), block(ZPShape<N>::THREADS);
-  const size_t sm = L::smem;
+  const dim3 block(ZPShape<N>::THREADS);
   if constexpr (ZPShape<N>::TMA_OK) {
     if (ztma) {
+      using L = ZPLayout<N, false, true>;
+      const dim3 grid(zp_grid(zp_tiles<N>(d, batch), L::MINB));
+      const size_t sm = L::smem;
       if (record)
         cgf::launch(d.pdl, kfp_zpass_p<N, true, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p,
                     S0, batch, *ztma);
@@ -1094,6 +1197,9 @@ void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDe
       return;
     }
   }
+  using L = ZPLayout<N, false, false>;
+  const dim3 grid(zp_grid(zp_tiles<N>(d, batch), L::MINB));
+  const size_t sm = L::smem;
   if (record)
     cgf::launch(d.pdl, kfp_zpass_p<N, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, kNoZTma);
   else
@@ -1104,7 +1210,7 @@ void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDe
 template <int N>
 void zp_run_half(bool inverse, const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
                  cudaStream_t st) {
-  using L = ZPLayout<N, false>;
+  using L = ZPLayout<N, false, false>;
   const int g = zp_grid(zp_tiles<N>(d, batch), L::MINB);
   SourceDev src;
   memset(&src, 0, sizeof(src));
@@ -1126,13 +1232,14 @@ static bool zp_allow(K kernel, size_t bytes) {
 
 template <int N>
 int zp_prepare() {
-  constexpr size_t su = ZPLayout<N, true>::smem, sp = ZPLayout<N, false>::smem;
+  constexpr size_t su = ZPLayout<N, true, false>::smem, sp = ZPLayout<N, false, false>::smem;
+  constexpr size_t tu = ZPLayout<N, true, true>::smem, tp = ZPLayout<N, false, true>::smem;
   bool ok = zp_allow(kfp_zpass_u<N>, su) && zp_allow(kfp_zpass_p<N, false, true>, sp) &&
             zp_allow(kfp_zpass_p<N, false, false, false, true>, sp) && zp_allow(kfp_zpass_p<N, true>, sp) &&
             zp_allow(kfp_zpass_p<N, false>, sp);
   if constexpr (ZPShape<N>::TMA_OK)
-    ok = ok && zp_allow(kfp_zpass_u<N, true>, su) && zp_allow(kfp_zpass_p<N, true, false, true>, sp) &&
-         zp_allow(kfp_zpass_p<N, false, false, true>, sp);
+    ok = ok && zp_allow(kfp_zpass_u<N, true>, tu) && zp_allow(kfp_zpass_p<N, true, false, true>, tp) &&
+         zp_allow(kfp_zpass_p<N, false, false, true>, tp);
   return ok ? 0 : -1;
 }
 
