@@ -1,6 +1,7 @@
 // Size-specialised pencil FFTs: register DFT codelets with compile-time
 // twiddles and a two-level ("four-step") transform with one shared-memory
-// exchange per pencil transform.
+// exchange per pencil transform (three levels and two exchanges on 125, 243, 250
+// and 375 points, see fft3).
 //
 // A pencil of length N = A * B is held by B threads on input: thread s < B
 // owns x[s + B a], a in [0, A). Phase 1 applies an A-point DFT in registers
@@ -233,6 +234,13 @@ constexpr int ct_even_split(int n) {
   return best;
 }
 
+// Whether a split (a, b) is transformed in three levels: where the codelets of
+// b points would leave most threads idle (a of b busy) on more than 20 values
+// each, and b = c d with c and d factors of a (125, 243, 250 and 375 points: a
+// step 251 -> 108 us at 125^3, 1207 -> 643 at 243^3, 3537 -> 2624 at 375^3).
+constexpr int ct_three_d(int b) { return ct_even_split(b); }
+constexpr bool ct_three(int a, int b) { return b > 20 && a % ct_three_d(b) == 0 && a % (b / ct_three_d(b)) == 0; }
+
 // Threads per pencil for a split whose larger factor is m: 8 or 16 (whole
 // pencils per warp), else m rounded up to 4 so that 8 pencils fill whole warps.
 constexpr int ct_tpp(int m) { return m <= 8 ? 8 : (m <= 16 ? 16 : (m + 3) / 4 * 4); }
@@ -241,21 +249,26 @@ constexpr int ct_tpp(int m) { return m <= 8 ? 8 : (m <= 16 ? 16 : (m + 3) / 4 * 
 // holding A values on input and A threads holding B values on output. The
 // most even split: fewest instructions for the warp that waits on its
 // longest codelet, and up to 400 points no thread holds more than 20 values
-// except on 243, 250, 375 and 384 (27, 25, 25, 24). Against 16 x (N / 16)
+// except on 384 (24), the lengths of three levels included. Against 16 x (N / 16)
 // for the multiples of 16: 64^3 33 -> 29 us a step, 96x96x128 54 -> 52,
 // 32^3 25 -> 20.
 template <int N>
 struct PSplit {
   static constexpr int A = ct_even_split(N), B = N / A;
-  static constexpr int TPP = ct_tpp(A > B ? A : B);  // threads per pencil
+  static constexpr bool THREE = ct_three(A, B);
+  static constexpr int OA = THREE ? B : A, OB = THREE ? A : B;  // threads and values after the transform
+  static constexpr int TW = N + (THREE ? B : 0);                // entries of a twiddle table
+  static constexpr int TPP = ct_tpp(A > B ? A : B);             // threads per pencil
 };
 template <>
 struct PSplit<512> {
-  static constexpr int A = 32, B = 16, TPP = 32;
+  static constexpr int A = 32, B = 16, OA = A, OB = B, TW = 512, TPP = 32;
+  static constexpr bool THREE = false;
 };
 template <>
 struct PSplit<640> {
-  static constexpr int A = 32, B = 20, TPP = 32;
+  static constexpr int A = 32, B = 20, OA = A, OB = B, TW = 640, TPP = 32;
+  static constexpr bool THREE = false;
 };
 
 // The split of the y-passes, whose threads read and write runs of a row: 16 x
@@ -265,6 +278,7 @@ template <int N>
 struct YSplit {
   static constexpr bool LINES = N % 16 == 0 && N > 64 && N <= 256;
   static constexpr int A = LINES ? N / 16 : PSplit<N>::A, B = N / A;
+  static constexpr int OA = LINES ? A : PSplit<N>::OA, OB = N / OA, TW = PSplit<N>::TW;
   static constexpr int TPP = ct_tpp(A > B ? A : B);
 };
 
@@ -304,30 +318,37 @@ __device__ __forceinline__ void ex_sync() {
 }
 
 // Twiddle table of an (A, B) transform in the order the threads read it:
-// twt[k1 * B + s] = exp(-2 pi i s k1 / N) (lanes run over s: conflict free).
-template <int A, int B>
+// twt[k1 * B + s] = exp(-2 pi i s k1 / N) (lanes run over s: conflict free);
+// behind it, for a three-level transform (R != B values per thread after it),
+// exp(-2 pi i m / B).
+template <int A, int B, int R = B>
 __device__ __forceinline__ void fill_twt(float2* twt, const float2* __restrict__ tw_lin) {
   for (int i = threadIdx.x; i < A * B; i += blockDim.x) {
     const int k1 = i / B, s = i - k1 * B;
     twt[i] = tw_lin[s * k1];
   }
+  if constexpr (R != B)
+    for (int i = threadIdx.x; i < B; i += blockDim.x) twt[A * B + i] = tw_lin[A * i];
 }
 
-// (A, B) transform of one pencil: thread s (< B) holds v[a] = x[s + B a];
-// afterwards thread s (< A) holds w[b] = X[s + A b]. `twt` is the table laid
-// out by fill_twt<A, B>. Every thread of the block calls it.
-template <int A, int B, bool INV, class Ex>
-__device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[B], int s, const float2* __restrict__ twt,
+// Three-level transform of one pencil of V T points, T = C D: thread s (< T)
+// holds v[a] = x[s + T a] before and w[a] = X[s + T a] after it. Level 1: V
+// points per thread; level 2: C points of every (k1, d), each thread V / C of
+// them, in the slots it read; level 3: D points of every m = k1 + V kc, m = s +
+// T j. All T threads work in every level and hold V values.
+template <int V, int T, bool INV, class Ex>
+__device__ __forceinline__ void fft3(const float2 (&v_in)[V], float2 (&w)[V], int s, const float2* __restrict__ twt,
                                      const Ex& ex) {
-  if (s < B) {
-    float2 v[A];
-    static_for<0, A>([&](auto i) { v[decltype(i)::value] = v_in[decltype(i)::value]; });
-    Dft<A, INV>::run(v);
-    static_for<0, A>([&](auto ki) {
+  constexpr int D = ct_three_d(T), C = T / D, JC = V / C, JD = V / D;
+  if (s < T) {
+    float2 v[V];
+    static_for<0, V>([&](auto i) { v[decltype(i)::value] = v_in[decltype(i)::value]; });
+    Dft<V, INV>::run(v);
+    static_for<0, V>([&](auto ki) {
       constexpr int k1 = decltype(ki)::value;
       float2 y = v[k1];
       if constexpr (k1 > 0) {
-        float2 t = twt[k1 * B + s];
+        float2 t = twt[k1 * T + s];
         if (INV) t.y = -t.y;
         y = c_mul(y, t);
       }
@@ -335,11 +356,71 @@ __device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[B], in
     });
   }
   ex_sync<Ex>();
-  if (s < A) {
-    static_for<0, B>([&](auto bi) { w[decltype(bi)::value] = ex.at(s, decltype(bi)::value); });
-    Dft<B, INV>::run(w);
+  if (s < T) {
+    const int d = s % D, k0 = s / D;
+    static_for<0, JC>([&](auto ji) {
+      const int k1 = k0 + C * decltype(ji)::value;
+      float2 q[C];
+      static_for<0, C>([&](auto ci) { q[decltype(ci)::value] = ex.at(k1, D * decltype(ci)::value + d); });
+      Dft<C, INV>::run(q);
+      static_for<0, C>([&](auto ki) {
+        constexpr int kc = decltype(ki)::value;
+        if constexpr (kc > 0) {
+          float2 t = twt[V * T + d * kc];
+          if (INV) t.y = -t.y;
+          q[kc] = c_mul(q[kc], t);
+        }
+        ex.at(k1, D * kc + d) = q[kc];
+      });
+    });
   }
   ex_sync<Ex>();
+  if (s < T) {
+    static_for<0, JD>([&](auto ji) {
+      constexpr int j = decltype(ji)::value;
+      const int m = s + T * j, kc = m / V, k1 = m - V * kc;
+      float2 q[D];
+      static_for<0, D>([&](auto di) { q[decltype(di)::value] = ex.at(k1, D * kc + decltype(di)::value); });
+      Dft<D, INV>::run(q);
+      static_for<0, D>([&](auto ki) { w[j + JD * decltype(ki)::value] = q[decltype(ki)::value]; });
+    });
+  }
+  ex_sync<Ex>();
+}
+
+// (A, B) transform of one pencil: thread s (< B) holds v[a] = x[s + B a];
+// afterwards thread s (< A) holds w[b] = X[s + A b], or, in three levels, s (<
+// B) w[a] = X[s + B a]. `twt` is the table laid out by fill_twt. Every thread
+// of the block calls it.
+template <int A, int B, bool INV, class Ex, int R>
+__device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[R], int s, const float2* __restrict__ twt,
+                                     const Ex& ex) {
+  if constexpr (R != B) {
+    fft3<A, B, INV>(v_in, w, s, twt, ex);
+    return;
+  } else {
+    if (s < B) {
+      float2 v[A];
+      static_for<0, A>([&](auto i) { v[decltype(i)::value] = v_in[decltype(i)::value]; });
+      Dft<A, INV>::run(v);
+      static_for<0, A>([&](auto ki) {
+        constexpr int k1 = decltype(ki)::value;
+        float2 y = v[k1];
+        if constexpr (k1 > 0) {
+          float2 t = twt[k1 * B + s];
+          if (INV) t.y = -t.y;
+          y = c_mul(y, t);
+        }
+        ex.at(k1, s) = y;
+      });
+    }
+    ex_sync<Ex>();
+    if (s < A) {
+      static_for<0, B>([&](auto bi) { w[decltype(bi)::value] = ex.at(s, decltype(bi)::value); });
+      Dft<B, INV>::run(w);
+    }
+    ex_sync<Ex>();
+  }
 }
 
 // Asynchronous 16-byte global -> shared copy (L2 only), completed by

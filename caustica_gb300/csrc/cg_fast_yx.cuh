@@ -56,19 +56,25 @@ using cgf::static_for;
 // 155 / 166 against 176 / 166, 400^3 323 / 333 against 297 / 302; with two,
 // 400^3 348 / 345), and five y-CTAs, or six up to 34 values (Y_INV_GRAD /
 // Y_FWD_DIV with six / five: 288^3 106 / 109 against 107 / 129, 320^3 146 / 144
-// against 129 / 133).
+// against 129 / 133). Three-level pencils: four x- and eight y-CTAs up to ten
+// values a thread, three and six above (250^3 with 4, 8 / 3, 6 / 2, 4 CTAs:
+// X_GRAD 78 / 86 / 107, Y_INV_GRAD 81 / 82 / 88; 375^3 308 / 293 / 316 and 321 /
+// 287 / 291).
 template <int N>
 struct YT {
   static constexpr int TPP = YSplit<N>::TPP, YP = TPP < 16 ? 2 * CG_YP : (TPP > 16 && TPP < 32 ? CG_YP20 : CG_YP);
   static constexpr int THREADS = TPP * YP;
-  static constexpr int SUM = YSplit<N>::A + YSplit<N>::B;
-  static constexpr int MINB = TPP <= 16 ? CG_FAST_MINB_Y : (TPP < 28 ? (SUM <= 34 ? 6 : 5) : 4);
+  static constexpr int SUM = YSplit<N>::A + YSplit<N>::B, VALS = YSplit<N>::A;
+  static constexpr bool THREE = PSplit<N>::THREE && !YSplit<N>::LINES;
+  static constexpr int MINB = TPP <= 16 ? CG_FAST_MINB_Y : (TPP < 28 ? (SUM <= 34 ? 6 : 5) : (THREE ? (VALS <= 10 ? 8 : 6) : 4));
 };
 template <int N>
 struct XT {
   static constexpr int TPP = PSplit<N>::TPP, XP = TPP > 16 ? CG_XP20 : CG_XP, THREADS = TPP * XP;
   static constexpr int minb(int mode) {
-    return TPP <= 16 ? 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X) : (TPP < 28 ? (PSplit<N>::A <= 16 && TPP == 20 ? 4 : 3) : 2);
+    if (TPP <= 16) return 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X);
+    if (PSplit<N>::THREE) return PSplit<N>::A <= 10 ? 4 : 3;
+    return TPP < 28 ? (PSplit<N>::A <= 16 && TPP == 20 ? 4 : 3) : 2;
   }
 };
 
@@ -80,21 +86,22 @@ template <int N, int MODE>
 __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, Tables t, float2* __restrict__ S0,
                                                                         float2* __restrict__ S1,
                                                                         float2* __restrict__ S2) {
-  constexpr int A = YSplit<N>::A, B = YSplit<N>::B, TPP = YSplit<N>::TPP;
+  constexpr int A = YSplit<N>::A, B = YSplit<N>::B, OA = YSplit<N>::OA, OB = YSplit<N>::OB, TW = YSplit<N>::TW,
+                TPP = YSplit<N>::TPP;
   using Ex = RowEx<A, B, (32 % TPP == 0)>;  // pencil-local exchange: warp barriers
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
   float2* tw = sm;  // (A, B) order
-  cgf::fill_twt<A, B>(tw, t.twy);
+  cgf::fill_twt<A, B, OB>(tw, t.twy);
   cgf::pdl_wait();
   const int s = threadIdx.x % TPP, p = threadIdx.x / TPP;
-  const Ex ex{sm + N + p * Ex::SLAB};
+  const Ex ex{sm + TW + p * Ex::SLAB};
   const long long nrows = (long long)d.nx * d.nzh;
   const long long row = (long long)blockIdx.x * YT<N>::YP + p;
   const bool valid = row < nrows;
   const long long off = (long long)blockIdx.y * d.nspec + row * N;
   __syncthreads();
-  float2 v[A], w[B];
+  float2 v[A], w[OB];
   auto load = [&](const float2* __restrict__ src) {
     static_for<0, A>([&](auto ai) {
       constexpr int a = decltype(ai)::value;
@@ -102,9 +109,9 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
     });
   };
   auto store = [&](float2* __restrict__ dst) {
-    if (valid && s < A) static_for<0, B>([&](auto bi) {
+    if (valid && s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      dst[off + s + A * b] = w[b];
+      dst[off + s + OA * b] = w[b];
     });
   };
   if constexpr (MODE == Y_FWD || MODE == Y_INV) {
@@ -134,15 +141,15 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
     store(S1);
     load(S0);
     fft2<A, B, false>(v, w, s, tw, ex);
-    float2 h[B];
-    static_for<0, B>([&](auto bi) {
+    float2 h[OB];
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const float k = (s < A) ? t.ky[s + A * b] : 0.f;
+      const float k = (s < OA) ? t.ky[s + OA * b] : 0.f;
       h[b] = c_muli(c_scale(w[b], k));
     });
     load(S2);
     fft2<A, B, false>(v, w, s, tw, ex);
-    static_for<0, B>([&](auto bi) { w[decltype(bi)::value] = c_add(w[decltype(bi)::value], h[decltype(bi)::value]); });
+    static_for<0, OB>([&](auto bi) { w[decltype(bi)::value] = c_add(w[decltype(bi)::value], h[decltype(bi)::value]); });
     store(S0);
   }
 }
@@ -159,26 +166,27 @@ template <int N, bool DIV>
 __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, float kcoef, float invN,
                                                               float2* __restrict__ S0, float2* __restrict__ S1,
                                                               float2* __restrict__ S2) {
-  constexpr int A = YSplit<N>::A, B = YSplit<N>::B, TPP = YSplit<N>::TPP;
+  constexpr int A = YSplit<N>::A, B = YSplit<N>::B, OA = YSplit<N>::OA, OB = YSplit<N>::OB, TW = YSplit<N>::TW,
+                TPP = YSplit<N>::TPP;
   using ExF = RowEx<A, B, (32 % TPP == 0)>;
-  using ExI = RowEx<B, A, (32 % TPP == 0)>;
+  using ExI = RowEx<OB, OA, (32 % TPP == 0)>;
   constexpr int SLAB = ExF::SLAB > ExI::SLAB ? ExF::SLAB : ExI::SLAB;
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
-  float2* tw = sm;       // (A, B) order
-  float2* twi = sm + N;  // (B, A) order
-  cgf::fill_twt<A, B>(tw, t.twy);
-  cgf::fill_twt<B, A>(twi, t.twy);
+  float2* tw = sm;        // (A, B) order
+  float2* twi = sm + TW;  // (OB, OA) order
+  cgf::fill_twt<A, B, OB>(tw, t.twy);
+  cgf::fill_twt<OB, OA, A>(twi, t.twy);
   cgf::pdl_wait();
   const int s = threadIdx.x % TPP, p = threadIdx.x / TPP;
-  const ExF exf{sm + 2 * N + p * SLAB};
-  const ExI exi{sm + 2 * N + p * SLAB};
+  const ExF exf{sm + 2 * TW + p * SLAB};
+  const ExI exi{sm + 2 * TW + p * SLAB};
   const int row = blockIdx.x * YT<N>::YP + p;  // kz
   const bool valid = row < d.nzh;
   const long long off = (long long)blockIdx.y * d.nspec + (long long)row * N;
   const float kz2 = valid ? t.kz2[row] : 0.f;
   __syncthreads();
-  float2 v[A], w[B], z[A];
+  float2 v[A], w[OB], z[A];
   auto load = [&](const float2* src) {
     static_for<0, A>([&](auto ai) {
       constexpr int a = decltype(ai)::value;
@@ -195,26 +203,26 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
   if constexpr (!DIV) {
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
-    float2 g[B];
-    static_for<0, B>([&](auto bi) {
+    float2 g[OB];
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int k = (s < A) ? s + A * b : 0;
+      const int k = (s < OA) ? s + OA * b : 0;
       w[b] = c_scale(w[b], kappa(k));
       g[b] = c_muli(c_scale(w[b], t.ky[k]));
     });
-    fft2<B, A, true>(g, z, s, twi, exi);
+    fft2<OB, OA, true>(g, z, s, twi, exi);
     store_z(S0);
-    fft2<B, A, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true>(w, z, s, twi, exi);
     store_z(S2);
     static_for<0, A>([&](auto ai) { z[decltype(ai)::value] = c_scale(z[decltype(ai)::value], 0.f); });
     store_z(S1);
   } else {
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
-    float2 h[B];
-    static_for<0, B>([&](auto bi) {
+    float2 h[OB];
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int k = (s < A) ? s + A * b : 0;
+      const int k = (s < OA) ? s + OA * b : 0;
       h[b] = c_muli(c_scale(w[b], t.ky[k]));
     });
     load(S2);
@@ -223,12 +231,12 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
       if (valid && s < B) v[a] = c_add(v[a], c_scale(S1[off + s + B * a], 0.f));
     });
     fft2<A, B, false>(v, w, s, tw, exf);
-    static_for<0, B>([&](auto bi) {
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int k = (s < A) ? s + A * b : 0;
+      const int k = (s < OA) ? s + OA * b : 0;
       w[b] = c_scale(c_add(w[b], h[b]), kappa(k));
     });
-    fft2<B, A, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true>(w, z, s, twi, exi);
     store_z(S0);
   }
 }
@@ -236,8 +244,8 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
 template <int N>
 static size_t smem_plane() {
   using F = RowEx<YSplit<N>::A, YSplit<N>::B>;
-  using I = RowEx<YSplit<N>::B, YSplit<N>::A>;
-  return sizeof(float2) * (2 * N + YT<N>::YP * (F::SLAB > I::SLAB ? F::SLAB : I::SLAB));
+  using I = RowEx<YSplit<N>::OB, YSplit<N>::OA>;
+  return sizeof(float2) * (2 * YSplit<N>::TW + YT<N>::YP * (F::SLAB > I::SLAB ? F::SLAB : I::SLAB));
 }
 
 template <int N, int MODE>
@@ -245,22 +253,23 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
                                                                         float2* __restrict__ S0,
                                                                         float2* __restrict__ S1,
                                                                         float2* __restrict__ S2) {
-  constexpr int A = PSplit<N>::A, B = PSplit<N>::B, XP = XT<N>::XP;
+  constexpr int A = PSplit<N>::A, B = PSplit<N>::B, OA = PSplit<N>::OA, OB = PSplit<N>::OB, TW = PSplit<N>::TW,
+                XP = XT<N>::XP;
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
-  float2* tw = sm;       // (A, B) order
-  float2* twi = sm + N;  // (B, A) order
-  cgf::fill_twt<A, B>(tw, t.twx);
-  cgf::fill_twt<B, A>(twi, t.twx);
-  float* kxs = reinterpret_cast<float*>(sm + 2 * N + 2 * N * XP);  // k_x | k_x^2
+  float2* tw = sm;        // (A, B) order
+  float2* twi = sm + TW;  // (OB, OA) order
+  cgf::fill_twt<A, B, OB>(tw, t.twx);
+  cgf::fill_twt<OB, OA, A>(twi, t.twx);
+  float* kxs = reinterpret_cast<float*>(sm + 2 * TW + 2 * N * XP);  // k_x | k_x^2
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     kxs[i] = t.kx[i];
     kxs[N + i] = t.kx2[i];
   }
   cgf::pdl_wait();
   const int c = threadIdx.x % XP, s = threadIdx.x / XP;
-  const ColEx<A, B, XP> exf{sm + 2 * N + c};
-  const ColEx<B, A, XP> exi{sm + 2 * N + c};
+  const ColEx<A, B, XP> exf{sm + 2 * TW + c};
+  const ColEx<OB, OA, XP> exi{sm + 2 * TW + c};
   const long long ncol = (long long)d.nzh * d.ny;
   const long long col = (long long)blockIdx.x * XP + c;
   const bool valid = col < ncol;
@@ -273,7 +282,7 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
     kyz2 = t.ky2[ky] + t.kz2[kz];
   }
   __syncthreads();
-  float2 v[A], w[B], z[A];
+  float2 v[A], w[OB], z[A];
   auto load = [&](const float2* __restrict__ src) {
     static_for<0, A>([&](auto ai) {
       constexpr int a = decltype(ai)::value;
@@ -289,7 +298,7 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
         v[a] = (valid && s < B) ? cgf::ld_once(g) : make_float2(0.f, 0.f);
     });
   };
-  // after an inverse (B, A) transform thread s < B owns z[a] = element s + B a
+  // after an inverse (OB, OA) transform thread s < B owns z[a] = element s + B a
   auto store_z = [&](float2* __restrict__ dst) {
     if (valid && s < B) static_for<0, A>([&](auto ai) {
       constexpr int a = decltype(ai)::value;
@@ -300,49 +309,49 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
   if constexpr (MODE == X_FWD || MODE == X_INV) {  // S0 <- (I)FFT(S1); S1 may be S0
     load(S1);
     fft2<A, B, MODE == X_INV>(v, w, s, tw, exf);
-    if (valid && s < A) static_for<0, B>([&](auto bi) {
+    if (valid && s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      S0[base + (long long)(s + A * b) * ncol] = w[b];
+      S0[base + (long long)(s + OA * b) * ncol] = w[b];
     });
   } else if constexpr (MODE == X_GRAD) {
     // S2 <- IFFT(q); S1 <- IFFT(i kx q), q = kappa/N FFT(S0); q waits in shared
     // memory during the first inverse transform instead of in registers
-    float2* qs = sm + 2 * N + N * XP;
+    float2* qs = sm + 2 * TW + N * XP;
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
-    static_for<0, B>([&](auto bi) {
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int k = (s < A) ? s + A * b : 0;
+      const int k = (s < OA) ? s + OA * b : 0;
       w[b] = c_scale(w[b], kappa(k));
-      if (s < A) qs[(s + A * b) * XP + c] = w[b];
+      if (s < OA) qs[(s + OA * b) * XP + c] = w[b];
     });
-    fft2<B, A, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true>(w, z, s, twi, exi);
     store_z(S2);
-    static_for<0, B>([&](auto bi) {
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int k = (s < A) ? s + A * b : 0;
-      w[b] = (s < A) ? c_muli(c_scale(qs[(s + A * b) * XP + c], kxs[k])) : make_float2(0.f, 0.f);
+      const int k = (s < OA) ? s + OA * b : 0;
+      w[b] = (s < OA) ? c_muli(c_scale(qs[(s + OA * b) * XP + c], kxs[k])) : make_float2(0.f, 0.f);
     });
-    fft2<B, A, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true>(w, z, s, twi, exi);
     store_z(S1);
   } else {
     // X_DIV: S0 <- IFFT(kappa/N (FFT(S0) + i kx FFT(S1))); FFT(S1) waits in shared memory
-    float2* hs = sm + 2 * N + N * XP;
+    float2* hs = sm + 2 * TW + N * XP;
     load(S1);
     fft2<A, B, false>(v, w, s, tw, exf);
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      hs[(s + A * b) * XP + c] = w[b];
+      hs[(s + OA * b) * XP + c] = w[b];
     });
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
-    static_for<0, B>([&](auto bi) {
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int k = (s < A) ? s + A * b : 0;
-      const float2 h = (s < A) ? hs[(s + A * b) * XP + c] : make_float2(0.f, 0.f);
+      const int k = (s < OA) ? s + OA * b : 0;
+      const float2 h = (s < OA) ? hs[(s + OA * b) * XP + c] : make_float2(0.f, 0.f);
       w[b] = c_scale(c_add(w[b], c_muli(c_scale(h, kxs[k]))), kappa(k));
     });
-    fft2<B, A, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true>(w, z, s, twi, exi);
     store_z(S0);
   }
 }
@@ -350,11 +359,11 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
 // twiddles | exchange | (x: a parked spectrum tile, k_x, k_x^2)
 template <int N>
 static size_t smem_y() {
-  return sizeof(float2) * (N + YT<N>::YP * RowEx<YSplit<N>::A, YSplit<N>::B>::SLAB);
+  return sizeof(float2) * (YSplit<N>::TW + YT<N>::YP * RowEx<YSplit<N>::A, YSplit<N>::B>::SLAB);
 }
 template <int N>
 static size_t smem_x() {
-  return sizeof(float2) * (2 * N + 2 * (size_t)N * XT<N>::XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
+  return sizeof(float2) * (2 * PSplit<N>::TW + 2 * (size_t)N * XT<N>::XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
 }
 
 // ------------------------------------------------ per-length launchers --

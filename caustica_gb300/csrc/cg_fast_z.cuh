@@ -36,13 +36,20 @@ using cgf::static_for;
 template <int N>
 struct ZSplit {
   using P = cgf::PSplit<N>;
-  static constexpr int A = P::A > P::B ? P::A : P::B, B = P::A > P::B ? P::B : P::A, TPP = P::TPP;
+  static constexpr bool SWAP = !P::THREE && P::A < P::B;
+  static constexpr int A = SWAP ? P::B : P::A, B = SWAP ? P::A : P::B;
+  static constexpr int OA = SWAP ? P::OB : P::OA, OB = SWAP ? P::OA : P::OB, TW = P::TW;
+  // three-level pencils fill a warp each, so that their three exchanges wait for
+  // no other pencil (u-/p-pass us, 32 / 28 threads a pencil, two CTAs to an SM:
+  // 250^3 242 / 95 against 254 / 103, 375^3 941 / 385 against 1303 / 667; three
+  // CTAs of 32: 255 / 99, 1254 / 607)
+  static constexpr int TPP = P::THREE ? 32 : P::TPP;
 };
 
 template <int N>
 struct ZShape {
-  static constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, NH = N / 2 + 1;
-  static constexpr int EX_I = RowEx<A, B>::SLAB, EX_F = RowEx<B, A>::SLAB;
+  static constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, OA = ZSplit<N>::OA, OB = ZSplit<N>::OB, NH = N / 2 + 1;
+  static constexpr int EX_I = RowEx<A, B>::SLAB, EX_F = RowEx<OB, OA>::SLAB;
   static constexpr int EX = EX_I > EX_F ? EX_I : EX_F;
   static constexpr int STG = (NH * 34 > N * 17) ? NH * 34 : N * 17;  // float2 units
   // twiddles (two orders) | staging (aliased by xb) | exchange | material table | labels
@@ -199,19 +206,19 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_u(Dims d, T
                                                            float2* __restrict__ S0, float2* __restrict__ S1,
                                                            float2* __restrict__ S2) {
   using Z = ZShape<N>;
-  constexpr int A = Z::A, B = Z::B;
+  constexpr int A = Z::A, B = Z::B, OA = Z::OA, OB = Z::OB;
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
   float2* tw = sm;        // (A, B) order: inverse transforms
   float2* twf = sm + N;   // (B, A) order: forward transforms
   float4* stg4 = reinterpret_cast<float4*>(sm + Z::OFF_STG);
   float2* xb = sm + Z::OFF_STG;
-  cgf::fill_twt<A, B>(tw, t.twz);
-  cgf::fill_twt<B, A>(twf, t.twz);
+  cgf::fill_twt<A, B, OB>(tw, t.twz);
+  cgf::fill_twt<OB, OA, A>(twf, t.twz);
   cgf::pdl_wait();
   const int s = threadIdx.x & 15, p = threadIdx.x >> 4;
   const RowEx<A, B, true> exi{sm + Z::OFF_EX + p * Z::EX};  // 16 threads per pencil: warp-local
-  const RowEx<B, A, true> exf{sm + Z::OFF_EX + p * Z::EX};
+  const RowEx<OB, OA, true> exf{sm + Z::OFF_EX + p * Z::EX};
   const int ytiles = (d.ny + CG_ZROWS - 1) / CG_ZROWS;
   const int x = blockIdx.x / ytiles;
   const int y0 = (blockIdx.x - x * ytiles) * CG_ZROWS;
@@ -235,21 +242,21 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_u(Dims d, T
     float* uc = u + ((long long)comp * gridDim.y + b_idx) * d.ncell;
     z_stage<N>(stg4, S, d, x, y0, mk);
     // the velocities of this thread's cells load while the inverse transform runs
-    float ua[B], ub[B];
-    static_for<0, B>([&](auto bi) {
+    float ua[OB], ub[OB];
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
-      ua[b] = (s < A && va) ? __ldg(uc + rowa + n) : 0.f;
-      ub[b] = (s < A && vb) ? __ldg(uc + rowb + n) : 0.f;
+      const int n = s + OA * b;
+      ua[b] = (s < OA && va) ? __ldg(uc + rowa + n) : 0.f;
+      ub[b] = (s < OA && vb) ? __ldg(uc + rowb + n) : 0.f;
     });
     __syncthreads();
-    float2 v[A], w[B];
+    float2 v[A], w[OB];
     z_inputs<N>(v, stg4, p, s);
     fft2<A, B, true>(v, w, s, tw, exi);
     // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       const float sz = t.sz[n];
       float2 r = make_float2(0.f, 0.f);
       if (va) {
@@ -271,7 +278,7 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_u(Dims d, T
       w[b] = r;
     });
     float2 X[A];
-    fft2<B, A, false>(w, X, s, twf, exf);
+    fft2<OB, OA, false>(w, X, s, twf, exf);
     z_split_store<N, CG_TILE, true>(xb, X, S, d, x, y0, p, s, mk);
   }
 }
@@ -283,7 +290,7 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
                                                            int record, float* __restrict__ p_all,
                                                            float2* __restrict__ S0) {
   using Z = ZShape<N>;
-  constexpr int A = Z::A, B = Z::B;
+  constexpr int A = Z::A, B = Z::B, OA = Z::OA, OB = Z::OB;
   extern __shared__ float2 sm[];
   __shared__ unsigned int s_peak;
   float2* tw = sm;        // (A, B) order: inverse transforms
@@ -291,13 +298,13 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
   float4* stg4 = reinterpret_cast<float4*>(sm + Z::OFF_STG);
   float2* xb = sm + Z::OFF_STG;
   cgf::pdl_trigger();
-  cgf::fill_twt<A, B>(tw, t.twz);
-  cgf::fill_twt<B, A>(twf, t.twz);
+  cgf::fill_twt<A, B, OB>(tw, t.twz);
+  cgf::fill_twt<OB, OA, A>(twf, t.twz);
   cgf::pdl_wait();
   if (threadIdx.x == 0) s_peak = 0u;
   const int s = threadIdx.x & 15, p = threadIdx.x >> 4;
   const RowEx<A, B, true> exi{sm + Z::OFF_EX + p * Z::EX};  // 16 threads per pencil: warp-local
-  const RowEx<B, A, true> exf{sm + Z::OFF_EX + p * Z::EX};
+  const RowEx<OB, OA, true> exf{sm + Z::OFF_EX + p * Z::EX};
   const int ytiles = (d.ny + CG_ZROWS - 1) / CG_ZROWS;
   const int x = blockIdx.x / ytiles;
   const int y0 = (blockIdx.x - x * ytiles) * CG_ZROWS;
@@ -308,11 +315,11 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
   float* pb = p_all + (long long)b_idx * d.ncell;
   const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
   __syncthreads();
-  float2 w[B];
+  float2 w[OB];
   if constexpr (MODE == 0) {
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       w[b] = make_float2(va ? pb[rowa + n] : 0.f, vb ? pb[rowb + n] : 0.f);
     });
   } else {
@@ -323,12 +330,12 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
     const uint8_t* lb = la + N;
     z_stage<N>(stg4, S, d, x, y0, nullptr);
     // this thread's pressures load while the inverse transform runs
-    float pa[B], pbv[B];
-    static_for<0, B>([&](auto bi) {
+    float pa[OB], pbv[OB];
+    static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
-      pa[b] = (s < A && va) ? __ldg(pb + rowa + n) : 0.f;
-      pbv[b] = (s < A && vb) ? __ldg(pb + rowb + n) : 0.f;
+      const int n = s + OA * b;
+      pa[b] = (s < OA && va) ? __ldg(pb + rowa + n) : 0.f;
+      pbv[b] = (s < OA && vb) ? __ldg(pb + rowb + n) : 0.f;
     });
     __syncthreads();
     float2 v[A];
@@ -338,9 +345,9 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
     const float spx = t.sx[x];
     const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
     // p <- (p - (rho c^2 dt [+ 2 beta dt p]) div u) * absorb * sponge   (engine.py:470-477)
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       const float sz = t.sz[n];
       float2 r = make_float2(0.f, 0.f);
       if (va) {
@@ -360,19 +367,19 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
       w[b] = r;
     });
     // source (engine.py:478-482): entries of rows ya, yb owned by this thread
-    if (src.S > 0 && n_step < src.n_drive && s < A && va) {
+    if (src.S > 0 && n_step < src.n_drive && s < OA && va) {
       const float4 dr = src.drive[n_step];
       const int ra = x * d.ny + ya;
       const int e0 = src.row_ptr[ra], e1 = src.row_ptr[ra + 1], e2 = vb ? src.row_ptr[ra + 2] : e1;
       for (int e = e0; e < e2; ++e) {
         const int zz = src.zidx[e];
-        if (zz % A != s) continue;
-        const int k2 = zz / A;
+        if (zz % OA != s) continue;
+        const int k2 = zz / OA;
         const float acv = src.ac[(long long)b_idx * src.S + e];
         const float asv = src.as[(long long)b_idx * src.S + e];
         const float add = dr.x * (dr.y * acv - dr.z * asv);
         const bool on_b = e >= e1;
-        static_for<0, B>([&](auto bi) {
+        static_for<0, OB>([&](auto bi) {
           constexpr int b = decltype(bi)::value;
           if (k2 == b) {
             if (on_b) w[b].y += add;
@@ -390,9 +397,9 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
     float* bins = rec.bins + ((long long)b_idx * rec.spp + m_bin) * rec.nrec;
     float* comp = rec.comp + ((long long)b_idx * rec.spp + m_bin) * rec.nrec;
     float* pmax = rec.pmax + (long long)b_idx * rec.nrec;
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       for (int r = 0; r < 2; ++r) {
         const int y = r ? yb : ya;
         if (r ? !vb : !va) continue;
@@ -422,7 +429,7 @@ __global__ void __launch_bounds__(CG_THREADS, CG_FAST_MINB) kf_zpass_p(Dims d, T
     }
   }
   float2 X[A];
-  fft2<B, A, false>(w, X, s, twf, exf);
+  fft2<OB, OA, false>(w, X, s, twf, exf);
   z_split_store<N, CG_TILE, false>(xb, X, S, d, x, y0, p, s, nullptr);
 }
 
@@ -456,15 +463,15 @@ constexpr size_t zp_fit(int ctas) {  // bytes a CTA may use when `ctas` share an
 
 template <int N>
 struct ZPShape {
-  static constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, NH = N / 2 + 1;
+  static constexpr int A = ZSplit<N>::A, B = ZSplit<N>::B, OA = ZSplit<N>::OA, OB = ZSplit<N>::OB, NH = N / 2 + 1;
   static constexpr int TPP = ZSplit<N>::TPP;           // threads per pencil
-  static constexpr int P = N == 256 || TPP == 32 ? 16 : 8;  // pencils per tile
+  static constexpr int P = N == 256 || (TPP == 32 && !ZSplit<N>::P::THREE) ? 16 : 8;  // pencils per tile
   static constexpr int ROWS = 2 * P, THREADS = P * TPP, BOXES = P / 8;
   static constexpr bool WARP = (32 % TPP) == 0;  // a pencil's threads in one warp
   // the field values of a thread load before its inverse transform unless
   // the transform's A values per thread leave no registers for them
   static constexpr bool EARLY = A <= 20;
-  static constexpr int EX_I = RowEx<A, B>::SLAB, EX_F = RowEx<B, A>::SLAB;
+  static constexpr int EX_I = RowEx<A, B>::SLAB, EX_F = RowEx<OB, OA>::SLAB;
   static constexpr int EX = EX_I > EX_F ? EX_I : EX_F;
   // staged boxes, each on a 1024-byte boundary (the 128-byte swizzle repeats
   // every 8 rows), plus 1024 bytes to align the first one in the item buffer
@@ -485,15 +492,16 @@ struct ZPShape {
 };
 
 // Shared-memory layout of the u-pass (U) or the p-pass:
-// twiddles (two orders, one when A == B) | two item buffers | material table
+// twiddles (two orders, one where they are the same) | two item buffers | material table
 // (u: (dt/rho, absorb); p: the four coefficients) | k_z (u) | z sponge | two
 // label tiles | field rows (bulk copies) | mbarriers. Offsets in float2 units.
 template <int N, bool U, bool TMA>
 struct ZPLayout {
   using Z = ZPShape<N>;
   static constexpr bool BULK = TMA && Z::BULK;
-  static constexpr int TWF = Z::A == Z::B ? 0 : N;  // twiddles of the forward order
-  static constexpr size_t OFF_BUF = (Z::A == Z::B ? N : 2 * N) + (Z::A == Z::B ? N % 2 : 0);
+  static constexpr int TW = ZSplit<N>::TW;
+  static constexpr int TWF = Z::A == Z::OB ? 0 : TW;  // twiddles of the forward order
+  static constexpr size_t OFF_BUF = Z::A == Z::OB ? TW + TW % 2 : 2 * TW;
   static constexpr size_t OFF_TAB = OFF_BUF + 2 * (size_t)Z::BUF;
   static constexpr size_t OFF_KZ = OFF_TAB + (U ? 256 : 512);
   static constexpr size_t LABB = 2 * ((size_t)Z::ROWS * N + 16);  // bytes, slots on multiples of 16
@@ -670,8 +678,8 @@ template <int N, bool U, bool TMA>
 __device__ __forceinline__ void zp_tables(float2* sm, const Tables& t, const MediumDev& m) {
   using L = ZPLayout<N, U, TMA>;
   using Z = ZPShape<N>;
-  cgf::fill_twt<Z::A, Z::B>(sm, t.twz);
-  if (L::TWF) cgf::fill_twt<Z::B, Z::A>(sm + L::TWF, t.twz);
+  cgf::fill_twt<Z::A, Z::B, Z::OB>(sm, t.twz);
+  if (L::TWF) cgf::fill_twt<Z::OB, Z::OA, Z::A>(sm + L::TWF, t.twz);
   if (L::TBL) {
     if (U) {
       float* kz_s = reinterpret_cast<float*>(sm + L::OFF_KZ);
@@ -717,7 +725,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
                 const __grid_constant__ ZTma ztma) {
   using Z = ZPShape<N>;
   using L = ZPLayout<N, true, TMA>;
-  constexpr int A = Z::A, B = Z::B;
+  constexpr int A = Z::A, B = Z::B, OA = Z::OA, OB = Z::OB;
   extern __shared__ float2 sm[];
   const int ytiles = (d.ny + Z::ROWS - 1) / Z::ROWS;  // the last tile may be ragged
   cgf::pdl_trigger();
@@ -772,13 +780,13 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     float* uc = u + ((long long)comp * n_members + b_idx) * d.ncell;
     // this thread's velocities load while the staged spectrum is transformed
     // (after it where A-value registers would not leave room for them)
-    float ua[B], ub[B];
+    float ua[OB], ub[OB];
     auto load_u = [&]() {
-      static_for<0, B>([&](auto bi) {
+      static_for<0, OB>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
-        const int n = s + A * b;
-        ua[b] = (s < A && va) ? __ldg(uc + rowa + n) : 0.f;
-        ub[b] = (s < A && vb) ? __ldg(uc + rowb + n) : 0.f;
+        const int n = s + OA * b;
+        ua[b] = (s < OA && va) ? __ldg(uc + rowa + n) : 0.f;
+        ub[b] = (s < OA && vb) ? __ldg(uc + rowb + n) : 0.f;
       });
     };
     float* const rows = rows_of(cur);
@@ -792,28 +800,28 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     cur.next(n_members, ytiles);
     if (cur.x < d.nx) prefetch(cur, j ^ 1);
     float2* bufj = sm + L::OFF_BUF + (size_t)j * Z::BUF;
-    float2 v[A], w[B];
+    float2 v[A], w[OB];
     if constexpr (TMA) zt_wait(bars, phase, j, ztma.err);
     z_inputs_box<N>(v, zt_stage<N, L>(sm, j), p, s, comp == 2 ? kz_s : nullptr);
     __syncthreads();  // the staging is read: the buffer becomes the exchange
     const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
-    const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
+    const RowEx<OB, OA, Z::WARP> exf{bufj + p * Z::EX};
     fft2<A, B, true>(v, w, s, sm, exi);
     if (!Z::EARLY && !L::BULK) load_u();
     if constexpr (L::BULK) {
       zt_wait(bars, phase, 2, ztma.err);
-      static_for<0, B>([&](auto bi) {
+      static_for<0, OB>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
-        ua[b] = (s < A) ? fld[2 * p * N + s + A * b] : 0.f;
-        ub[b] = (s < A) ? fld[(2 * p + 1) * N + s + A * b] : 0.f;
+        ua[b] = (s < OA) ? fld[2 * p * N + s + OA * b] : 0.f;
+        ub[b] = (s < OA) ? fld[(2 * p + 1) * N + s + OA * b] : 0.f;
       });
     }
     const float spx = t.sx[x];
     const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
     // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       const float sz = sz_s[n];
       // (dt/rho, absorb) of the two cells
       const float2 ca = lab ? tab2_s[la[n]] : (va ? make_float2(m.dtr[rowa + n], m.ab[rowa + n]) : make_float2(0.f, 0.f));
@@ -839,7 +847,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
       if (threadIdx.x == 0) cgf::bulk_store(rows, fld, bytes);
     }
     float2 X[A];
-    fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+    fft2<OB, OA, false>(w, X, s, sm + L::TWF, exf);
     if constexpr (L::BULK)
       if (threadIdx.x == 0 && cur.x < d.nx) {  // cur: the next item
         cgf::bulk_wait_read();
@@ -865,7 +873,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
                 const __grid_constant__ ZTma ztma) {
   using Z = ZPShape<N>;
   using L = ZPLayout<N, false, TMA>;
-  constexpr int A = Z::A, B = Z::B;
+  constexpr int A = Z::A, B = Z::B, OA = Z::OA, OB = Z::OB;
   static_assert(!(FWD && (TMA || INV)), "the forward-only pass stages no spectrum");
   extern __shared__ float2 sm[];
   const int ytiles = (d.ny + Z::ROWS - 1) / Z::ROWS;  // the last tile may be ragged
@@ -874,10 +882,10 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
   unsigned phase = 0u;  // bit j: parity of item buffer j's next staging phase
   if constexpr (TMA) zt_init(bars);
   if constexpr (FWD) {
-    cgf::fill_twt<Z::B, Z::A>(sm + L::TWF, t.twz);
+    cgf::fill_twt<Z::OB, Z::OA, Z::A>(sm + L::TWF, t.twz);
     __syncthreads();
   } else if constexpr (INV) {
-    cgf::fill_twt<Z::A, Z::B>(sm, t.twz);
+    cgf::fill_twt<Z::A, Z::B, Z::OB>(sm, t.twz);
   } else {
     zp_tables<N, false, TMA>(sm, t, m);
   }
@@ -908,16 +916,16 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
       const bool va = ya < d.ny, vb = ya + 1 < d.ny;
       const float* pb = p_all + b_idx * d.ncell;
       const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
-      float2 w[B];
-      if (s < A) static_for<0, B>([&](auto bi) {
+      float2 w[OB];
+      if (s < OA) static_for<0, OB>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
-        const int n = s + A * b;
+        const int n = s + OA * b;
         w[b] = make_float2(va ? __ldg(pb + rowa + n) : 0.f, vb ? __ldg(pb + rowb + n) : 0.f);
       });
       float2* bufj = sm + L::OFF_BUF + (size_t)jf * Z::BUF;
-      const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
+      const RowEx<OB, OA, Z::WARP> exf{bufj + p * Z::EX};
       float2 X[A];
-      fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+      fft2<OB, OA, false>(w, X, s, sm + L::TWF, exf);
       z_split_store<N, Z::P, false>(bufj, X, S0 + b_idx * d.nspec, d, x, y0, p, s, nullptr);
     }
     return;
@@ -943,11 +951,11 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
   const long long Ry = rec.hi[1] - rec.lo[1], Rz = rec.hi[2] - rec.lo[2];
   const bool drive_on = src.S > 0 && n_step < src.n_drive;
   const float4 dr = drive_on ? src.drive[n_step] : make_float4(0.f, 0.f, 0.f, 0.f);
-  static_assert(B <= 32, "one mask bit per cell of a thread");
+  static_assert(OB <= 32, "one mask bit per cell of a thread");
   unsigned int zconv = 0u, zrec = 0u;  // bit b: this thread's cell z = s + A b is in the box
-  if (s < A) static_for<0, B>([&](auto bi) {
+  if (s < OA) static_for<0, OB>([&](auto bi) {
     constexpr int b = decltype(bi)::value;
-    const int n = s + A * b;
+    const int n = s + OA * b;
     if (n >= rec.clo[2] && n < rec.chi[2]) zconv |= 1u << b;
     if (n >= rec.lo[2] && n < rec.hi[2]) zrec |= 1u << b;
   });
@@ -965,13 +973,13 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
     // this thread's pressures load while the staged spectrum is transformed
     // (after it where A-value registers would not leave room for them)
-    float pa[B], pbv[B];
+    float pa[OB], pbv[OB];
     auto load_p = [&]() {
-      static_for<0, B>([&](auto bi) {
+      static_for<0, OB>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
-        const int n = s + A * b;
-        pa[b] = (s < A && va) ? __ldg(pb + rowa + n) : 0.f;
-        pbv[b] = (s < A && vb) ? __ldg(pb + rowb + n) : 0.f;
+        const int n = s + OA * b;
+        pa[b] = (s < OA && va) ? __ldg(pb + rowa + n) : 0.f;
+        pbv[b] = (s < OA && vb) ? __ldg(pb + rowb + n) : 0.f;
       });
     };
     float* const rows = rows_of(cur);
@@ -983,17 +991,17 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     cur.next(n_members, ytiles);
     if (cur.x < d.nx) prefetch(cur, j ^ 1);
     float2* bufj = sm + L::OFF_BUF + (size_t)j * Z::BUF;
-    float2 v[A], w[B];
+    float2 v[A], w[OB];
     if constexpr (TMA) zt_wait(bars, phase, j, ztma.err);
     z_inputs_box<N>(v, zt_stage<N, L>(sm, j), p, s, nullptr);
     __syncthreads();  // the staging is read: the buffer becomes the exchange
     const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
-    const RowEx<B, A, Z::WARP> exf{bufj + p * Z::EX};
+    const RowEx<OB, OA, Z::WARP> exf{bufj + p * Z::EX};
     fft2<A, B, true>(v, w, s, sm, exi);
     if constexpr (INV) {
-      if (s < A) static_for<0, B>([&](auto bi) {
+      if (s < OA) static_for<0, OB>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
-        const int n = s + A * b;
+        const int n = s + OA * b;
         if (va) pb[rowa + n] = w[b].x;
         if (vb) pb[rowb + n] = w[b].y;
       });
@@ -1002,18 +1010,18 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     if (!Z::EARLY && !L::BULK) load_p();
     if constexpr (L::BULK) {
       zt_wait(bars, phase, 2, ztma.err);
-      static_for<0, B>([&](auto bi) {
+      static_for<0, OB>([&](auto bi) {
         constexpr int b = decltype(bi)::value;
-        pa[b] = (s < A) ? fld[2 * p * N + s + A * b] : 0.f;
-        pbv[b] = (s < A) ? fld[(2 * p + 1) * N + s + A * b] : 0.f;
+        pa[b] = (s < OA) ? fld[2 * p * N + s + OA * b] : 0.f;
+        pbv[b] = (s < OA) ? fld[(2 * p + 1) * N + s + OA * b] : 0.f;
       });
     }
     const float spx = t.sx[x];
     const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
     // p <- (p - (rho c^2 dt [+ 2 beta dt p]) div u) * absorb * sponge   (engine.py:470-477)
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       const float sz = sz_s[n];
       const float4 ca = lab ? tab_s[la[n]] : (va ? cell_coef(m, rowa + n) : make_float4(0.f, 0.f, 0.f, 0.f));
       const float4 cb = lab ? tab_s[lb[n]] : (vb ? cell_coef(m, rowb + n) : make_float4(0.f, 0.f, 0.f, 0.f));
@@ -1027,18 +1035,18 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
       w[b] = make_float2(__fmul_rn(pna, spa * sz), vb ? __fmul_rn(pnb, spb * sz) : 0.f);
     });
     // source (engine.py:478-482): entries of rows ya, yb owned by this thread
-    if (drive_on && s < A && va) {
+    if (drive_on && s < OA && va) {
       const int ra = x * d.ny + ya;
       const int e0 = src.row_ptr[ra], e1 = src.row_ptr[ra + 1], e2 = vb ? src.row_ptr[ra + 2] : e1;
       for (int e = e0; e < e2; ++e) {
         const int zz = src.zidx[e];
-        if (zz % A != s) continue;
-        const int k2 = zz / A;
+        if (zz % OA != s) continue;
+        const int k2 = zz / OA;
         const float acv = src.ac[b_idx * src.S + e];
         const float asv = src.as[b_idx * src.S + e];
         const float add = dr.x * (dr.y * acv - dr.z * asv);
         const bool on_b = e >= e1;
-        static_for<0, B>([&](auto bi) {
+        static_for<0, OB>([&](auto bi) {
           constexpr int b = decltype(bi)::value;
           if (k2 == b) {
             if (on_b) w[b].y += add;
@@ -1056,9 +1064,9 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     const bool conv_b = x_conv && vb && yb >= rec.clo[1] && yb < rec.chi[1];
     const bool rec_a = x_rec && va && ya >= rec.lo[1] && ya < rec.hi[1];
     const bool rec_b = x_rec && vb && yb >= rec.lo[1] && yb < rec.hi[1];
-    if (s < A) static_for<0, B>([&](auto bi) {
+    if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
-      const int n = s + A * b;
+      const int n = s + OA * b;
       const float pna = w[b].x, pnb = w[b].y;
       if constexpr (L::BULK) {
         fld[2 * p * N + n] = pna;
@@ -1077,19 +1085,19 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
       // thread's recorded cells, RC cells per row at a time: every load of a
       // chunk is issued before its first store, so the chunk costs one round
       // trip to memory instead of one per cell
-      if (s < A && (rec_a || rec_b)) {
+      if (s < OA && (rec_a || rec_b)) {
         float* __restrict__ bins = rec.bins + (b_idx * rec.spp + m_bin) * rec.nrec;
         float* __restrict__ comp = rec.comp + (b_idx * rec.spp + m_bin) * rec.nrec;
         float* __restrict__ pmax = rec.pmax + b_idx * rec.nrec;
         const long long ra = ((long long)(x - rec.lo[0]) * Ry + (ya - rec.lo[1])) * Rz - rec.lo[2];
         const long long rb = ra + Rz;  // row yb = ya + 1
-        constexpr int RC = B % 4 == 0 ? 4 : (B % 5 == 0 ? 5 : (B % 3 == 0 ? 3 : (B % 2 == 0 ? 2 : 1)));
-        static_for<0, B / RC>([&](auto ci) {
+        constexpr int RC = OB % 4 == 0 ? 4 : (OB % 5 == 0 ? 5 : (OB % 3 == 0 ? 3 : (OB % 2 == 0 ? 2 : 1)));
+        static_for<0, OB / RC>([&](auto ci) {
           constexpr int c0 = decltype(ci)::value * RC;
           float sv[2 * RC], cm[2 * RC], pm[2 * RC];
           static_for<0, RC>([&](auto ji) {
             constexpr int j = decltype(ji)::value, b = c0 + j;
-            const int n = s + A * b;
+            const int n = s + OA * b;
             const bool in = (zrec >> b) & 1u;
             sv[j] = (in && rec_a) ? bins[ra + n] : 0.f;
             cm[j] = (in && rec_a) ? comp[ra + n] : 0.f;
@@ -1100,7 +1108,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
           });
           static_for<0, RC>([&](auto ji) {
             constexpr int j = decltype(ji)::value, b = c0 + j;
-            const int n = s + A * b;
+            const int n = s + OA * b;
             if (!((zrec >> b) & 1u)) return;
             for (int r = 0; r < 2; ++r) {
               if (r ? !rec_b : !rec_a) continue;
@@ -1134,7 +1142,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
       if (threadIdx.x == 0) cgf::bulk_store(rows, fld, bytes);
     }
     float2 X[A];
-    fft2<B, A, false>(w, X, s, sm + L::TWF, exf);
+    fft2<OB, OA, false>(w, X, s, sm + L::TWF, exf);
     if constexpr (L::BULK)
       if (threadIdx.x == 0 && cur.x < d.nx) {  // cur: the next tile
         cgf::bulk_wait_read();
