@@ -96,15 +96,68 @@ __host__ __device__ __forceinline__ float2 rot(float2 a) {  // forward: -i a ; i
   return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
+constexpr int ct_gcd(int a, int b) { return b == 0 ? a : ct_gcd(b, a % b); }
+// Largest power of the smallest prime factor of R: coprime to the rest.
+constexpr int ct_prime_power(int R) {
+  const int p = R % 2 == 0 ? 2 : (R % 3 == 0 ? 3 : 5);
+  int q = 1;
+  while (R % p == 0) {
+    q *= p;
+    R /= p;
+  }
+  return q;
+}
 constexpr int ct_first_factor(int R) {
-  return (R % 4 == 0 && R > 8) ? 4 : (R % 2 == 0 ? 2 : (R % 3 == 0 ? 3 : 5));
+  const int q = ct_prime_power(R);
+  return q < R ? q : ((R % 4 == 0 && R > 8) ? 4 : (R % 2 == 0 ? 2 : (R % 3 == 0 ? 3 : 5)));
+}
+// The k < A B with k = k1 mod A and k = k2 mod B (A, B coprime).
+constexpr int ct_crt(int k1, int k2, int A, int B) {
+  int k = k1;
+  while (k % B != k2) k += A;
+  return k;
 }
 
 // ------------------------------------------------------- DFT codelets --
+// Composite sizes of coprime factors A, B by the prime-factor algorithm (Good
+// 1958, Thomas 1963): n = (B n1 + A n2) mod R, k = k1 mod A = k2 mod B, an A x B
+// transform without twiddles; the permutations are register names. Powers of
+// one prime by Cooley and Tukey's, with twiddles in between. A step with twiddles
+// everywhere -> as it is: 192x192x256 275.7 -> 274.6 us, 320^3 1182 -> 1165,
+// 384^3 1946 -> 1895, 400^3 2173 -> 2111; the error of a round trip against 64
+// bits 1.86e-7 -> 1.79e-7 at 180 points, 2.05e-7 -> 1.89e-7 at 400.
 template <int R, bool INV>
 struct Dft {
   static constexpr int A = ct_first_factor(R), B = R / A;
+  static constexpr bool COPRIME = ct_gcd(A, B) == 1;
   __host__ __device__ __forceinline__ static void run(float2* v) {
+    if constexpr (COPRIME)
+      run_coprime(v);
+    else
+      run_twiddled(v);
+  }
+  __host__ __device__ __forceinline__ static void run_coprime(float2* v) {
+    float2 o[R];  // o[B k1 + n2], then o[B k1 + k2]
+    static_for<0, B>([&](auto ni) {
+      constexpr int n2 = decltype(ni)::value;
+      float2 t[A];
+      static_for<0, A>([&](auto mi) {
+        constexpr int n1 = decltype(mi)::value;
+        t[n1] = v[(B * n1 + A * n2) % R];
+      });
+      Dft<A, INV>::run(t);
+      static_for<0, A>([&](auto ki) { o[B * decltype(ki)::value + n2] = t[decltype(ki)::value]; });
+    });
+    static_for<0, A>([&](auto ki) { Dft<B, INV>::run(o + B * decltype(ki)::value); });
+    static_for<0, A>([&](auto k1i) {
+      static_for<0, B>([&](auto k2i) {
+        constexpr int k1 = decltype(k1i)::value, k2 = decltype(k2i)::value;
+        constexpr int k = ct_crt(k1, k2, A, B);
+        v[k] = o[B * k1 + k2];
+      });
+    });
+  }
+  __host__ __device__ __forceinline__ static void run_twiddled(float2* v) {
     static_for<0, B>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       float2 t[A];
@@ -218,7 +271,6 @@ struct Dft<8, INV> {
 
 // ------------------------------------------------ two-level transform --
 // Split of a pencil length N into (A, B): B = gcd(N, 16), A = N / B.
-constexpr int ct_gcd(int a, int b) { return b == 0 ? a : ct_gcd(b, a % b); }
 template <int N>
 struct Split {
   static constexpr int B = ct_gcd(N, 16);
