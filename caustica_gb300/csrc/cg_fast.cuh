@@ -356,9 +356,12 @@ struct RowEx {
 template <int A, int B, int P = 16>
 struct ColEx {
   float2* base;  // + lane pencil
-  static constexpr int SLAB = 0;
+  // below 16 columns a row is part of the banks: an odd row count puts the rows
+  // s and s + 1 that a warp reads together on different ones
+  static constexpr int LD = P < 16 ? ct_odd(B) : B;
+  static constexpr int SLAB = A * LD * P;
   static constexpr bool kWarp = false;  // a column pencil spans the whole block
-  __device__ __forceinline__ float2& at(int k1, int n2) const { return base[(k1 * B + n2) * P]; }
+  __device__ __forceinline__ float2& at(int k1, int n2) const { return base[(k1 * LD + n2) * P]; }
 };
 
 template <class Ex>
@@ -442,9 +445,9 @@ __device__ __forceinline__ void fft3(const float2 (&v_in)[V], float2 (&w)[V], in
 
 // (A, B) transform of one pencil: thread s (< B) holds v[a] = x[s + B a];
 // afterwards thread s (< A) holds w[b] = X[s + A b], or, in three levels, s (<
-// B) w[a] = X[s + B a]. `twt` is the table laid out by fill_twt. Every thread
-// of the block calls it.
-template <int A, int B, bool INV, class Ex, int R>
+// B) w[a] = X[s + B a]. `twt` is the table laid out by fill_twt, or (TR) that of
+// the (B, A) transform. Every thread of the block calls it.
+template <int A, int B, bool INV, bool TR = false, class Ex, int R>
 __device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[R], int s, const float2* __restrict__ twt,
                                      const Ex& ex) {
   if constexpr (R != B) {
@@ -459,7 +462,7 @@ __device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[R], in
         constexpr int k1 = decltype(ki)::value;
         float2 y = v[k1];
         if constexpr (k1 > 0) {
-          float2 t = twt[k1 * B + s];
+          float2 t = twt[TR ? s * A + k1 : k1 * B + s];
           if (INV) t.y = -t.y;
           y = c_mul(y, t);
         }

@@ -71,6 +71,15 @@ struct YT {
 template <int N>
 struct XT {
   static constexpr int TPP = PSplit<N>::TPP, XP = TPP > 16 ? CG_XP20 : CG_XP, THREADS = TPP * XP;
+  using S = PSplit<N>;
+  static constexpr int EX_F = ColEx<S::A, S::B, XP>::SLAB, EX_I = ColEx<S::OB, S::OA, XP>::SLAB;
+  static constexpr int EX = EX_F > EX_I ? EX_F : EX_I;  // the exchange tile
+  // the (OB, OA) twiddles: the (A, B) ones where the two orders are the same, or
+  // read across (TR) unless the few rows s of a warp then share their banks
+  // (with padded exchange rows, X_GRAD / X_DIV us: 400^3 285 / 294 -> 266 / 275,
+  // 324^3 173 / 174 -> 162 / 164, 144x180x192 25.4 / 26.6 -> 25.0 / 24.6)
+  static constexpr bool TR = S::A != S::OB && S::OB % 16 != 0;
+  static constexpr int TABLES = S::A == S::OB || TR ? 1 : 2;
   static constexpr int minb(int mode) {
     if (TPP <= 16) return 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X);
     if (PSplit<N>::THREE) return PSplit<N>::A <= 10 ? 4 : 3;
@@ -92,7 +101,14 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
   float2* tw = sm;  // (A, B) order
-  cgf::fill_twt<A, B, OB>(tw, t.twy);
+  // The first row loads while the twiddles are put in place (us, row first /
+  // tables first: 400^3 Y_FWD 88 / 92, Y_INV_GRAD 221 / 227, 160x160x192 x 8
+  // Y_FWD_DIV 129 / 134; a 100x125x135 step 94 / 99). Tables first, before the wait
+  // for the pass before, where that pass is an x-pass and this one is launched
+  // programmatically (y_pdl; 192x192x256 274.6 us a step against 276.3) and on
+  // the smallest grids (64^3 27.6 against 29.3).
+  constexpr bool FIRST = TPP > 16 || (TPP == 16 && (MODE == Y_FWD || MODE == Y_FWD_DIV || N > 192));
+  if (!FIRST) cgf::fill_twt<A, B, OB>(tw, t.twy);
   cgf::pdl_wait();
   const int s = threadIdx.x % TPP, p = threadIdx.x / TPP;
   const Ex ex{sm + TW + p * Ex::SLAB};
@@ -100,7 +116,6 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
   const long long row = (long long)blockIdx.x * YT<N>::YP + p;
   const bool valid = row < nrows;
   const long long off = (long long)blockIdx.y * d.nspec + row * N;
-  __syncthreads();
   float2 v[A], w[OB];
   auto load = [&](const float2* __restrict__ src) {
     static_for<0, A>([&](auto ai) {
@@ -114,13 +129,17 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
       dst[off + s + OA * b] = w[b];
     });
   };
+  if (!FIRST) __syncthreads();
+  load(MODE == Y_FWD || MODE == Y_INV ? S0 : S1);
+  if (FIRST) {
+    cgf::fill_twt<A, B, OB>(tw, t.twy);
+    __syncthreads();
+  }
   if constexpr (MODE == Y_FWD || MODE == Y_INV) {
-    load(S0);
     fft2<A, B, MODE == Y_INV>(v, w, s, tw, ex);
     store(S0);
   } else if constexpr (MODE == Y_INV_GRAD) {
     // S1 <- IFFT(S1); S0 <- IFFT(i ky S2); S2 <- IFFT(S2)
-    load(S1);
     fft2<A, B, true>(v, w, s, tw, ex);
     store(S1);
     load(S2);
@@ -136,7 +155,6 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
     store(S2);
   } else {
     // Y_FWD_DIV: S1 <- FFT(S1); S0 <- i ky FFT(S0) + FFT(S2)
-    load(S1);
     fft2<A, B, false>(v, w, s, tw, ex);
     store(S1);
     load(S0);
@@ -257,19 +275,21 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
                 XP = XT<N>::XP;
   extern __shared__ float2 sm[];
   cgf::pdl_trigger();
-  float2* tw = sm;        // (A, B) order
-  float2* twi = sm + TW;  // (OB, OA) order
+  constexpr bool TR = XT<N>::TR;
+  constexpr int XB = XT<N>::TABLES * TW;  // behind the twiddles
+  float2* tw = sm;                        // (A, B) order
+  float2* twi = sm + (XB - TW);           // (OB, OA) order, or the one table
+  float* kxs = reinterpret_cast<float*>(sm + XB + XT<N>::EX + N * XP);  // k_x | k_x^2
   cgf::fill_twt<A, B, OB>(tw, t.twx);
-  cgf::fill_twt<OB, OA, A>(twi, t.twx);
-  float* kxs = reinterpret_cast<float*>(sm + 2 * TW + 2 * N * XP);  // k_x | k_x^2
+  if (XT<N>::TABLES == 2) cgf::fill_twt<OB, OA, A>(twi, t.twx);
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     kxs[i] = t.kx[i];
     kxs[N + i] = t.kx2[i];
   }
   cgf::pdl_wait();
   const int c = threadIdx.x % XP, s = threadIdx.x / XP;
-  const ColEx<A, B, XP> exf{sm + 2 * TW + c};
-  const ColEx<OB, OA, XP> exi{sm + 2 * TW + c};
+  const ColEx<A, B, XP> exf{sm + XB + c};
+  const ColEx<OB, OA, XP> exi{sm + XB + c};
   const long long ncol = (long long)d.nzh * d.ny;
   const long long col = (long long)blockIdx.x * XP + c;
   const bool valid = col < ncol;
@@ -281,7 +301,6 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
     const int ky = (int)(cc - (unsigned)kz * (unsigned)d.ny);
     kyz2 = t.ky2[ky] + t.kz2[kz];
   }
-  __syncthreads();
   float2 v[A], w[OB], z[A];
   auto load = [&](const float2* __restrict__ src) {
     static_for<0, A>([&](auto ai) {
@@ -306,8 +325,11 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
     });
   };
   auto kappa = [&](int k) { return sinc_a2(kcoef * (kxs[N + k] + kyz2)) * invN; };
+  // above 16 threads a pencil the first tile's loads need not wait for the tables
+  if (XT<N>::TPP <= 16) __syncthreads();
+  load(MODE == X_GRAD ? S0 : S1);
+  if (XT<N>::TPP > 16) __syncthreads();
   if constexpr (MODE == X_FWD || MODE == X_INV) {  // S0 <- (I)FFT(S1); S1 may be S0
-    load(S1);
     fft2<A, B, MODE == X_INV>(v, w, s, tw, exf);
     if (valid && s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
@@ -316,8 +338,7 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
   } else if constexpr (MODE == X_GRAD) {
     // S2 <- IFFT(q); S1 <- IFFT(i kx q), q = kappa/N FFT(S0); q waits in shared
     // memory during the first inverse transform instead of in registers
-    float2* qs = sm + 2 * TW + N * XP;
-    load(S0);
+    float2* qs = sm + XB + XT<N>::EX;
     fft2<A, B, false>(v, w, s, tw, exf);
     static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
@@ -325,19 +346,18 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
       w[b] = c_scale(w[b], kappa(k));
       if (s < OA) qs[(s + OA * b) * XP + c] = w[b];
     });
-    fft2<OB, OA, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true, TR>(w, z, s, twi, exi);
     store_z(S2);
     static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int k = (s < OA) ? s + OA * b : 0;
       w[b] = (s < OA) ? c_muli(c_scale(qs[(s + OA * b) * XP + c], kxs[k])) : make_float2(0.f, 0.f);
     });
-    fft2<OB, OA, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true, TR>(w, z, s, twi, exi);
     store_z(S1);
   } else {
     // X_DIV: S0 <- IFFT(kappa/N (FFT(S0) + i kx FFT(S1))); FFT(S1) waits in shared memory
-    float2* hs = sm + 2 * TW + N * XP;
-    load(S1);
+    float2* hs = sm + XB + XT<N>::EX;
     fft2<A, B, false>(v, w, s, tw, exf);
     if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
@@ -351,7 +371,7 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
       const float2 h = (s < OA) ? hs[(s + OA * b) * XP + c] : make_float2(0.f, 0.f);
       w[b] = c_scale(c_add(w[b], c_muli(c_scale(h, kxs[k]))), kappa(k));
     });
-    fft2<OB, OA, true>(w, z, s, twi, exi);
+    fft2<OB, OA, true, TR>(w, z, s, twi, exi);
     store_z(S0);
   }
 }
@@ -363,7 +383,7 @@ static size_t smem_y() {
 }
 template <int N>
 static size_t smem_x() {
-  return sizeof(float2) * (2 * PSplit<N>::TW + 2 * (size_t)N * XT<N>::XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
+  return sizeof(float2) * (XT<N>::TABLES * PSplit<N>::TW + XT<N>::EX + (size_t)N * XT<N>::XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
 }
 
 // ------------------------------------------------ per-length launchers --
