@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, 
 // FFT(S2 + 0 S1)))). The zero multiples carry a non-finite u_x or p over, as
 // the products with k_x = 0 do. Bound: launch latency (a 135x192 step takes
 // 34 us in eight launches, the arithmetic of one fits in two); four launches a
-// step take 17 us. Rows as in the y-pass.
+// step take 28 us. Rows as in the y-pass.
 template <int N, bool DIV>
 __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, float kcoef, float invN,
                                                               float2* __restrict__ S0, float2* __restrict__ S1,
@@ -195,7 +195,12 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
   float2* twi = sm + TW;  // (OB, OA) order
   cgf::fill_twt<A, B, OB>(tw, t.twy);
   cgf::fill_twt<OB, OA, A>(twi, t.twy);
-  cgf::pdl_wait();
+  // k_y | k_y^2, ready before the wait: a 135x192 step 32.7 -> 27.9 us, 64x96 16.4 -> 13.7
+  float* kys = reinterpret_cast<float*>(sm + 2 * TW + YT<N>::YP * SLAB);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    kys[i] = t.ky[i];
+    kys[N + i] = t.ky2[i];
+  }
   const int s = threadIdx.x % TPP, p = threadIdx.x / TPP;
   const ExF exf{sm + 2 * TW + p * SLAB};
   const ExI exi{sm + 2 * TW + p * SLAB};
@@ -203,6 +208,7 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
   const bool valid = row < d.nzh;
   const long long off = (long long)blockIdx.y * d.nspec + (long long)row * N;
   const float kz2 = valid ? t.kz2[row] : 0.f;
+  cgf::pdl_wait();
   __syncthreads();
   float2 v[A], w[OB], z[A];
   auto load = [&](const float2* src) {
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
       dst[off + s + B * a] = z[a];
     });
   };
-  auto kappa = [&](int k) { return sinc_a2(kcoef * (t.ky2[k] + kz2)) * invN; };
+  auto kappa = [&](int k) { return sinc_a2(kcoef * (kys[N + k] + kz2)) * invN; };
   if constexpr (!DIV) {
     load(S0);
     fft2<A, B, false>(v, w, s, tw, exf);
@@ -226,7 +232,7 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
       constexpr int b = decltype(bi)::value;
       const int k = (s < OA) ? s + OA * b : 0;
       w[b] = c_scale(w[b], kappa(k));
-      g[b] = c_muli(c_scale(w[b], t.ky[k]));
+      g[b] = c_muli(c_scale(w[b], kys[k]));
     });
     fft2<OB, OA, true>(g, z, s, twi, exi);
     store_z(S0);
@@ -241,7 +247,7 @@ __global__ void __launch_bounds__(YT<N>::THREADS, 4) kf_plane(Dims d, Tables t, 
     static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
       const int k = (s < OA) ? s + OA * b : 0;
-      h[b] = c_muli(c_scale(w[b], t.ky[k]));
+      h[b] = c_muli(c_scale(w[b], kys[k]));
     });
     load(S2);
     static_for<0, A>([&](auto ai) {
@@ -263,7 +269,8 @@ template <int N>
 static size_t smem_plane() {
   using F = RowEx<YSplit<N>::A, YSplit<N>::B>;
   using I = RowEx<YSplit<N>::OB, YSplit<N>::OA>;
-  return sizeof(float2) * (2 * YSplit<N>::TW + YT<N>::YP * (F::SLAB > I::SLAB ? F::SLAB : I::SLAB));
+  return sizeof(float2) * (2 * YSplit<N>::TW + YT<N>::YP * (F::SLAB > I::SLAB ? F::SLAB : I::SLAB)) +
+         2 * sizeof(float) * N;  // + k_y, k_y^2
 }
 
 template <int N, int MODE>

@@ -791,6 +791,9 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     };
     float* const rows = rows_of(cur);
     const unsigned bytes = rows_bytes(cur);
+    // the sponge's x and y factors, read ahead of the transform (192x192x256 97.1 ->
+    // 93.0 us, 160x160x192 x 8 375 -> 369; lengths of 20 threads the same)
+    const float spx = t.sx[x], sya = va ? t.sy[ya] : 0.f, syb = vb ? t.sy[yb] : 0.f;
     if (Z::EARLY && !L::BULK) load_u();
     // (tensor-map path) this thread's generic accesses to the buffer the
     // next copy fills are ordered before that copy
@@ -816,8 +819,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
         ub[b] = (s < OA) ? fld[(2 * p + 1) * N + s + OA * b] : 0.f;
       });
     }
-    const float spx = t.sx[x];
-    const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
+    const float spa = spx * sya, spb = spx * syb;
     // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
     if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
@@ -984,6 +986,17 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     };
     float* const rows = rows_of(cur);
     const unsigned bytes = rows_bytes(cur);
+    // the sponge's x and y factors, read ahead of the transform where 16 threads
+    // hold the cells (192x192x256 41.0 -> 39.4 us, 160x160x192 x 8 148 -> 144); else
+    // they would spill (300^3 138 -> 148, 150^3 24.6 -> 26.0)
+    constexpr bool SP = A == 16 && !INV;
+    float spx = 0.f, sya = 0.f, syb = 0.f;
+    auto sponge_xy = [&]() {
+      spx = t.sx[x];
+      sya = va ? t.sy[ya] : 0.f;
+      syb = vb ? t.sy[yb] : 0.f;
+    };
+    if (SP) sponge_xy();
     if (Z::EARLY && !INV && !L::BULK) load_p();
     if constexpr (TMA) cgf::fence_proxy_async();  // see the u-pass
     cgf::cp_async_wait0();
@@ -1016,8 +1029,8 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
         pbv[b] = (s < OA) ? fld[(2 * p + 1) * N + s + OA * b] : 0.f;
       });
     }
-    const float spx = t.sx[x];
-    const float spa = va ? spx * t.sy[ya] : 0.f, spb = vb ? spx * t.sy[yb] : 0.f;
+    if (!SP) sponge_xy();
+    const float spa = spx * sya, spb = spx * syb;
     // p <- (p - (rho c^2 dt [+ 2 beta dt p]) div u) * absorb * sponge   (engine.py:470-477)
     if (s < OA) static_for<0, OB>([&](auto bi) {
       constexpr int b = decltype(bi)::value;
