@@ -674,6 +674,16 @@ __device__ __forceinline__ void z_inputs_box(float2 (&v)[ZSplit<N>::A], const ch
   });
 }
 
+// Cells of a row that a thread reads at a time, of its B: all loads of a chunk
+// before its first store, which the compiler will not move a load across. (A
+// dense medium's coefficients, u- / p-pass us, a cell at a time -> in chunks:
+// 192x192x256 170 / 67 -> 108 / 57, 150^3 76 / 39 -> 50 / 31.)
+constexpr int z_chunk(int B) { return B % 4 == 0 ? 4 : (B % 5 == 0 ? 5 : (B % 3 == 0 ? 3 : (B % 2 == 0 ? 2 : 1))); }
+// A dense medium's coefficients of the p-pass: (-, rho c^2 dt, absorb, 2 beta dt).
+__device__ __forceinline__ float4 z_dense_p(const MediumDev& m, long long i) {
+  return make_float4(0.f, __ldg(m.rc2 + i), __ldg(m.ab + i), m.b2 ? __ldg(m.b2 + i) : 0.f);
+}
+
 template <int N, bool U, bool TMA>
 __device__ __forceinline__ void zp_tables(float2* sm, const Tables& t, const MediumDev& m) {
   using L = ZPLayout<N, U, TMA>;
@@ -718,7 +728,10 @@ __device__ __forceinline__ void zt_init(unsigned long long* bars) {
 // TMA: the tile's half spectra arrive by tensor-map box copies (ztma: the
 // descriptors, by value) instead of per-thread cp.async; the labels keep
 // cp.async. Other instantiations ignore ztma.
-template <int N, bool TMA = false>
+// DENSE: the medium is maps, not labels. Instantiations of their own, for the
+// registers: u- / p-pass us with labels, both in one kernel -> apart: 400^3 677 /
+// 259 -> 637 / 240, 300^3 344 / 137 -> 330 / 132.
+template <int N, bool TMA = false, bool DENSE = false>
 __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::MINB)
     kfp_zpass_u(Dims d, Tables t, MediumDev m, float* __restrict__ u, float2* __restrict__ S0,
                 float2* __restrict__ S1, float2* __restrict__ S2, int n_members,
@@ -738,7 +751,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
   const float* sz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_SZ) : t.sz;
   const float2* tab2_s = sm + L::OFF_TAB;
   uint8_t* lab0 = reinterpret_cast<uint8_t*>(sm + L::OFF_LAB);
-  const bool lab = m.labels != nullptr;
+  constexpr bool lab = !DENSE;
   const int s = threadIdx.x % Z::TPP, p = threadIdx.x / Z::TPP;
   auto spec = [&](int comp, long long b) { return (comp == 0 ? S1 : (comp == 1 ? S0 : S2)) + b * d.nspec; };
   auto prefetch = [&](const ZCursor<3>& c, int j) {
@@ -749,7 +762,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     } else {
       z_prefetch<N>(stg, spec(c.comp, c.b), d, c.x, y0);
     }
-    if (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
+    if constexpr (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
     cgf::cp_async_commit();
   };
   ZCursor<3> cur(n_members, ytiles);
@@ -821,13 +834,11 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     }
     const float spa = spx * sya, spb = spx * syb;
     // u <- (u - dt/rho g) * absorb * sponge   (engine.py:462-464)
-    if (s < OA) static_for<0, OB>([&](auto bi) {
+    // ca, cb: (dt/rho, absorb) of cells n of the two rows
+    auto update = [&](auto bi, float2 ca, float2 cb) {
       constexpr int b = decltype(bi)::value;
       const int n = s + OA * b;
       const float sz = sz_s[n];
-      // (dt/rho, absorb) of the two cells
-      const float2 ca = lab ? tab2_s[la[n]] : (va ? make_float2(m.dtr[rowa + n], m.ab[rowa + n]) : make_float2(0.f, 0.f));
-      const float2 cb = lab ? tab2_s[lb[n]] : (vb ? make_float2(m.dtr[rowb + n], m.ab[rowb + n]) : make_float2(0.f, 0.f));
       float una = ua[b] - ca.x * w[b].x;
       una = una * ca.y;
       una = una * (spa * sz);
@@ -842,7 +853,29 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
         if (vb) uc[rowb + n] = unb;
       }
       w[b] = make_float2(una, vb ? unb : 0.f);
-    });
+    };
+    if constexpr (lab) {
+      if (s < OA) static_for<0, OB>([&](auto bi) {
+        const int n = s + OA * decltype(bi)::value;
+        update(bi, tab2_s[la[n]], tab2_s[lb[n]]);
+      });
+    } else if (s < OA) {
+      constexpr int RC = z_chunk(OB);
+      static_for<0, OB / RC>([&](auto ci) {
+        constexpr int c0 = decltype(ci)::value * RC;
+        float2 ca[RC], cb[RC];
+        static_for<0, RC>([&](auto ji) {
+          constexpr int j = decltype(ji)::value;
+          const int n = s + OA * (c0 + j);
+          ca[j] = va ? make_float2(__ldg(m.dtr + rowa + n), __ldg(m.ab + rowa + n)) : make_float2(0.f, 0.f);
+          cb[j] = vb ? make_float2(__ldg(m.dtr + rowb + n), __ldg(m.ab + rowb + n)) : make_float2(0.f, 0.f);
+        });
+        static_for<0, RC>([&](auto ji) {
+          constexpr int j = decltype(ji)::value;
+          update(std::integral_constant<int, c0 + j>{}, ca[j], cb[j]);
+        });
+      });
+    }
     if constexpr (L::BULK) {
       cgf::fence_proxy_async();
       __syncthreads();
@@ -868,7 +901,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
 // the very code the step runs, so a restored run continues bit for bit.
 // INV: only the opening inverse transform, its values to the pressure.
 // TMA: the half spectra arrive by tensor-map box copies (as in the u-pass).
-template <int N, bool REC, bool FWD = false, bool TMA = false, bool INV = false>
+template <int N, bool REC, bool FWD = false, bool TMA = false, bool INV = false, bool DENSE = false>
 __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::MINB)
     kfp_zpass_p(Dims d, Tables t, MediumDev m, SourceDev src, RecordDev rec, const long long* ctl, int n_local,
                 int record, float* __restrict__ p_all, float2* __restrict__ S0, int n_members,
@@ -895,7 +928,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
   const float* sz_s = L::TBL ? reinterpret_cast<const float*>(sm + L::OFF_SZ) : t.sz;
   const float4* tab_s = reinterpret_cast<const float4*>(sm + L::OFF_TAB);
   uint8_t* lab0 = reinterpret_cast<uint8_t*>(sm + L::OFF_LAB);
-  const bool lab = !INV && m.labels != nullptr;
+  constexpr bool lab = !INV && !DENSE;
   const int s = threadIdx.x % Z::TPP, p = threadIdx.x / Z::TPP;
   auto prefetch = [&](const ZCursor<1>& c, int j) {
     const int y0 = c.yt * Z::ROWS;
@@ -905,7 +938,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     } else {
       z_prefetch<N>(stg, S0 + c.b * d.nspec, d, c.x, y0);
     }
-    if (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
+    if constexpr (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
     cgf::cp_async_commit();
   };
   ZCursor<1> cur(n_members, ytiles);
@@ -1032,12 +1065,11 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
     if (!SP) sponge_xy();
     const float spa = spx * sya, spb = spx * syb;
     // p <- (p - (rho c^2 dt [+ 2 beta dt p]) div u) * absorb * sponge   (engine.py:470-477)
-    if (s < OA) static_for<0, OB>([&](auto bi) {
+    constexpr int RC = z_chunk(OB);
+    auto update = [&](auto bi, float4 ca, float4 cb) {
       constexpr int b = decltype(bi)::value;
       const int n = s + OA * b;
       const float sz = sz_s[n];
-      const float4 ca = lab ? tab_s[la[n]] : (va ? cell_coef(m, rowa + n) : make_float4(0.f, 0.f, 0.f, 0.f));
-      const float4 cb = lab ? tab_s[lb[n]] : (vb ? cell_coef(m, rowb + n) : make_float4(0.f, 0.f, 0.f, 0.f));
       const float poa = pa[b], pob = pbv[b];
       float pna = m.nonlinear ? poa - (ca.y + ca.w * poa) * w[b].x : poa - ca.y * w[b].x;
       float pnb = m.nonlinear ? pob - (cb.y + cb.w * pob) * w[b].y : pob - cb.y * w[b].y;
@@ -1046,7 +1078,28 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
       // rounded here: the transform below takes the stored value, so that the
       // forward-only pass rebuilds the same spectrum from it bit for bit
       w[b] = make_float2(__fmul_rn(pna, spa * sz), vb ? __fmul_rn(pnb, spb * sz) : 0.f);
-    });
+    };
+    if constexpr (lab) {
+      if (s < OA) static_for<0, OB>([&](auto bi) {
+        const int n = s + OA * decltype(bi)::value;
+        update(bi, tab_s[la[n]], tab_s[lb[n]]);
+      });
+    } else if (s < OA) {
+      static_for<0, OB / RC>([&](auto ci) {
+        constexpr int c0 = decltype(ci)::value * RC;
+        float4 ca[RC], cb[RC];
+        static_for<0, RC>([&](auto ji) {
+          constexpr int j = decltype(ji)::value;
+          const int n = s + OA * (c0 + j);
+          ca[j] = va ? z_dense_p(m, rowa + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+          cb[j] = vb ? z_dense_p(m, rowb + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        });
+        static_for<0, RC>([&](auto ji) {
+          constexpr int j = decltype(ji)::value;
+          update(std::integral_constant<int, c0 + j>{}, ca[j], cb[j]);
+        });
+      });
+    }
     // source (engine.py:478-482): entries of rows ya, yb owned by this thread
     if (drive_on && s < OA && va) {
       const int ra = x * d.ny + ya;
@@ -1104,7 +1157,6 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::
         float* __restrict__ pmax = rec.pmax + b_idx * rec.nrec;
         const long long ra = ((long long)(x - rec.lo[0]) * Ry + (ya - rec.lo[1])) * Rz - rec.lo[2];
         const long long rb = ra + Rz;  // row yb = ya + 1
-        constexpr int RC = OB % 4 == 0 ? 4 : (OB % 5 == 0 ? 5 : (OB % 3 == 0 ? 3 : (OB % 2 == 0 ? 2 : 1)));
         static_for<0, OB / RC>([&](auto ci) {
           constexpr int c0 = decltype(ci)::value * RC;
           float sv[2 * RC], cm[2 * RC], pm[2 * RC];
@@ -1182,49 +1234,65 @@ template <int N>
 static long long zp_tiles(const Dims& d, int batch) {
   return (long long)d.nx * ((d.ny + ZPShape<N>::ROWS - 1) / ZPShape<N>::ROWS) * batch;
 }
-template <int N>
-void zp_run_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
-              int batch, cudaStream_t st, const ZTma* ztma) {
+template <int N, bool DENSE>
+void zp_launch_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
+                 int batch, cudaStream_t st, const ZTma* ztma) {
   const long long items = 3 * zp_tiles<N>(d, batch);
+  const dim3 block(ZPShape<N>::THREADS);
   if constexpr (ZPShape<N>::TMA_OK) {
     if (ztma) {
       using L = ZPLayout<N, true, true>;
-      cgf::launch(d.pdl, kfp_zpass_u<N, true>, dim3(zp_grid(items, L::MINB)), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
-                  *ztma);
+      cgf::launch(d.pdl, kfp_zpass_u<N, true, DENSE>, dim3(zp_grid(items, L::MINB)), block, L::smem, st, d, t, m, u, S0, S1,
+                  S2, batch, *ztma);
       return;
     }
   }
   using L = ZPLayout<N, true, false>;
-  cgf::launch(d.pdl, kfp_zpass_u<N>, dim3(zp_grid(items, L::MINB)), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, u, S0, S1, S2, batch,
-              kNoZTma);
+  cgf::launch(d.pdl, kfp_zpass_u<N, false, DENSE>, dim3(zp_grid(items, L::MINB)), block, L::smem, st, d, t, m, u, S0, S1, S2,
+              batch, kNoZTma);
+}
+template <int N>
+void zp_run_u(const Dims& d, const Tables& t, const MediumDev& m, float* u, float2* S0, float2* S1, float2* S2,
+              int batch, cudaStream_t st, const ZTma* ztma) {
+  if (m.labels)
+    zp_launch_u<N, false>(d, t, m, u, S0, S1, S2, batch, st, ztma);
+  else
+    zp_launch_u<N, true>(d, t, m, u, S0, S1, S2, batch, st, ztma);
 }
 
-template <int N>
-void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
-              const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
-              const ZTma* ztma) {
+template <int N, bool REC, bool DENSE>
+void zp_launch_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
+                 const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
+                 const ZTma* ztma) {
   const dim3 block(ZPShape<N>::THREADS);
   if constexpr (ZPShape<N>::TMA_OK) {
     if (ztma) {
       using L = ZPLayout<N, false, true>;
-      const dim3 grid(zp_grid(zp_tiles<N>(d, batch), L::MINB));
-      const size_t sm = L::smem;
-      if (record)
-        cgf::launch(d.pdl, kfp_zpass_p<N, true, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p,
-                    S0, batch, *ztma);
-      else
-        cgf::launch(d.pdl, kfp_zpass_p<N, false, false, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record,
-                    p, S0, batch, *ztma);
+      cgf::launch(d.pdl, kfp_zpass_p<N, REC, false, true, false, DENSE>, dim3(zp_grid(zp_tiles<N>(d, batch), L::MINB)), block,
+                  L::smem, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, *ztma);
       return;
     }
   }
   using L = ZPLayout<N, false, false>;
-  const dim3 grid(zp_grid(zp_tiles<N>(d, batch), L::MINB));
-  const size_t sm = L::smem;
-  if (record)
-    cgf::launch(d.pdl, kfp_zpass_p<N, true>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, kNoZTma);
+  cgf::launch(d.pdl, kfp_zpass_p<N, REC, false, false, false, DENSE>, dim3(zp_grid(zp_tiles<N>(d, batch), L::MINB)), block,
+              L::smem, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, kNoZTma);
+}
+template <int N>
+void zp_run_p(const Dims& d, const Tables& t, const MediumDev& m, const SourceDev& src, const RecordDev& rec,
+              const long long* ctl, int n_local, int record, float* p, float2* S0, int batch, cudaStream_t st,
+              const ZTma* ztma) {
+  auto run = [&](auto rec_, auto dense) {
+    zp_launch_p<N, decltype(rec_)::value, decltype(dense)::value>(d, t, m, src, rec, ctl, n_local, record, p, S0, batch,
+                                                                  st, ztma);
+  };
+  if (m.labels && record)
+    run(std::true_type{}, std::false_type{});
+  else if (m.labels)
+    run(std::false_type{}, std::false_type{});
+  else if (record)
+    run(std::true_type{}, std::true_type{});
   else
-    cgf::launch(d.pdl, kfp_zpass_p<N, false>, grid, block, sm, st, d, t, m, src, rec, ctl, n_local, record, p, S0, batch, kNoZTma);
+    run(std::false_type{}, std::true_type{});
 }
 
 // p -> S0 (forward) or S0 -> p (inverse) alone
@@ -1251,16 +1319,18 @@ static bool zp_allow(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
 
+template <int N, bool TMA, bool DENSE>
+static bool zp_allow_step() {
+  constexpr size_t su = ZPLayout<N, true, TMA>::smem, sp = ZPLayout<N, false, TMA>::smem;
+  return zp_allow(kfp_zpass_u<N, TMA, DENSE>, su) && zp_allow(kfp_zpass_p<N, true, false, TMA, false, DENSE>, sp) &&
+         zp_allow(kfp_zpass_p<N, false, false, TMA, false, DENSE>, sp);
+}
 template <int N>
 int zp_prepare() {
-  constexpr size_t su = ZPLayout<N, true, false>::smem, sp = ZPLayout<N, false, false>::smem;
-  constexpr size_t tu = ZPLayout<N, true, true>::smem, tp = ZPLayout<N, false, true>::smem;
-  bool ok = zp_allow(kfp_zpass_u<N>, su) && zp_allow(kfp_zpass_p<N, false, true>, sp) &&
-            zp_allow(kfp_zpass_p<N, false, false, false, true>, sp) && zp_allow(kfp_zpass_p<N, true>, sp) &&
-            zp_allow(kfp_zpass_p<N, false>, sp);
-  if constexpr (ZPShape<N>::TMA_OK)
-    ok = ok && zp_allow(kfp_zpass_u<N, true>, tu) && zp_allow(kfp_zpass_p<N, true, false, true>, tp) &&
-         zp_allow(kfp_zpass_p<N, false, false, true>, tp);
+  constexpr size_t sp = ZPLayout<N, false, false>::smem;
+  bool ok = zp_allow(kfp_zpass_p<N, false, true>, sp) && zp_allow(kfp_zpass_p<N, false, false, false, true>, sp) &&
+            zp_allow_step<N, false, false>() && zp_allow_step<N, false, true>();
+  if constexpr (ZPShape<N>::TMA_OK) ok = ok && zp_allow_step<N, true, false>() && zp_allow_step<N, true, true>();
   return ok ? 0 : -1;
 }
 
