@@ -197,14 +197,16 @@ struct Dft<2, INV> {
 template <bool INV>
 struct Dft<3, INV> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
-    const float h = 0.86602540378443864676f;
+    // sqrt(3)/2 as a pair of floats: the error of one, 1.6e-8, is the same in
+    // every transform of every step and adds up
+    const float h = 0.86602540378443864676f, hl = (float)(0.86602540378443864676 - (double)h);
     float2 t = c_add(v[1], v[2]);
     float2 d = c_sub(v[1], v[2]);
     float2 m = c_fma(t, -0.5f, v[0]);
-    float2 r = rot<INV>(d);
+    float2 r = rot<INV>(c_fma(d, h, c_scale(d, hl)));
     v[0] = c_add(v[0], t);
-    v[1] = c_fma(r, h, m);
-    v[2] = c_fma(r, -h, m);
+    v[1] = c_add(m, r);
+    v[2] = c_sub(m, r);
   }
 };
 
@@ -227,6 +229,7 @@ struct Dft<5, INV> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
     const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
     const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
+    const float s1l = (float)(0.95105651629515357212 - (double)s1);  // as in the 3-point transform; 2.4e-8
     float2 t1 = c_add(v[1], v[4]);
     float2 t2 = c_add(v[2], v[3]);
     float2 t3 = c_sub(v[1], v[4]);
@@ -234,8 +237,8 @@ struct Dft<5, INV> {
     float2 y0 = c_add(v[0], c_add(t1, t2));
     float2 b1 = c_fma(t2, c2, c_fma(t1, c1, v[0]));
     float2 b2 = c_fma(t2, c1, c_fma(t1, c2, v[0]));
-    float2 e1 = c_fma(t3, s1, c_scale(t4, s2));
-    float2 e2 = c_fma(t3, s2, c_scale(t4, -s1));
+    float2 e1 = c_fma(t3, s1, c_fma(t3, s1l, c_scale(t4, s2)));
+    float2 e2 = c_fma(t4, -s1, c_fma(t4, -s1l, c_scale(t3, s2)));
     float2 r1 = rot<INV>(e1);
     float2 r2 = rot<INV>(e2);
     v[0] = y0;
