@@ -88,9 +88,8 @@ struct XT {
 };
 
 // One instantiation per mode keeps each kernel's code small enough for the
-// instruction cache (the x-pass gradient loops over one copy of its inverse
-// transform; the y-pass modes stay straight-line, where the compiler hoists
-// the next input's loads above the current transform).
+// instruction cache; the modes stay straight-line, where the compiler hoists
+// the next input's loads above the current transform.
 template <int N, int MODE>
 __global__ void __launch_bounds__(YT<N>::THREADS, YT<N>::MINB) kf_ypass(Dims d, Tables t, float2* __restrict__ S0,
                                                                         float2* __restrict__ S1,
