@@ -164,7 +164,9 @@ def _traffic_from_profiles(kernel: str):
 SLOTS = ["k_ypass:fwd", "k_xpass:grad", "k_ypass:inv_grad", "k_zpass_u", "k_ypass:fwd_div", "k_xpass:div",
          "k_ypass:inv", "k_zpass_p"]
 FAST_SIZES = {8, 16, 24, 32, 48, 64, 96, 128, 160, 192, 256}  # every size-specialised kernel family
-FAST_XYZ_SIZES = FAST_SIZES | {320, 400, 512, 640}  # x/y passes and the persistent z-passes only
+# x/y passes and the persistent z-passes only
+FAST_XYZ_SIZES = FAST_SIZES | {2**a * 3**b * 5**c for a in range(8) for b in range(6) for c in range(4)
+                               if 36 <= 2**a * 3**b * 5**c <= 400} | {512, 640}
 
 
 def slot_symbols(padded3, persistent_z: bool = True, tma: bool = False) -> list[str]:

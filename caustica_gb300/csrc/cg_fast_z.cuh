@@ -528,6 +528,23 @@ struct ZPLayout {
   static_assert(smem <= zp_fit(1), "persistent z-pass tile does not fit shared memory");
 };
 
+// The forward-only pass holds no tables, labels or field rows: twiddles and two
+// item buffers, 16 warps an SM. (Three CTAs instead of two of the 20-thread
+// pencils: a 320^3 forward transform 191 -> 175 us, 300^3 165 -> 154. 24 warps of
+// the 16-thread ones: 160x160x192 x 2 59 -> 57, but 100x120x135 x 2 32.5 -> 33.6
+// and 256^3 83 -> 84.)
+template <int N>
+struct ZPFwd {
+  using Z = ZPShape<N>;
+  static constexpr size_t smem = sizeof(float2) * (ZPLayout<N, false, false>::OFF_BUF + 2 * (size_t)Z::BUF);
+  static constexpr int ctas() {
+    int c = 512 / Z::THREADS;
+    while (c > 1 && smem > zp_fit(c)) --c;
+    return c > 1 ? c : 1;
+  }
+  static constexpr int MINB = ctas();
+};
+
 // An item's place: velocity component comp (radix NC: 3 in the u-pass, 1 in
 // the p-pass), member b, y-tile yt of plane x, the first fastest. CTA i takes
 // items i, i + G, i + 2 G, ...: at any time the resident CTAs work on
@@ -902,7 +919,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
 // INV: only the opening inverse transform, its values to the pressure.
 // TMA: the half spectra arrive by tensor-map box copies (as in the u-pass).
 template <int N, bool REC, bool FWD = false, bool TMA = false, bool INV = false, bool DENSE = false>
-__global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, false, TMA>::MINB)
+__global__ void __launch_bounds__(ZPShape<N>::THREADS, FWD ? ZPFwd<N>::MINB : ZPLayout<N, false, TMA>::MINB)
     kfp_zpass_p(Dims d, Tables t, MediumDev m, SourceDev src, RecordDev rec, const long long* ctl, int n_local,
                 int record, float* __restrict__ p_all, float2* __restrict__ S0, int n_members,
                 const __grid_constant__ ZTma ztma) {
@@ -1300,18 +1317,18 @@ template <int N>
 void zp_run_half(bool inverse, const Dims& d, const Tables& t, const MediumDev& m, float* p, float2* S0, int batch,
                  cudaStream_t st) {
   using L = ZPLayout<N, false, false>;
-  const int g = zp_grid(zp_tiles<N>(d, batch), L::MINB);
   SourceDev src;
   memset(&src, 0, sizeof(src));
   RecordDev rec;
   memset(&rec, 0, sizeof(rec));
   rec.spp = 1;
   if (inverse)
-    cgf::launch(d.pdl, kfp_zpass_p<N, false, false, false, true>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m,
-                src, rec, (const long long*)nullptr, 0, 0, p, S0, batch, kNoZTma);
+    cgf::launch(d.pdl, kfp_zpass_p<N, false, false, false, true>, dim3(zp_grid(zp_tiles<N>(d, batch), L::MINB)),
+                dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, src, rec, (const long long*)nullptr, 0, 0, p, S0, batch, kNoZTma);
   else
-    cgf::launch(d.pdl, kfp_zpass_p<N, false, true>, dim3(g), dim3(ZPShape<N>::THREADS), L::smem, st, d, t, m, src, rec,
-                (const long long*)nullptr, 0, 0, p, S0, batch, kNoZTma);
+    cgf::launch(d.pdl, kfp_zpass_p<N, false, true>, dim3(zp_grid(zp_tiles<N>(d, batch), ZPFwd<N>::MINB)),
+                dim3(ZPShape<N>::THREADS), ZPFwd<N>::smem, st, d, t, m, src, rec, (const long long*)nullptr, 0, 0, p, S0, batch,
+                kNoZTma);
 }
 
 template <typename K>
@@ -1328,7 +1345,7 @@ static bool zp_allow_step() {
 template <int N>
 int zp_prepare() {
   constexpr size_t sp = ZPLayout<N, false, false>::smem;
-  bool ok = zp_allow(kfp_zpass_p<N, false, true>, sp) && zp_allow(kfp_zpass_p<N, false, false, false, true>, sp) &&
+  bool ok = zp_allow(kfp_zpass_p<N, false, true>, ZPFwd<N>::smem) && zp_allow(kfp_zpass_p<N, false, false, false, true>, sp) &&
             zp_allow_step<N, false, false>() && zp_allow_step<N, false, true>();
   if constexpr (ZPShape<N>::TMA_OK) ok = ok && zp_allow_step<N, true, false>() && zp_allow_step<N, true, true>();
   return ok ? 0 : -1;
