@@ -629,25 +629,25 @@ __device__ __forceinline__ void zt_issue(char* stg, unsigned long long* bar, con
 
 // The tile's labels (ROWS rows of N bytes, contiguous) into lab_s +
 // label_shift, asynchronously: 16 bytes at a time where every plane of ny N
-// bytes starts on 16 (a tile starts a multiple of 16 N bytes into its plane),
-// else the 4-byte words that hold them; the last word of the volume, if it is
-// not whole, byte by byte.
+// bytes starts on 16 (a tile starts a multiple of 16 N bytes into its plane, a
+// slab on a plane), else the aligned 4-byte words that hold them; the last word
+// of the volume, if it is not whole, byte by byte. The words before a tile's
+// first byte are the volume's own: it starts on a multiple of 256.
 template <int N>
-__device__ __forceinline__ int label_shift(const Dims& d, int x) {
-  return (int)(((unsigned)x * (unsigned)(d.ny * N)) & 3u);
+__device__ __forceinline__ int label_shift(const MediumDev& m, const Dims& d, int x) {
+  return (int)(((unsigned)(uintptr_t)m.labels + (unsigned)x * (unsigned)(d.ny * N)) & 3u);
 }
 template <int N>
-__device__ __forceinline__ void z_prefetch_labels(uint8_t* lab_s, const uint8_t* __restrict__ labels, const Dims& d,
-                                                  int x, int y0) {
+__device__ __forceinline__ void z_prefetch_labels(uint8_t* lab_s, const MediumDev& m, const Dims& d, int x, int y0) {
   using Z = ZPShape<N>;
-  const long long first = ((long long)x * d.ny + y0) * N;
+  const uint8_t* first = m.labels + ((long long)x * d.ny + y0) * N;
   const int nb = min(Z::ROWS, d.ny - y0) * N;
   if ((d.ny * N) % 16 == 0) {
-    for (int i = 16 * threadIdx.x; i < nb; i += 16 * Z::THREADS) cgf::cp_async16(lab_s + i, labels + first + i);
+    for (int i = 16 * threadIdx.x; i < nb; i += 16 * Z::THREADS) cgf::cp_async16(lab_s + i, first + i);
   } else {
-    const int mis = label_shift<N>(d, x);
-    const uint8_t* src = labels + first - mis;  // the volume starts on a multiple of 256
-    const long long avail = d.ncell - (first - mis);
+    const int mis = label_shift<N>(m, d, x);
+    const uint8_t* src = first - mis;
+    const long long avail = m.labels_end - src;
     for (int i = 4 * threadIdx.x; i < nb + mis; i += 4 * Z::THREADS) {
       if (i + 4 <= avail)
         cgf::cp_async4(lab_s + i, src + i);
@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     } else {
       z_prefetch<N>(stg, spec(c.comp, c.b), d, c.x, y0);
     }
-    if constexpr (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
+    if constexpr (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m, d, c.x, y0);
     cgf::cp_async_commit();
   };
   ZCursor<3> cur(n_members, ytiles);
@@ -802,7 +802,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     const int comp = cur.comp;
     const long long b_idx = cur.b;
     const int x = cur.x, y0 = cur.yt * Z::ROWS;
-    const uint8_t* la = lab0 + j * (Z::ROWS * N + 16) + label_shift<N>(d, x) + (2 * p) * N;
+    const uint8_t* la = lab0 + j * (Z::ROWS * N + 16) + label_shift<N>(m, d, x) + (2 * p) * N;
     const uint8_t* lb = la + N;
     const int ya = y0 + 2 * p, yb = ya + 1;
     const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist
@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, FWD ? ZPFwd<N>::MINB : ZP
     } else {
       z_prefetch<N>(stg, S0 + c.b * d.nspec, d, c.x, y0);
     }
-    if constexpr (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m.labels, d, c.x, y0);
+    if constexpr (lab) z_prefetch_labels<N>(lab0 + j * (Z::ROWS * N + 16), m, d, c.x, y0);
     cgf::cp_async_commit();
   };
   ZCursor<1> cur(n_members, ytiles);
@@ -1016,7 +1016,7 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, FWD ? ZPFwd<N>::MINB : ZP
   for (; cur.x < d.nx; j ^= 1) {
     const long long b_idx = cur.b;
     const int x = cur.x, y0 = cur.yt * Z::ROWS;
-    const uint8_t* la = lab0 + j * (Z::ROWS * N + 16) + label_shift<N>(d, x) + (2 * p) * N;
+    const uint8_t* la = lab0 + j * (Z::ROWS * N + 16) + label_shift<N>(m, d, x) + (2 * p) * N;
     const uint8_t* lb = la + N;
     const int ya = y0 + 2 * p, yb = ya + 1;
     const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist

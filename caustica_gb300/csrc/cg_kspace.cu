@@ -700,6 +700,7 @@ static Tables make_tables(const cg_solver* s) {
 static MediumDev make_medium(const cg_solver* s) {
   MediumDev m;
   m.labels = s->labels;
+  m.labels_end = s->labels ? s->labels + s->d.ncell : nullptr;
   m.ltab = s->ltab;
   m.dtr = s->dtr; m.rc2 = s->rc2; m.ab = s->ab; m.b2 = s->b2;
   m.nonlinear = s->nonlinear;

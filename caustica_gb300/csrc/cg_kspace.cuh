@@ -40,6 +40,7 @@ struct Tables {
 
 struct MediumDev {
   const uint8_t* labels;  // null when dense
+  const uint8_t* labels_end;  // behind the whole grid's labels, in a slab too
   const float4* ltab;     // per label (dt/rho, rho c^2 dt, absorb, 2 beta dt)
   const float* dtr;
   const float* rc2;
