@@ -31,6 +31,7 @@
 #include <string.h>
 
 #include "cg_common.cuh"
+#include "cg_fast.cuh"
 #include "cg_fft.cuh"
 
 using cgfft::tile_fft;
@@ -521,15 +522,20 @@ __global__ void __launch_bounds__(CG_THREADS) k_zpass_p(int mode, Dims d, AxisPl
 // spp factors are formed in FP64 once per block, in shared memory; every bin is
 // read once and feeds all harmonics, each summed over m in increasing order.
 //
-// Bound: HBM, 8 spp bytes read and 8 nh written per voxel. FP64 arithmetic is
-// slow on GB300 and took 4.9 ms for three harmonics of 192x192x256 (13 bins,
-// 1.2 GB of traffic) where the traffic takes 0.2 ms, so the products and sums run on unevaluated
-// pairs of floats (Dekker's two-sum and the fused two-product: relative error
-// below 2^-44 of the largest term, far inside the final rounding to float32).
-// That needs the error terms to be representable: a voxel whose bins are not
-// all zero and not all within [2^-60, 2^120] takes the FP64 sum. u carries the factor 2/K
+// Bound: HBM, 8 spp bytes read and 8 nh written per voxel, and the arithmetic of
+// the sums. FP64 units are slow on GB300 (4.8 ms for three harmonics of
+// 192x192x256, 13 bins, whose 1.2 GB take 0.2 ms), so the sums run on floats, and
+// on three of them each: bins are exact pairs, factors hold 72 bits, products
+// and sums keep the rounding errors of their first two levels exactly (Dekker's
+// two-sum and the fused two-product) and add the third level's plainly. The
+// error, 2^-70 a term, is less than that of an FP64 sum (2^-53 a term), which
+// shows where a sum cancels: a weak harmonic beside a strong one. (Three
+// harmonics of 192x192x256, 12 bins: pairs alone, 2^-44, 0.47 ms, triples 1.16.)
+//
+// The error terms have to be representable: a voxel whose bins are not all zero
+// and not all within [2^-60, 2^120] takes the FP64 sum. u carries the factor 2/K
 // from the start, so no partial sum exceeds twice the largest pressure.
-constexpr float kPairLo = 8.6736174e-19f, kPairHi = 1.3292280e36f;  // 2^-60, 2^120
+constexpr float kSumLo = 8.6736174e-19f, kSumHi = 1.3292280e36f;  // 2^-60, 2^120
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   s = __fadd_rn(a, b);
@@ -537,17 +543,59 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
 }
 
+// x = hi + mid + lo to 72 bits, given its FP64 rounding and the rest
+struct Float3 {
+  float hi, mid, lo;
+};
+__device__ __forceinline__ Float3 float3_of(double x, double rest) {
+  Float3 r;
+  r.hi = (float)x;
+  const double d = x - (double)r.hi;
+  r.mid = (float)d;
+  r.lo = (float)((d - (double)r.mid) + rest);
+  return r;
+}
+
+// s += (v + w) u
+__device__ __forceinline__ void add_product(Float3& s, float v, float w, Float3 u) {
+  const float p0 = __fmul_rn(v, u.hi), e0 = __fmaf_rn(v, u.hi, -p0);
+  float p1 = __fmul_rn(v, u.mid);
+  const float e1 = __fmaf_rn(v, u.mid, -p1);
+  const float p2 = __fmul_rn(w, u.hi), e2 = __fmaf_rn(w, u.hi, -p2);
+  float lo = __fadd_rn(__fmaf_rn(v, u.lo, __fmul_rn(w, u.mid)), __fadd_rn(e1, e2));
+  float t, e;
+  two_sum(s.hi, p0, s.hi, t);
+  two_sum(t, e0, t, e);
+  lo = __fadd_rn(lo, e);
+  two_sum(p1, p2, p1, e);
+  lo = __fadd_rn(lo, e);
+  two_sum(t, p1, t, e);
+  lo = __fadd_rn(lo, e);
+  two_sum(s.mid, t, s.mid, e);
+  s.lo = __fadd_rn(s.lo, __fadd_rn(lo, e));
+}
+
+__device__ __forceinline__ float rounded(Float3 s) {
+  float a, b, c, d;
+  two_sum(s.mid, s.lo, a, b);
+  two_sum(s.hi, a, c, d);
+  return __fadd_rn(c, __fadd_rn(d, b));
+}
+
 template <int NH>
 __global__ void __launch_bounds__(256) k_finalize(RecordDev rec, int B, const int* harm, int K, float2* out) {
-  extern __shared__ float4 upf[];  // [NH][spp] float pairs (re hi, re lo, im hi, im lo)
+  extern __shared__ float2 ufac[];  // [NH][spp] x (re hi, im hi), (re mid, im mid), (re lo, im lo)
+  const int nf = NH * rec.spp;
   const double sc = 2.0 / K;
-  for (int i = threadIdx.x; i < NH * rec.spp; i += blockDim.x) {
+  for (int i = threadIdx.x; i < nf; i += blockDim.x) {
     const int h = i / rec.spp, mm = i - h * rec.spp;
     double sn, cs;
     sincospi(2.0 * (double)((harm[h] * (long long)mm) % rec.spp) / rec.spp, &sn, &cs);
     const double re = cs * sc, im = sn * sc;
-    const float rh = (float)re, ih = (float)im;
-    upf[i] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
+    const Float3 r = float3_of(re, fma(cs, sc, -re)), q = float3_of(im, fma(sn, sc, -im));
+    ufac[i] = make_float2(r.hi, q.hi);
+    ufac[nf + i] = make_float2(r.mid, q.mid);
+    ufac[2 * nf + i] = make_float2(r.lo, q.lo);
   }
   __syncthreads();
   const long long total = (long long)B * rec.nrec;
@@ -557,9 +605,9 @@ __global__ void __launch_bounds__(256) k_finalize(RecordDev rec, int B, const in
     const long long r = i - b * rec.nrec;
     const float* bins = rec.bins + b * rec.spp * rec.nrec + r;
     const float* comp = rec.comp + b * rec.spp * rec.nrec + r;
-    float re[NH], ree[NH], im[NH], ime[NH];  // sums and their error terms
+    Float3 re[NH], im[NH];
 #pragma unroll
-    for (int h = 0; h < NH; ++h) re[h] = ree[h] = im[h] = ime[h] = 0.f;
+    for (int h = 0; h < NH; ++h) re[h] = im[h] = {0.f, 0.f, 0.f};
     bool exact = true;
     constexpr int U = 4;  // bins loaded ahead of their use
     for (int m0 = 0; m0 < rec.spp; m0 += U) {
@@ -576,34 +624,30 @@ __global__ void __launch_bounds__(256) k_finalize(RecordDev rec, int B, const in
         float v, w;  // s - c as an exact pair
         two_sum(sv[j], -cv[j], v, w);
         const float av = fabsf(v);
-        exact = exact && (av == 0.f || (av >= kPairLo && av <= kPairHi));
+        exact = exact && (av == 0.f || (av >= kSumLo && av <= kSumHi));
 #pragma unroll
         for (int h = 0; h < NH; ++h) {
-          const float4 u = upf[h * rec.spp + m0 + j];
-          float p = __fmul_rn(v, u.x), e;
-          float t = __fmaf_rn(w, u.x, __fmaf_rn(v, u.y, __fmaf_rn(v, u.x, -p)));
-          two_sum(re[h], p, re[h], e);
-          ree[h] = __fadd_rn(ree[h], __fadd_rn(e, t));
-          p = __fmul_rn(v, u.z);
-          t = __fmaf_rn(w, u.z, __fmaf_rn(v, u.w, __fmaf_rn(v, u.z, -p)));
-          two_sum(im[h], p, im[h], e);
-          ime[h] = __fadd_rn(ime[h], __fadd_rn(e, t));
+          const int k = h * rec.spp + m0 + j;
+          const float2 u0 = ufac[k], u1 = ufac[nf + k], u2 = ufac[2 * nf + k];
+          add_product(re[h], v, w, {u0.x, u1.x, u2.x});
+          add_product(im[h], v, w, {u0.y, u1.y, u2.y});
         }
       }
     }
     if (exact) {
 #pragma unroll
       for (int h = 0; h < NH; ++h)
-        out[(b * NH + h) * rec.nrec + r] = make_float2(__fadd_rn(re[h], ree[h]), __fadd_rn(im[h], ime[h]));
+        out[(b * NH + h) * rec.nrec + r] = make_float2(rounded(re[h]), rounded(im[h]));
     } else {
 #pragma unroll 1
       for (int h = 0; h < NH; ++h) {
         double dr = 0.0, di = 0.0;
         for (int mm = 0; mm < rec.spp; ++mm) {
           const double v = (double)bins[mm * rec.nrec] - (double)comp[mm * rec.nrec];
-          const float4 u = upf[h * rec.spp + mm];
-          dr += v * ((double)u.x + (double)u.y);
-          di += v * ((double)u.z + (double)u.w);
+          const int k = h * rec.spp + mm;
+          const float2 u0 = ufac[k], u1 = ufac[nf + k], u2 = ufac[2 * nf + k];
+          dr += v * ((double)u0.x + ((double)u1.x + (double)u2.x));
+          di += v * ((double)u0.y + ((double)u1.y + (double)u2.y));
         }
         out[(b * NH + h) * rec.nrec + r] = make_float2((float)dr, (float)di);
       }
@@ -611,7 +655,7 @@ __global__ void __launch_bounds__(256) k_finalize(RecordDev rec, int B, const in
   }
 }
 
-static size_t smem_finalize(int nh, int spp) { return sizeof(float4) * (size_t)nh * spp; }
+static size_t smem_finalize(int nh, int spp) { return 3 * sizeof(float2) * (size_t)nh * spp; }
 
 static const void* finalize_kernel(int nh) {
   static const void* const k[CG_MAX_H] = {(const void*)k_finalize<1>, (const void*)k_finalize<2>,
@@ -1423,7 +1467,7 @@ extern "C" int cg_solver_finalize(cg_solver* s, int n_record_steps, float* phaso
   }
   RecordDev rec = make_record(s);
   void* args[] = {&rec, &s->B, &s->harm_dev, &n_record_steps, &s->ph};
-  const long long blocks = ((long long)s->B * s->nrec + 255) / 256, most = 152LL * 8 * 4;  // four waves
+  const long long blocks = ((long long)s->B * s->nrec + 255) / 256, most = 8LL * 4 * cgf::sm_count();  // four waves
   cudaError_t e = cudaLaunchKernel(finalize_kernel(s->nh), dim3((unsigned)(blocks < most ? blocks : most)), dim3(256),
                                    args, smem_finalize(s->nh, s->spp), s->stream);
   if (e == cudaSuccess && phasors)

@@ -94,8 +94,8 @@ int cg_solver_begin_record(cg_solver* s);
 /* Per-period max |p| over the convergence box (engine.py:490-495) for
  * periods [first, first+count), as float [batch][count]. Synchronises. */
 int cg_solver_read_peaks(cg_solver* s, int first, int count, float* out);
-/* Phasors of every harmonic, FP64-normalised by 2/n_record_steps
- * (engine.py:551-552), as complex64 [batch][n_harmonics][record box], and
+/* Phasors of every harmonic, summed and normalised by 2/n_record_steps
+ * (engine.py:551-552) to FP64 accuracy or better, as complex64 [batch][n_harmonics][record box], and
  * p_max [batch][record box]; either may be NULL. Host or device. */
 int cg_solver_finalize(cg_solver* s, int n_record_steps, float* phasors, float* pmax);
 /* Checkpoint state (engine.py:359-371): p [batch][cells], u [3][batch][cells]. */
