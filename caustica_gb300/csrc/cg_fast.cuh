@@ -126,7 +126,10 @@ constexpr int ct_crt(int k1, int k2, int A, int B) {
 // everywhere -> as it is: 192x192x256 275.7 -> 274.6 us, 320^3 1182 -> 1165,
 // 384^3 1946 -> 1895, 400^3 2173 -> 2111; the error of a round trip against 64
 // bits 1.86e-7 -> 1.79e-7 at 180 points, 2.05e-7 -> 1.89e-7 at 400.
-template <int R, bool INV>
+// FINE: the factors of 3 multiply by sqrt(3)/2 as a pair of floats. So in the
+// powers of 3, whose twiddles between the factors add errors of their own (a
+// transform of 81, 162, 243 or 324 points 5 % further off 64 bits without).
+template <int R, bool INV, bool FINE = (R % 9 == 0)>
 struct Dft {
   static constexpr int A = ct_first_factor(R), B = R / A;
   static constexpr bool COPRIME = ct_gcd(A, B) == 1;
@@ -145,10 +148,10 @@ struct Dft {
         constexpr int n1 = decltype(mi)::value;
         t[n1] = v[(B * n1 + A * n2) % R];
       });
-      Dft<A, INV>::run(t);
+      Dft<A, INV, FINE>::run(t);
       static_for<0, A>([&](auto ki) { o[B * decltype(ki)::value + n2] = t[decltype(ki)::value]; });
     });
-    static_for<0, A>([&](auto ki) { Dft<B, INV>::run(o + B * decltype(ki)::value); });
+    static_for<0, A>([&](auto ki) { Dft<B, INV, FINE>::run(o + B * decltype(ki)::value); });
     static_for<0, A>([&](auto k1i) {
       static_for<0, B>([&](auto k2i) {
         constexpr int k1 = decltype(k1i)::value, k2 = decltype(k2i)::value;
@@ -162,13 +165,13 @@ struct Dft {
       constexpr int b = decltype(bi)::value;
       float2 t[A];
       static_for<0, A>([&](auto ai) { t[decltype(ai)::value] = v[B * decltype(ai)::value + b]; });
-      Dft<A, INV>::run(t);
+      Dft<A, INV, FINE>::run(t);
       static_for<0, A>([&](auto ai) {
         constexpr int a = decltype(ai)::value;
         v[B * a + b] = twiddle_ct<R, a * b, INV>(t[a]);
       });
     });
-    static_for<0, A>([&](auto ki) { Dft<B, INV>::run(v + B * decltype(ki)::value); });
+    static_for<0, A>([&](auto ki) { Dft<B, INV, FINE>::run(v + B * decltype(ki)::value); });
     float2 o[R];
     static_for<0, A>([&](auto k1i) {
       static_for<0, B>([&](auto k2i) {
@@ -180,13 +183,13 @@ struct Dft {
   }
 };
 
-template <bool INV>
-struct Dft<1, INV> {
+template <bool INV, bool FINE>
+struct Dft<1, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2*) {}
 };
 
-template <bool INV>
-struct Dft<2, INV> {
+template <bool INV, bool FINE>
+struct Dft<2, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
     float2 a = v[0], b = v[1];
     v[0] = c_add(a, b);
@@ -194,24 +197,22 @@ struct Dft<2, INV> {
   }
 };
 
-template <bool INV>
-struct Dft<3, INV> {
+template <bool INV, bool FINE>
+struct Dft<3, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
-    // sqrt(3)/2 as a pair of floats: the error of one, 1.6e-8, is the same in
-    // every transform of every step and adds up
     const float h = 0.86602540378443864676f, hl = (float)(0.86602540378443864676 - (double)h);
     float2 t = c_add(v[1], v[2]);
     float2 d = c_sub(v[1], v[2]);
     float2 m = c_fma(t, -0.5f, v[0]);
-    float2 r = rot<INV>(c_fma(d, h, c_scale(d, hl)));
+    float2 r = rot<INV>(FINE ? c_fma(d, h, c_scale(d, hl)) : c_scale(d, h));
     v[0] = c_add(v[0], t);
     v[1] = c_add(m, r);
     v[2] = c_sub(m, r);
   }
 };
 
-template <bool INV>
-struct Dft<4, INV> {
+template <bool INV, bool FINE>
+struct Dft<4, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
     float2 t0 = c_add(v[0], v[2]);
     float2 t1 = c_sub(v[0], v[2]);
@@ -224,12 +225,11 @@ struct Dft<4, INV> {
   }
 };
 
-template <bool INV>
-struct Dft<5, INV> {
+template <bool INV, bool FINE>
+struct Dft<5, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
     const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
     const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
-    const float s1l = (float)(0.95105651629515357212 - (double)s1);  // as in the 3-point transform; 2.4e-8
     float2 t1 = c_add(v[1], v[4]);
     float2 t2 = c_add(v[2], v[3]);
     float2 t3 = c_sub(v[1], v[4]);
@@ -237,8 +237,8 @@ struct Dft<5, INV> {
     float2 y0 = c_add(v[0], c_add(t1, t2));
     float2 b1 = c_fma(t2, c2, c_fma(t1, c1, v[0]));
     float2 b2 = c_fma(t2, c1, c_fma(t1, c2, v[0]));
-    float2 e1 = c_fma(t3, s1, c_fma(t3, s1l, c_scale(t4, s2)));
-    float2 e2 = c_fma(t4, -s1, c_fma(t4, -s1l, c_scale(t3, s2)));
+    float2 e1 = c_fma(t3, s1, c_scale(t4, s2));
+    float2 e2 = c_fma(t4, -s1, c_scale(t3, s2));
     float2 r1 = rot<INV>(e1);
     float2 r2 = rot<INV>(e2);
     v[0] = y0;
@@ -249,8 +249,8 @@ struct Dft<5, INV> {
   }
 };
 
-template <bool INV>
-struct Dft<8, INV> {
+template <bool INV, bool FINE>
+struct Dft<8, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
     const float r2 = 0.70710678118654752440f;
     float2 e[4] = {v[0], v[2], v[4], v[6]};
