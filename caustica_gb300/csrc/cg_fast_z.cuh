@@ -33,10 +33,18 @@ using cgf::static_for;
 // The pencil split with the larger factor first: after the inverse (A, B)
 // transform A threads hold B cells each at n = s + A b, so the pointwise
 // update runs on more lanes and every row access is a run of A floats.
+// Smaller factor first on 192, 240 and 320 points, for accuracy: which codelet
+// is next to the field decides how the rounding of the loud part of a field
+// spreads to the quiet part. Error of phasors in a quiet middle of 96x96xN (1e-6
+// of their norm, mean of two fields), larger first / smaller first: 192 18.7 /
+// 12.5, 240 18.7 / 16.1, 320 24.2 / 19.5; but 160 11.7 / 12.5, 180 17.2 / 19.2,
+// 216 11.6 / 15.0, 288 18.0 / 19.2, 384 20.3 / 21.8, 300 14.3 / 13.8. It costs
+// 160x160x192 x 8 1135 -> 1159 us a step, 192x192x320 369 -> 382 (128x128x240 137
+// -> 135).
 template <int N>
 struct ZSplit {
   using P = cgf::PSplit<N>;
-  static constexpr bool SWAP = !P::THREE && P::A < P::B;
+  static constexpr bool SWAP = !P::THREE && P::A < P::B && N != 192 && N != 240 && N != 320;
   static constexpr int A = SWAP ? P::B : P::A, B = SWAP ? P::A : P::B;
   static constexpr int OA = SWAP ? P::OB : P::OA, OB = SWAP ? P::OA : P::OB, TW = P::TW;
   // three-level pencils fill a warp each, so that their three exchanges wait for
