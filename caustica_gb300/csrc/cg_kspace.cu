@@ -1267,9 +1267,9 @@ static int launch_step_slabs(cg_solver* s, int n_local, int record, EvLog* log) 
   return CG_OK;
 }
 
-// One step = 8 launches (or 2 + 6 per slab in slab mode). With `log` an
-// event is recorded before each launch and after the last, for per-kernel
-// timing.
+// One step = 8 launches (4 where one launch runs a transverse chain, 2 + 6 per
+// slab in slab mode: launches_per_step). With `log` an event is recorded
+// before each launch and after the last, for per-kernel timing.
 static int launch_step(cg_solver* s, int n_local, int record, EvLog* log = nullptr) {
   if (s->slabs > 1) return launch_step_slabs(s, n_local, record, log);
   const Dims d = s->d;
@@ -1513,6 +1513,12 @@ extern "C" int cg_solver_query(cg_solver* s, int* idle) {
   return CG_OK;
 }
 
+// Kernels that launch_step launches.
+static int launches_per_step(const cg_solver* s) {
+  if (s->slabs > 1) return 2 + 6 * s->slabs;
+  return (s->d.nx == 1 && fast_xy_has(s->d.ny)) || s->fused_xy ? 4 : 8;
+}
+
 extern "C" int cg_solver_info(const cg_solver* s, long long* out /* 8 */) {
   CG_REQUIRE(s && out, "null argument");
   out[0] = s->d.ncell;
@@ -1522,7 +1528,7 @@ extern "C" int cg_solver_info(const cg_solver* s, long long* out /* 8 */) {
   out[4] = (long long)s->smem_x;
   out[5] = (long long)s->smem_z;
   out[6] = s->B;
-  out[7] = s->slabs > 1 ? 2 + 6 * s->slabs : (s->fused_xy ? 4 : 8);  // passes per step
+  out[7] = launches_per_step(s);
   return CG_OK;
 }
 
@@ -1749,7 +1755,7 @@ extern "C" int cg_solver_get_config(const cg_solver* s, int* out4) {
   out4[0] = s->fused_xy;
   out4[1] = s->zpers;
   out4[2] = s->slabs;
-  out4[3] = s->slabs > 1 ? 2 + 6 * s->slabs : (s->fused_xy ? 4 : 8);
+  out4[3] = launches_per_step(s);
   return CG_OK;
 }
 

@@ -111,9 +111,9 @@ int cg_solver_timed_run(cg_solver* s, int n_steps, int record, int graph, float*
 /* Per-launch device time [ms] summed over n_steps steps, 8 entries in step
  * order (y fwd, x grad, y inv grad, z u, y fwd div, x div, y inv, z p). */
 int cg_solver_profile(cg_solver* s, int n_steps, int record, float* ms8);
-/* ncell, nspec, nrec, smem y/x/z, batch, passes per step: 8 (one kernel launch
- * each; a grid of one x plane runs three of them in one launch), 4 with the
- * cluster-fused chain, 2 + 6 k with k slabs. */
+/* ncell, nspec, nrec, smem y/x/z, batch, kernel launches per step: 8, 4 with the
+ * cluster-fused chain and on grids of one x plane (whose row length has
+ * size-specialised kernels), 2 + 6 k with k slabs. */
 int cg_solver_info(const cg_solver* s, long long* out8);
 /* Autotuner: on a fresh handle (medium, source and drive set) time each
  * launch configuration the grid admits -- cluster-fused or three-pass
@@ -149,7 +149,7 @@ int cg_solver_set_slabs(cg_solver* s, int slabs);
 int cg_solver_set_zstaging(cg_solver* s, int tma);
 int cg_solver_get_zstaging(const cg_solver* s, int* tma);
 /* out4 = {cluster-fused transverse chain, persistent z-passes, slabs,
- * passes per step, as cg_solver_info} of the handle's current launch configuration. */
+ * kernel launches per step} of the handle's current launch configuration. */
 int cg_solver_get_config(const cg_solver* s, int* out4);
 
 /* ------------------------------------------------- batched 3-D R2C/C2R */
