@@ -1361,10 +1361,39 @@ extern "C" int cg_solver_run(cg_solver* s, int n_steps, int record) {
   return CG_OK;
 }
 
-extern "C" int cg_solver_run_periods(cg_solver* s, int n_periods, int record) {
+static int check_run(const cg_solver* s, int record) {
   CG_REQUIRE(s, "null solver");
   CG_REQUIRE(!record || s->bins, "recording needs cg_solver_begin_record first");
   CG_REQUIRE(s->has_medium, "set a medium before running");
+  return CG_OK;
+}
+
+// The graph of one period, built on first use.
+static int period_graph(cg_solver* s, int record) {
+  const int gi = record ? 1 : 0;
+  if (s->graph[gi]) return CG_OK;
+  cudaGraph_t g;
+  CG_CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+  for (int i = 0; i < s->spp; ++i) launch_step(s, i, record);
+  k_advance<<<1, 1, 0, s->stream>>>(s->ctl, s->spp);
+  cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+  if (e != cudaSuccess) {
+    cg_set_error("graph capture: %s", cudaGetErrorString(e));
+    return CG_ERR_CUDA;
+  }
+  e = cudaGraphInstantiate(&s->graph[gi], g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) {
+    cg_set_error("graph instantiate: %s", cudaGetErrorString(e));
+    s->graph[gi] = nullptr;
+    return CG_ERR_CUDA;
+  }
+  return CG_OK;
+}
+
+extern "C" int cg_solver_run_periods(cg_solver* s, int n_periods, int record) {
+  int rc = check_run(s, record);
+  if (rc != CG_OK) return rc;
   CG_REQUIRE(n_periods >= 0, "n_periods must be >= 0");
   const int gi = record ? 1 : 0;
   // Building a period's graph (some hundred nodes) takes about 0.4 ms of host
@@ -1376,30 +1405,13 @@ extern "C" int cg_solver_run_periods(cg_solver* s, int n_periods, int record) {
     const int n = n_periods <= 2 && !s->plain[gi] ? n_periods : 1;
     s->plain[gi] = 1;
     for (int k = 0; k < n; ++k) {
-      const int rc = cg_solver_run(s, s->spp, record);
+      rc = cg_solver_run(s, s->spp, record);
       if (rc != CG_OK) return rc;
     }
     n_periods -= n;
   }
   if (n_periods == 0) return CG_OK;
-  if (!s->graph[gi]) {
-    cudaGraph_t g;
-    CG_CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    for (int i = 0; i < s->spp; ++i) launch_step(s, i, record);
-    k_advance<<<1, 1, 0, s->stream>>>(s->ctl, s->spp);
-    cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-    if (e != cudaSuccess) {
-      cg_set_error("graph capture: %s", cudaGetErrorString(e));
-      return CG_ERR_CUDA;
-    }
-    e = cudaGraphInstantiate(&s->graph[gi], g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) {
-      cg_set_error("graph instantiate: %s", cudaGetErrorString(e));
-      s->graph[gi] = nullptr;
-      return CG_ERR_CUDA;
-    }
-  }
+  if ((rc = period_graph(s, record)) != CG_OK) return rc;
   for (int i = 0; i < n_periods; ++i) CG_CUDA_TRY(cudaGraphLaunch(s->graph[gi], s->stream));
   return CG_OK;
 }
@@ -1539,11 +1551,15 @@ extern "C" int cg_solver_info(const cg_solver* s, long long* out /* 8 */) {
 extern "C" int cg_solver_timed_run(cg_solver* s, int n_steps, int record, int graph, float* ms) {
   CG_REQUIRE(s && ms, "null argument");
   CG_REQUIRE(!graph || n_steps % s->spp == 0, "graph timing needs whole periods (n_steps %% spp == 0)");
+  int rc = CG_OK;
+  if (graph && n_steps > 0) {  // built here, so that every timed period is a replay
+    if ((rc = check_run(s, record)) != CG_OK || (rc = period_graph(s, record)) != CG_OK) return rc;
+  }
   cudaEvent_t a, b;
   CG_CUDA_TRY(cudaEventCreate(&a));
   CG_CUDA_TRY(cudaEventCreate(&b));
   CG_CUDA_TRY(cudaEventRecord(a, s->stream));
-  int rc = graph ? cg_solver_run_periods(s, n_steps / s->spp, record) : cg_solver_run(s, n_steps, record);
+  rc = graph ? cg_solver_run_periods(s, n_steps / s->spp, record) : cg_solver_run(s, n_steps, record);
   CG_CUDA_TRY(cudaEventRecord(b, s->stream));
   CG_CUDA_TRY(cudaEventSynchronize(b));
   CG_CUDA_TRY(cudaEventElapsedTime(ms, a, b));

@@ -2,10 +2,13 @@
 
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import caustica_gb300 as cg
+from caustica_gb300 import _lib
 from caustica_gb300 import engine as eng
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +62,18 @@ def test_a_step_makes_the_launches_that_the_handle_reports(torch, shape, slabs, 
 
         kernels = [k for k in _profiled(torch, steps)[0] if "pass" in k or "plane" in k]
         assert len(kernels) == 5 * launches
+
+
+@pytest.mark.parametrize("warmup", [0, 1])
+def test_a_run_timed_by_graph_times_graph_launches_only(torch, warmup):
+    with _solver((64, 96)) as dev:
+        dev.run_periods(warmup)  # one period: plain launches, no graph yet
+        ms = C.c_float()
+
+        def timed():
+            _lib.call("cg_solver_timed_run", dev.h, 2 * dev.plan.spp, 0, 1, C.byref(ms))
+
+        calls = _profiled(torch, timed)[1]
+        first = calls.index("cudaEventRecord")
+        last = len(calls) - 1 - calls[::-1].index("cudaEventRecord")
+        assert calls[first + 1:last] == ["cudaGraphLaunch"] * 2
