@@ -790,18 +790,17 @@ extern "C" int cg_pennes_run(cg_pennes* h, int n_sub) {
   const int tzc = pair ? 2 * PP_Z : (P.labels ? PS_Z : 32), tyc = pair ? PP_Y : (P.labels ? PS_Y : PD_Y);
   const dim3 sblock(pair ? PP_Z : tzc, tyc);
   const long long tiles_zy = (long long)((h->cfg.nz + tzc - 1) / tzc) * ((h->cfg.ny + tyc - 1) / tyc);
-  const int xs = xs_pin > 0 ? xs_pin : pennes_planes(tiles_zy, h->cfg.nx);
+  // at least as many as keep the blocks along x within a grid dimension
+  const int x_min = (h->cfg.nx + 65534) / 65535, x_want = xs_pin > 0 ? xs_pin : pennes_planes(tiles_zy, h->cfg.nx);
+  const int xs = x_want > x_min ? x_want : x_min;
   const dim3 sgrid((unsigned)((h->cfg.nz + tzc - 1) / tzc), (unsigned)((h->cfg.ny + tyc - 1) / tyc),
                    (unsigned)((h->cfg.nx + xs - 1) / xs));
-  // dense maps: z-y tiles along one grid dimension (any ny), as many x planes
-  // a block as keep the other within its limit
-  const int xd = xs > (h->cfg.nx + 65534) / 65535 ? xs : (h->cfg.nx + 65534) / 65535;
-  const dim3 dgrid((unsigned)tiles_zy, (unsigned)((h->cfg.nx + xd - 1) / xd));
+  const dim3 dgrid((unsigned)tiles_zy, sgrid.z);  // dense maps: z-y tiles along one grid dimension (any ny)
   for (int i = 0; i < n_sub; ++i) {
     if (P.labels)
       launch_stream(pair, P, sgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
     else
-      launch_dense(P, dgrid, sblock, h->stream, xd, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
+      launch_dense(P, dgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
     h->cur = 1 - h->cur;
   }
   CG_CUDA_TRY(cudaGetLastError());
