@@ -44,3 +44,16 @@ def _check(shape, mode, boundary, n_steps, dose):
 @pytest.mark.parametrize("mode", ["labels", "dense"])
 def test_grids_longer_than_one_block_dimension(shape, mode):
     _check(shape, mode, "insulated", 2, False)
+
+
+@pytest.mark.parametrize("boundary,dose", [("insulated", True), ("dirichlet", False)])
+@pytest.mark.parametrize("shape,mode", [
+    ((37, 130, 131), "dense"),   # 85 tiles: four planes
+    ((37, 180, 190), "dense"),   # 138 tiles: eight planes
+    ((37, 130, 131), "labels"),  # single cells
+    ((37, 180, 191), "labels"),
+    ((37, 180, 190), "labels"),  # z-pairs, 72 tiles: four planes
+    ((37, 290, 190), "labels"),  # 114 tiles: eight planes
+])
+def test_blocks_that_walk_four_and_eight_planes(shape, mode, boundary, dose):
+    _check(shape, mode, boundary, 7, dose)
