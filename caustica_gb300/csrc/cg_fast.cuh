@@ -18,6 +18,8 @@
 // Taylor series of sin and cos (double precision, rounded once to float).
 #pragma once
 
+#include <stdlib.h>
+
 #include <type_traits>
 #include <utility>
 
@@ -572,6 +574,11 @@ __device__ __forceinline__ float2 ld_once(const float2* p) {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
+// Whether a handle's launches are programmatic: unless CG_PDL=0 when it is created.
+inline int pdl_default() {
+  const char* e = getenv("CG_PDL");
+  return (e && e[0] == '0') ? 0 : 1;
+}
 // Launch, with programmatic stream serialisation when `pdl` is set.
 template <typename... KArgs, typename... Args>
 inline void launch(int pdl, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

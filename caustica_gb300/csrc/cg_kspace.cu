@@ -840,13 +840,6 @@ static size_t smem_zpass(int nz) {
   return sizeof(float2) * ((size_t)nz + a + (a > st ? a : st));
 }
 
-// Programmatic dependent launch of the x- and z-passes unless CG_PDL=0 (the
-// y-passes never take it, yx_launch_y).
-static int pdl_default() {
-  const char* e = getenv("CG_PDL");
-  return (e && e[0] == '0') ? 0 : 1;
-}
-
 extern "C" int cg_solver_create(const cg_solver_config* cfg, cg_solver** out) {
   CG_REQUIRE(cfg && out, "null argument");
   *out = nullptr;
@@ -866,7 +859,7 @@ extern "C" int cg_solver_create(const cg_solver_config* cfg, cg_solver** out) {
   s->d.nzh = cfg->nz / 2 + 1;
   s->d.ncell = (long long)cfg->nx * cfg->ny * cfg->nz;
   s->d.nspec = (long long)cfg->nx * s->d.nzh * cfg->ny;
-  s->d.pdl = pdl_default();
+  s->d.pdl = cgf::pdl_default();
   s->B = cfg->batch;
   if (cg_make_plan(cfg->nx, &s->px) || cg_make_plan(cfg->ny, &s->py) || cg_make_plan(cfg->nz, &s->pz)) {
     cg_set_error("grid %dx%dx%d: every axis must be 2/3/5-smooth and <= %d", cfg->nx, cfg->ny, cfg->nz, CG_MAX_N);
@@ -1835,7 +1828,7 @@ extern "C" int cg_fft3d_create(int nx, int ny, int nz, int batch, cg_fft3d** out
   f->d.nx = nx; f->d.ny = ny; f->d.nz = nz; f->d.nzh = nz / 2 + 1;
   f->d.ncell = (long long)nx * ny * nz;
   f->d.nspec = (long long)nx * f->d.nzh * ny;
-  f->d.pdl = pdl_default();
+  f->d.pdl = cgf::pdl_default();
   f->B = batch;
   if (cg_make_plan(nx, &f->px) || cg_make_plan(ny, &f->py) || cg_make_plan(nz, &f->pz)) {
     cg_set_error("FFT shape %dx%dx%d: every axis must be 2/3/5-smooth and <= %d", nx, ny, nz, CG_MAX_N);

@@ -20,7 +20,7 @@ struct Dims {
   int nx, ny, nz, nzh;
   long long ncell;  // nx*ny*nz
   long long nspec;  // nx*nzh*ny
-  int pdl = 0;      // host: launch the x- and z-passes with programmatic stream serialisation
+  int pdl = 0;      // host: programmatic stream serialisation (x- and z-passes, y-passes by y_pdl)
 };
 
 struct Tables {

@@ -485,50 +485,50 @@ __global__ void __launch_bounds__(PP_Z * PP_Y) k_pennes_stream2(PennesDev P, int
 }
 
 template <bool FT, bool DOSE, bool DIR>
-static void launch_stream_k(bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs, const float* th,
-                            float* thn, float* thmax, float* dose, float* dcomp) {
+static void launch_stream_k(int pdl, bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs,
+                            const float* th, float* thn, float* thmax, float* dose, float* dcomp) {
   if (pair)
-    cgf::launch(1, k_pennes_stream2<FT, DOSE, DIR>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+    cgf::launch(pdl, k_pennes_stream2<FT, DOSE, DIR>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
   else
-    cgf::launch(1, k_pennes_stream<FT, DOSE, DIR>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+    cgf::launch(pdl, k_pennes_stream<FT, DOSE, DIR>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
 }
 
 template <bool FT, bool DOSE>
-static void launch_stream_dir(bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs,
+static void launch_stream_dir(int pdl, bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs,
                               const float* th, float* thn, float* thmax, float* dose, float* dcomp) {
   if (P.dirichlet)
-    launch_stream_k<FT, DOSE, true>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+    launch_stream_k<FT, DOSE, true>(pdl, pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
   else
-    launch_stream_k<FT, DOSE, false>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+    launch_stream_k<FT, DOSE, false>(pdl, pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
 }
 
-static void launch_stream(bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs, const float* th,
-                          float* thn, float* thmax, float* dose, float* dcomp) {
+static void launch_stream(int pdl, bool pair, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs,
+                          const float* th, float* thn, float* thmax, float* dose, float* dcomp) {
   if (P.ftab) {
     if (P.dose)
-      launch_stream_dir<true, true>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+      launch_stream_dir<true, true>(pdl, pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
     else
-      launch_stream_dir<true, false>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+      launch_stream_dir<true, false>(pdl, pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
   } else {
     if (P.dose)
-      launch_stream_dir<false, true>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+      launch_stream_dir<false, true>(pdl, pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
     else
-      launch_stream_dir<false, false>(pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
+      launch_stream_dir<false, false>(pdl, pair, P, g, b, st, xs, th, thn, thmax, dose, dcomp);
   }
 }
 
-static void launch_dense(const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs, const float* th, float* thn,
-                         float* thmax, float* dose, float* dcomp) {
+static void launch_dense(int pdl, const PennesDev& P, dim3 g, dim3 b, cudaStream_t st, int xs, const float* th,
+                         float* thn, float* thmax, float* dose, float* dcomp) {
   if (P.dose) {
     if (P.dirichlet)
-      cgf::launch(1, k_pennes_dense<true, true>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+      cgf::launch(pdl, k_pennes_dense<true, true>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
     else
-      cgf::launch(1, k_pennes_dense<true, false>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+      cgf::launch(pdl, k_pennes_dense<true, false>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
   } else {
     if (P.dirichlet)
-      cgf::launch(1, k_pennes_dense<false, true>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+      cgf::launch(pdl, k_pennes_dense<false, true>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
     else
-      cgf::launch(1, k_pennes_dense<false, false>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
+      cgf::launch(pdl, k_pennes_dense<false, false>, g, b, 0, st, P, xs, th, thn, thmax, dose, dcomp);
   }
 }
 
@@ -563,6 +563,7 @@ struct cg_pennes {
   float inv_dx2 = 0.f;
   int lab_poff = 0, wall_axes = 7;
   int has_coef = 0, has_state = 0;
+  int pdl = 0;  // launch the sub-steps programmatically
   cudaStream_t stream = nullptr;
 };
 
@@ -596,6 +597,7 @@ extern "C" int cg_pennes_create(const cg_pennes_config* cfg, cg_pennes** out) {
              "fewer than 2^31 cells", cfg->nx, cfg->ny, cfg->nz);
   cg_pennes* h = new cg_pennes();
   h->cfg = *cfg;
+  h->pdl = cgf::pdl_default();
   const long long nx = cfg->nx, ny = cfg->ny, nz = cfg->nz;
   h->ncell = nx * ny * nz;
   int rc = CG_OK;
@@ -776,8 +778,8 @@ extern "C" int cg_pennes_run(cg_pennes* h, int n_sub) {
   const PennesDev P = make_dev(h);
   // Both modes stream along x; label media take z-pairs when nz is even
   // (CG_PENNES_PAIR=0 keeps single cells). x planes per block (CG_PENNES_XS
-  // pins it): pennes_planes. Each sub-step is launched programmatically: its
-  // blocks fill their tables while the step before drains.
+  // pins it): pennes_planes. Each sub-step is launched programmatically (unless
+  // CG_PDL=0): its blocks fill their tables while the step before drains.
   static const int xs_pin = [] {
     const char* e = getenv("CG_PENNES_XS");
     return e ? atoi(e) : 0;
@@ -798,9 +800,11 @@ extern "C" int cg_pennes_run(cg_pennes* h, int n_sub) {
   const dim3 dgrid((unsigned)tiles_zy, sgrid.z);  // dense maps: z-y tiles along one grid dimension (any ny)
   for (int i = 0; i < n_sub; ++i) {
     if (P.labels)
-      launch_stream(pair, P, sgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
+      launch_stream(h->pdl, pair, P, sgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose,
+                    h->dcomp);
     else
-      launch_dense(P, dgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose, h->dcomp);
+      launch_dense(h->pdl, P, dgrid, sblock, h->stream, xs, h->th[h->cur], h->th[1 - h->cur], h->thmax, h->dose,
+                   h->dcomp);
     h->cur = 1 - h->cur;
   }
   CG_CUDA_TRY(cudaGetLastError());
