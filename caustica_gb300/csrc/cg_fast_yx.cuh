@@ -335,13 +335,7 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
   if (XT<N>::TPP <= 16) __syncthreads();
   load(MODE == X_GRAD ? S0 : S1);
   if (XT<N>::TPP > 16) __syncthreads();
-  if constexpr (MODE == X_FWD || MODE == X_INV) {  // S0 <- (I)FFT(S1); S1 may be S0
-    fft2<A, B, MODE == X_INV>(v, w, s, tw, exf);
-    if (valid && s < OA) static_for<0, OB>([&](auto bi) {
-      constexpr int b = decltype(bi)::value;
-      S0[base + (long long)(s + OA * b) * ncol] = w[b];
-    });
-  } else if constexpr (MODE == X_GRAD) {
+  if constexpr (MODE == X_GRAD) {
     // S2 <- IFFT(q); S1 <- IFFT(i kx q), q = kappa/N FFT(S0); q waits in shared
     // memory during the first inverse transform instead of in registers
     float2* qs = sm + XB + XT<N>::EX;
@@ -382,6 +376,40 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
   }
 }
 
+// The x-transform alone: dst <- (I)FFT(src). src may be dst (a column is read
+// whole before any of it is written), so neither is __restrict__.
+template <int N, bool INV>
+__global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(X_FWD)) kf_xhalf(Dims d, Tables t, const float2* src,
+                                                                           float2* dst) {
+  constexpr int A = PSplit<N>::A, B = PSplit<N>::B, OA = PSplit<N>::OA, OB = PSplit<N>::OB, XP = XT<N>::XP;
+  extern __shared__ float2 sm[];
+  cgf::pdl_trigger();
+  cgf::fill_twt<A, B, OB>(sm, t.twx);  // (A, B) order
+  cgf::pdl_wait();
+  const int c = threadIdx.x % XP, s = threadIdx.x / XP;
+  const ColEx<A, B, XP> ex{sm + PSplit<N>::TW + c};
+  const long long ncol = (long long)d.nzh * d.ny;
+  const long long col = (long long)blockIdx.x * XP + c;
+  const bool valid = col < ncol;
+  const long long base = (long long)blockIdx.y * d.nspec + col;
+  if (XT<N>::TPP <= 16) __syncthreads();
+  float2 v[A], w[OB];
+  static_for<0, A>([&](auto ai) {
+    constexpr int a = decltype(ai)::value;
+    const float2* g = src + (base + (long long)(s + B * a) * ncol);
+    if constexpr (XT<N>::TPP == 20)  // as in kf_xpass
+      v[a] = (valid && s < B) ? *g : make_float2(0.f, 0.f);
+    else
+      v[a] = (valid && s < B) ? cgf::ld_once(g) : make_float2(0.f, 0.f);
+  });
+  if (XT<N>::TPP > 16) __syncthreads();
+  fft2<A, B, INV>(v, w, s, sm, ex);
+  if (valid && s < OA) static_for<0, OB>([&](auto bi) {
+    constexpr int b = decltype(bi)::value;
+    dst[base + (long long)(s + OA * b) * ncol] = w[b];
+  });
+}
+
 // twiddles | exchange | (x: a parked spectrum tile, k_x, k_x^2)
 template <int N>
 static size_t smem_y() {
@@ -390,6 +418,10 @@ static size_t smem_y() {
 template <int N>
 static size_t smem_x() {
   return sizeof(float2) * (XT<N>::TABLES * PSplit<N>::TW + XT<N>::EX + (size_t)N * XT<N>::XP) + 2 * sizeof(float) * N;  // + parked tile, k_x, k_x^2
+}
+template <int N>
+static size_t smem_xhalf() {
+  return sizeof(float2) * (PSplit<N>::TW + ColEx<PSplit<N>::A, PSplit<N>::B, XT<N>::XP>::SLAB);
 }
 
 // ------------------------------------------------ per-length launchers --
@@ -430,8 +462,8 @@ bool yx_launch_x(int mode, const Dims& d, const Tables& t, float kcoef, float in
   switch (mode) {
     case X_GRAD: cgf::launch(d.pdl, kf_xpass<N, X_GRAD>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
     case X_DIV: cgf::launch(d.pdl, kf_xpass<N, X_DIV>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
-    case X_FWD: cgf::launch(d.pdl, kf_xpass<N, X_FWD>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
-    default: cgf::launch(d.pdl, kf_xpass<N, X_INV>, grid, block, smem_x<N>(), st, d, t, kcoef, invN, S0, S1, S2); break;
+    case X_FWD: cgf::launch(d.pdl, kf_xhalf<N, false>, grid, block, smem_xhalf<N>(), st, d, t, (const float2*)S1, S0); break;
+    default: cgf::launch(d.pdl, kf_xhalf<N, true>, grid, block, smem_xhalf<N>(), st, d, t, (const float2*)S1, S0); break;
   }
   return true;
 }
@@ -447,22 +479,19 @@ bool plane_launch(bool div, const Dims& d, const Tables& t, float kcoef, float i
   return true;
 }
 
-template <int N, int M>
-static int allow_yx() {
-  const int sy = (int)smem_y<N>(), sx = (int)smem_x<N>();
-  if (cudaFuncSetAttribute(kf_ypass<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, sy) != cudaSuccess) return -1;
-  if (cudaFuncSetAttribute(kf_xpass<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx) != cudaSuccess) return -1;
-  return 0;
+template <typename K>
+static bool yx_allow(K kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
-
-// Y_* and X_* modes are both 0..3
 template <int N>
 int yx_prepare() {
-  const int sp = (int)smem_plane<N>();
-  if (cudaFuncSetAttribute(kf_plane<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp) != cudaSuccess ||
-      cudaFuncSetAttribute(kf_plane<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp) != cudaSuccess)
-    return -1;
-  return (allow_yx<N, 0>() || allow_yx<N, 1>() || allow_yx<N, 2>() || allow_yx<N, 3>()) ? -1 : 0;
+  const size_t sy = smem_y<N>(), sx = smem_x<N>(), sh = smem_xhalf<N>(), sp = smem_plane<N>();
+  return yx_allow(kf_ypass<N, Y_FWD>, sy) && yx_allow(kf_ypass<N, Y_INV>, sy) && yx_allow(kf_ypass<N, Y_INV_GRAD>, sy) &&
+                 yx_allow(kf_ypass<N, Y_FWD_DIV>, sy) && yx_allow(kf_xpass<N, X_GRAD>, sx) &&
+                 yx_allow(kf_xpass<N, X_DIV>, sx) && yx_allow(kf_xhalf<N, false>, sh) &&
+                 yx_allow(kf_xhalf<N, true>, sh) && yx_allow(kf_plane<N, false>, sp) && yx_allow(kf_plane<N, true>, sp)
+             ? 0
+             : -1;
 }
 
 #define CG_YX_INSTANTIATE(n)                                                                                   \
