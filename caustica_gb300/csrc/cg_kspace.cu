@@ -22,6 +22,7 @@
 //   Yf_div(-> S1 = FFTy Vx, S0 = i ky FFTy Vy + FFTy Wz) -> Xdiv(-> S0) ->
 //   Yinv(S0) -> Zp(p update, source, peak, record, R2C p -> S0)
 // The 1/N of the inverse transforms is folded into kappa.
+#include <cudaTypedefs.h>  // PFN_cuMemGetAddressRange_v3020
 #include <math.h>
 
 #include <map>
@@ -1891,17 +1892,30 @@ static Tables fft_tables(const cg_fft3d* f) {
 }
 
 // Whether a transform can work on the caller's buffer itself: memory of the
-// current device, aligned for the passes' accesses. Host buffers and others go
-// through the handle's staging arrays.
-static bool direct(const void* p, size_t align) {
+// current device, aligned for the passes' accesses, and all of it within one
+// allocation. Host buffers and others go through the handle's staging arrays,
+// by copies that the driver checks.
+static bool direct(const void* p, size_t bytes, size_t align) {
+  static const PFN_cuMemGetAddressRange_v3020 range = []() -> PFN_cuMemGetAddressRange_v3020 {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+    cudaGetLastError();
+    return nullptr;
+  }();
   int dev = 0;
   cudaPointerAttributes at;
-  if (((uintptr_t)p & (align - 1)) != 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (!range || ((uintptr_t)p & (align - 1)) != 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return (at.type == cudaMemoryTypeDevice && at.device == dev) || at.type == cudaMemoryTypeManaged;
+  if (!((at.type == cudaMemoryTypeDevice && at.device == dev) || at.type == cudaMemoryTypeManaged)) return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  return range(&base, &size, (CUdeviceptr)(uintptr_t)p) == CUDA_SUCCESS && (uintptr_t)p + bytes <= (uintptr_t)base + size;
 }
 
 extern "C" int cg_fft3d_forward(cg_fft3d* f, const float* in, float* out_spec) {
@@ -1920,7 +1934,7 @@ extern "C" int cg_fft3d_forward(cg_fft3d* f, const float* in, float* out_spec) {
   // overlap are staged
   const uintptr_t ia = (uintptr_t)in, oa = (uintptr_t)out_spec;
   const bool apart = ia + in_bytes <= oa || oa + out_bytes <= ia;
-  const bool in_ok = apart && direct(in, 4), out_ok = direct(out_spec, 16);
+  const bool in_ok = apart && direct(in, in_bytes, 4), out_ok = direct(out_spec, out_bytes, 16);
   float* real = in_ok ? const_cast<float*>(in) : f->real;
   float2* spec = out_ok ? (float2*)out_spec : f->spec;
   if (!in_ok) CG_CUDA_TRY(cudaMemcpyAsync(real, in, in_bytes, cudaMemcpyDefault, f->stream));
@@ -1952,11 +1966,12 @@ extern "C" int cg_fft3d_inverse(cg_fft3d* f, const float* in_spec, float* out) {
   rd.spp = 1;
   // the x-pass takes the caller's spectrum to the handle's (which it leaves as
   // it is), the z-pass writes the caller's rows; by then the spectrum is read
-  const bool in_ok = direct(in_spec, 8), out_ok = direct(out, 4);
+  const size_t in_bytes = sizeof(float2) * f->B * d.nspec, out_bytes = sizeof(float) * f->B * d.ncell;
+  const bool in_ok = direct(in_spec, in_bytes, 8), out_ok = direct(out, out_bytes, 4);
   float2* src = in_ok ? (float2*)const_cast<float*>(in_spec) : f->spec;
   float* real = out_ok ? out : f->real;
   if (!in_ok)
-    CG_CUDA_TRY(cudaMemcpyAsync(src, in_spec, sizeof(float2) * f->B * d.nspec, cudaMemcpyDefault, f->stream));
+    CG_CUDA_TRY(cudaMemcpyAsync(src, in_spec, in_bytes, cudaMemcpyDefault, f->stream));
   const dim3 gy((unsigned)((d.nx * (long long)d.nzh + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gx((unsigned)(((long long)d.nzh * d.ny + CG_TILE - 1) / CG_TILE), f->B);
   const dim3 gz((unsigned)(d.nx * ((d.ny + CG_ZROWS - 1) / CG_ZROWS)), f->B);
@@ -1968,7 +1983,7 @@ extern "C" int cg_fft3d_inverse(cg_fft3d* f, const float* in_spec, float* out) {
     k_zpass_p<<<gz, CG_THREADS, f->smem_z, f->stream>>>(2, d, f->pz, t, m, sd, rd, nullptr, 0, 0, real, f->spec);
   CG_CUDA_TRY(cudaGetLastError());
   if (!out_ok)
-    CG_CUDA_TRY(cudaMemcpyAsync(out, real, sizeof(float) * f->B * d.ncell, cudaMemcpyDefault, f->stream));
+    CG_CUDA_TRY(cudaMemcpyAsync(out, real, out_bytes, cudaMemcpyDefault, f->stream));
   CG_CUDA_TRY(cudaStreamSynchronize(f->stream));
   return CG_OK;
 }
