@@ -169,20 +169,28 @@ FAST_XYZ_SIZES = FAST_SIZES | {2**a * 3**b * 5**c for a in range(8) for b in ran
                                if 36 <= 2**a * 3**b * 5**c <= 400} | {512, 640}
 
 
-def slot_symbols(padded3, persistent_z: bool = True, tma: bool = False) -> list[str]:
+def slot_symbols(padded3, persistent_z: bool = True, tma: bool = False, config: dict | None = None) -> list[str]:
     """The kernel each step slot launches on this grid (size-specialised where the axis allows);
     ``persistent_z`` and ``tma`` are the autotuner's z-pass choices (lengths without a per-tile
-    kernel are always persistent when ny is even; ``tma``: tensor-map staging of the z-tiles)."""
+    kernel are always persistent when ny is even; ``tma``: tensor-map staging of the z-tiles).
+    ``config``, a handle's own (``DeviceSolver.config()``), overrides both and names what it runs:
+    persistent z-passes on an odd ny too, and one kernel per transverse chain of one x plane
+    (slots 0 and 4; the chain's other slots launch nothing)."""
     nx, ny, nz = padded3
+    if config is not None:
+        persistent_z, tma = config["persistent_z"], config["tma_staging"]
     y = f"kf_ypass<{ny},{{}}>" if ny in FAST_XYZ_SIZES else "k_ypass"
     x = f"kf_xpass<{nx},{{}}>" if nx in FAST_XYZ_SIZES else "k_xpass"
-    zp = "kfp" if ny % 2 == 0 and (persistent_z or nz not in FAST_SIZES) else "kf"
+    rows_ok = ny % 2 == 0 or config is not None
+    zp = "kfp" if rows_ok and (persistent_z or nz not in FAST_SIZES) else "kf"
     zfast = nz in (FAST_XYZ_SIZES if zp == "kfp" else FAST_SIZES)
     tma = bool(tma and zp == "kfp" and zfast)
     zu = (f"{zp}_zpass_u<{nz},true>" if tma else f"{zp}_zpass_u<{nz}>") if zfast else "k_zpass_u"
     # the timed steps do not record: the persistent p-pass runs its record-free instantiation
     zpp = ((f"{zp}_zpass_p<{nz},false,false,true>" if tma else f"{zp}_zpass_p<{nz},false>") if zp == "kfp"
            else f"kf_zpass_p<{nz},1>") if zfast else "k_zpass_p"
+    if config is not None and nx == 1 and ny in FAST_XYZ_SIZES:
+        return [f"kf_plane<{ny},false>", "", "", zu, f"kf_plane<{ny},true>", "", "", zpp]
     return [y.format("Y_FWD"), x.format("X_GRAD"), y.format("Y_INV_GRAD"), zu, y.format("Y_FWD_DIV"),
             x.format("X_DIV"), y.format("Y_INV"), zpp]
 
@@ -303,7 +311,7 @@ def run_gb300(args, dist, rank, ws, local):
     dev = eng.DeviceSolver(plan)
     launches_per_step = dev.launches_per_step
     tuning = dev.tuning
-    staging_tma = dev.config()["tma_staging"]  # the staging in effect (also without the autotuner)
+    config = dev.config()  # the launch configuration in effect (also without the autotuner)
     try:
         # drive table long enough that the source keeps injecting through the timed steps
         dev.extend_drive((plan.eff_min + 4) * plan.spp + W + 2 * K)
@@ -336,7 +344,7 @@ def run_gb300(args, dist, rank, ws, local):
     dom = int(np.argmax(per_launch_ms))
     achieved = bytes_slot[dom] / (per_launch_ms[dom] * 1e-3) / 1e9
     kernel_name = SLOTS[dom]
-    symbols = slot_symbols(plan.padded3, bool((tuning or {}).get("persistent_z", True)), bool(staging_tma))
+    symbols = slot_symbols(plan.padded3, config=config)
     traffic = _traffic_from_profiles(kernel_name)
     step_b = step_algorithmic_bytes(info_labels, True)
     step_achieved = step_b * value / ws / 1e9
