@@ -128,10 +128,8 @@ constexpr int ct_crt(int k1, int k2, int A, int B) {
 // everywhere -> as it is: 192x192x256 275.7 -> 274.6 us, 320^3 1182 -> 1165,
 // 384^3 1946 -> 1895, 400^3 2173 -> 2111; the error of a round trip against 64
 // bits 1.86e-7 -> 1.79e-7 at 180 points, 2.05e-7 -> 1.89e-7 at 400.
-// FINE: the factors of 3 multiply by sqrt(3)/2 as a pair of floats. So in the
-// powers of 3, whose twiddles between the factors add errors of their own (a
-// transform of 81, 162, 243 or 324 points 5 % further off 64 bits without).
-template <int R, bool INV, bool FINE = (R % 9 == 0)>
+// FINE: the factors of 5 multiply by sin(2 pi/5) as a pair of floats (fft2).
+template <int R, bool INV, bool FINE>
 struct Dft {
   static constexpr int A = ct_first_factor(R), B = R / A;
   static constexpr bool COPRIME = ct_gcd(A, B) == 1;
@@ -202,11 +200,14 @@ struct Dft<2, INV, FINE> {
 template <bool INV, bool FINE>
 struct Dft<3, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
+    // sqrt(3)/2 as a pair of floats: the error of one, 1.6e-8, is the same in
+    // every transform of every step and adds up (whole-field phasors of
+    // 144x180x192 2.0e-6 -> 1.4e-6 from 64 bits)
     const float h = 0.86602540378443864676f, hl = (float)(0.86602540378443864676 - (double)h);
     float2 t = c_add(v[1], v[2]);
     float2 d = c_sub(v[1], v[2]);
     float2 m = c_fma(t, -0.5f, v[0]);
-    float2 r = rot<INV>(FINE ? c_fma(d, h, c_scale(d, hl)) : c_scale(d, h));
+    float2 r = rot<INV>(c_fma(d, h, c_scale(d, hl)));
     v[0] = c_add(v[0], t);
     v[1] = c_add(m, r);
     v[2] = c_sub(m, r);
@@ -232,6 +233,7 @@ struct Dft<5, INV, FINE> {
   __host__ __device__ __forceinline__ static void run(float2* v) {
     const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
     const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
+    const float s1l = (float)(0.95105651629515357212 - (double)s1);
     float2 t1 = c_add(v[1], v[4]);
     float2 t2 = c_add(v[2], v[3]);
     float2 t3 = c_sub(v[1], v[4]);
@@ -239,8 +241,9 @@ struct Dft<5, INV, FINE> {
     float2 y0 = c_add(v[0], c_add(t1, t2));
     float2 b1 = c_fma(t2, c2, c_fma(t1, c1, v[0]));
     float2 b2 = c_fma(t2, c1, c_fma(t1, c2, v[0]));
-    float2 e1 = c_fma(t3, s1, c_scale(t4, s2));
-    float2 e2 = c_fma(t4, -s1, c_scale(t3, s2));
+    const float2 e1l = c_scale(t4, s2), e2l = c_scale(t3, s2);
+    float2 e1 = c_fma(t3, s1, FINE ? c_fma(t3, s1l, e1l) : e1l);
+    float2 e2 = c_fma(t4, -s1, FINE ? c_fma(t4, -s1l, e2l) : e2l);
     float2 r1 = rot<INV>(e1);
     float2 r2 = rot<INV>(e2);
     v[0] = y0;
@@ -257,8 +260,8 @@ struct Dft<8, INV, FINE> {
     const float r2 = 0.70710678118654752440f;
     float2 e[4] = {v[0], v[2], v[4], v[6]};
     float2 o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<4, INV>::run(e);
-    Dft<4, INV>::run(o);
+    Dft<4, INV, FINE>::run(e);
+    Dft<4, INV, FINE>::run(o);
     // o[1] and o[3] without their factor r2, which the last sums apply
     o[1] = INV ? make_float2(o[1].x - o[1].y, o[1].x + o[1].y) : make_float2(o[1].x + o[1].y, o[1].y - o[1].x);
     o[2] = rot<INV>(o[2]);
@@ -297,6 +300,15 @@ constexpr int ct_even_split(int n) {
 // step 251 -> 108 us at 125^3, 1207 -> 643 at 243^3, 3537 -> 2624 at 375^3).
 constexpr int ct_three_d(int b) { return ct_even_split(b); }
 constexpr bool ct_three(int a, int b) { return b > 20 && a % ct_three_d(b) == 0 && a % (b / ct_three_d(b)) == 0; }
+
+// Whether the 5-point codelets of a split (a, b) take sin(2 pi/5) as a pair of
+// floats. One float is 2.5e-8 too large, in every transform of every step; the
+// twiddles inside a codelet of 8, 16 or 32 points (cos(pi/4), cos(pi/8)) are up
+// to 2.9e-8 too small, and beside one of those the two make up for each other.
+// Phasors from 64 bits (1e-6), pair / float: 100x125x135 0.91 / 1.9, 200^3 1.2 /
+// 1.9, 125^3 1.2 / 1.9; beside 16 points 128x128x320 2.0 / 1.8, quiet phasors of
+// 96x96x320 24.5 / 20.0.
+constexpr bool ct_fine(int a, int b) { return a % 8 != 0 && b % 8 != 0; }
 
 // Threads per pencil for a split whose larger factor is m: 8 or 16 (whole
 // pencils per warp), else m rounded up to 4 so that 8 pencils fill whole warps.
@@ -400,10 +412,11 @@ template <int V, int T, bool INV, class Ex>
 __device__ __forceinline__ void fft3(const float2 (&v_in)[V], float2 (&w)[V], int s, const float2* __restrict__ twt,
                                      const Ex& ex) {
   constexpr int D = ct_three_d(T), C = T / D, JC = V / C, JD = V / D;
+  constexpr bool FINE = ct_fine(V, T);
   if (s < T) {
     float2 v[V];
     static_for<0, V>([&](auto i) { v[decltype(i)::value] = v_in[decltype(i)::value]; });
-    Dft<V, INV>::run(v);
+    Dft<V, INV, FINE>::run(v);
     static_for<0, V>([&](auto ki) {
       constexpr int k1 = decltype(ki)::value;
       float2 y = v[k1];
@@ -422,7 +435,7 @@ __device__ __forceinline__ void fft3(const float2 (&v_in)[V], float2 (&w)[V], in
       const int k1 = k0 + C * decltype(ji)::value;
       float2 q[C];
       static_for<0, C>([&](auto ci) { q[decltype(ci)::value] = ex.at(k1, D * decltype(ci)::value + d); });
-      Dft<C, INV>::run(q);
+      Dft<C, INV, FINE>::run(q);
       static_for<0, C>([&](auto ki) {
         constexpr int kc = decltype(ki)::value;
         if constexpr (kc > 0) {
@@ -441,7 +454,7 @@ __device__ __forceinline__ void fft3(const float2 (&v_in)[V], float2 (&w)[V], in
       const int m = s + T * j, kc = m / V, k1 = m - V * kc;
       float2 q[D];
       static_for<0, D>([&](auto di) { q[decltype(di)::value] = ex.at(k1, D * kc + decltype(di)::value); });
-      Dft<D, INV>::run(q);
+      Dft<D, INV, FINE>::run(q);
       static_for<0, D>([&](auto ki) { w[j + JD * decltype(ki)::value] = q[decltype(ki)::value]; });
     });
   }
@@ -459,10 +472,11 @@ __device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[R], in
     fft3<A, B, INV>(v_in, w, s, twt, ex);
     return;
   } else {
+    constexpr bool FINE = ct_fine(A, B);
     if (s < B) {
       float2 v[A];
       static_for<0, A>([&](auto i) { v[decltype(i)::value] = v_in[decltype(i)::value]; });
-      Dft<A, INV>::run(v);
+      Dft<A, INV, FINE>::run(v);
       static_for<0, A>([&](auto ki) {
         constexpr int k1 = decltype(ki)::value;
         float2 y = v[k1];
@@ -477,7 +491,7 @@ __device__ __forceinline__ void fft2(const float2 (&v_in)[A], float2 (&w)[R], in
     ex_sync<Ex>();
     if (s < A) {
       static_for<0, B>([&](auto bi) { w[decltype(bi)::value] = ex.at(s, decltype(bi)::value); });
-      Dft<B, INV>::run(w);
+      Dft<B, INV, FINE>::run(w);
     }
     ex_sync<Ex>();
   }
