@@ -581,6 +581,16 @@ __device__ __forceinline__ float2 ld_once(const float2* p) {
   return v;
 }
 
+// A read-only value, loaded in program order.
+__device__ __forceinline__ float ld_ordered(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];\n" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Starts the fetch of the line that holds *p into the L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
 // Programmatic dependent launch: a pass lets the next one launch as soon as
 // all of its own CTAs are running (pdl_trigger), and waits for the previous
 // pass to complete and its writes to be visible (pdl_wait) before its first

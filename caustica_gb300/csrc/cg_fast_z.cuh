@@ -816,23 +816,39 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     const bool va = ya < d.ny, vb = yb < d.ny;  // this pencil's rows exist
     const long long rowa = ((long long)x * d.ny + ya) * N, rowb = rowa + N;
     float* uc = u + ((long long)comp * n_members + b_idx) * d.ncell;
-    // this thread's velocities load while the staged spectrum is transformed
-    // (after it where A-value registers would not leave room for them)
+    // this thread's velocities load while the staged spectrum is transformed.
+    // LATE: after it, where A-value registers would not leave room for them, a
+    // chunk of cells at a time and in program order, from the L2, where the pencil
+    // fetches its rows when the item starts. (The compiler otherwise moves each
+    // load down to its use, a round trip to memory a cell. u-pass us, one block of
+    // loads / in chunks / and fetched: 128x128x512 220 / 220 / 127, 512^3 3173 / 3166 /
+    // 1733, 256x256x640 804 / 770 / 640, dense 128x128x640 273 / 242 / 222. One CTA
+    // of 16 warps an SM: nothing else hides the latency.)
+    constexpr bool LATE = !Z::EARLY && !L::BULK;
     float ua[OB], ub[OB];
-    auto load_u = [&]() {
-      static_for<0, OB>([&](auto bi) {
-        constexpr int b = decltype(bi)::value;
+    auto load_u = [&](auto first, auto count) {
+      static_for<0, decltype(count)::value>([&](auto ji) {
+        constexpr int b = decltype(first)::value + decltype(ji)::value;
         const int n = s + OA * b;
-        ua[b] = (s < OA && va) ? __ldg(uc + rowa + n) : 0.f;
-        ub[b] = (s < OA && vb) ? __ldg(uc + rowb + n) : 0.f;
+        if constexpr (LATE) {
+          ua[b] = va ? cgf::ld_ordered(uc + rowa + n) : 0.f;
+          ub[b] = vb ? cgf::ld_ordered(uc + rowb + n) : 0.f;
+        } else {
+          ua[b] = (s < OA && va) ? __ldg(uc + rowa + n) : 0.f;
+          ub[b] = (s < OA && vb) ? __ldg(uc + rowb + n) : 0.f;
+        }
       });
     };
+    using All = std::integral_constant<int, OB>;
+    using Zero = std::integral_constant<int, 0>;
     float* const rows = rows_of(cur);
     const unsigned bytes = rows_bytes(cur);
     // the sponge's x and y factors, read ahead of the transform (192x192x256 97.1 ->
     // 93.0 us, 160x160x192 x 8 375 -> 369; lengths of 20 threads the same)
     const float spx = t.sx[x], sya = va ? t.sy[ya] : 0.f, syb = vb ? t.sy[yb] : 0.f;
-    if (Z::EARLY && !L::BULK) load_u();
+    if (Z::EARLY && !L::BULK) load_u(Zero{}, All{});
+    if constexpr (LATE)
+      for (int i = s; 32 * i < (va + vb) * N; i += Z::TPP) cgf::prefetch_l2(uc + rowa + 32 * i);
     // (tensor-map path) this thread's generic accesses to the buffer the
     // next copy fills are ordered before that copy
     if constexpr (TMA) cgf::fence_proxy_async();
@@ -848,7 +864,6 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
     const RowEx<A, B, Z::WARP> exi{bufj + p * Z::EX};
     const RowEx<OB, OA, Z::WARP> exf{bufj + p * Z::EX};
     fft2<A, B, true>(v, w, s, sm, exi);
-    if (!Z::EARLY && !L::BULK) load_u();
     if constexpr (L::BULK) {
       zt_wait(bars, phase, 2, ztma.err);
       static_for<0, OB>([&](auto bi) {
@@ -879,15 +894,22 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, ZPLayout<N, true, TMA>::M
       }
       w[b] = make_float2(una, vb ? unb : 0.f);
     };
+    constexpr int RC = z_chunk(OB);
+    using Chunk = std::integral_constant<int, RC>;
     if constexpr (lab) {
-      if (s < OA) static_for<0, OB>([&](auto bi) {
-        const int n = s + OA * decltype(bi)::value;
-        update(bi, tab2_s[la[n]], tab2_s[lb[n]]);
+      if (s < OA) static_for<0, OB / RC>([&](auto ci) {
+        constexpr int c0 = decltype(ci)::value * RC;
+        if constexpr (LATE) load_u(std::integral_constant<int, c0>{}, Chunk{});
+        static_for<0, RC>([&](auto ji) {
+          constexpr int b = c0 + decltype(ji)::value;
+          const int n = s + OA * b;
+          update(std::integral_constant<int, b>{}, tab2_s[la[n]], tab2_s[lb[n]]);
+        });
       });
     } else if (s < OA) {
-      constexpr int RC = z_chunk(OB);
       static_for<0, OB / RC>([&](auto ci) {
         constexpr int c0 = decltype(ci)::value * RC;
+        if constexpr (LATE) load_u(std::integral_constant<int, c0>{}, Chunk{});
         float2 ca[RC], cb[RC];
         static_for<0, RC>([&](auto ji) {
           constexpr int j = decltype(ji)::value;
@@ -1045,8 +1067,8 @@ __global__ void __launch_bounds__(ZPShape<N>::THREADS, FWD ? ZPFwd<N>::MINB : ZP
     float* const rows = rows_of(cur);
     const unsigned bytes = rows_bytes(cur);
     // the sponge's x and y factors, read ahead of the transform where 16 threads
-    // hold the cells (192x192x256 41.0 -> 39.4 us, 160x160x192 x 8 148 -> 144); else
-    // they would spill (300^3 138 -> 148, 150^3 24.6 -> 26.0)
+    // hold the cells (192x192x256 41.0 -> 39.4 us); else they would spill (300^3 138
+    // -> 148, 150^3 24.6 -> 26.0) or not pay (160x160x192 x 8, 12 threads, 149 -> 152)
     constexpr bool SP = A == 16 && !INV;
     float spx = 0.f, sya = 0.f, syb = 0.f;
     auto sponge_xy = [&]() {
