@@ -80,6 +80,10 @@ struct XT {
   // 324^3 173 / 174 -> 162 / 164, 144x180x192 25.4 / 26.6 -> 25.0 / 24.6)
   static constexpr bool TR = S::A != S::OB && S::OB % 16 != 0;
   static constexpr int TABLES = S::A == S::OB || TR ? 1 : 2;
+  // X_GRAD loops over one copy of its inverse transform, whose 32-value codelets
+  // are long: two copies / one, 512x128x128 62 / 49 us, 640x128x128 76 / 65, 512^3
+  // 709 / 603
+  static constexpr bool LOOP = TPP == 32;
   static constexpr int minb(int mode) {
     if (TPP <= 16) return 16 / TPP * (mode != X_DIV ? CG_FAST_MINB_XG : CG_FAST_MINB_X);
     if (PSplit<N>::THREE) return PSplit<N>::A <= 10 ? 4 : 3;
@@ -346,15 +350,27 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
       w[b] = c_scale(w[b], kappa(k));
       if (s < OA) qs[(s + OA * b) * XP + c] = w[b];
     });
-    fft2<OB, OA, true, TR>(w, z, s, twi, exi);
-    store_z(S2);
-    static_for<0, OB>([&](auto bi) {
-      constexpr int b = decltype(bi)::value;
-      const int k = (s < OA) ? s + OA * b : 0;
-      w[b] = (s < OA) ? c_muli(c_scale(qs[(s + OA * b) * XP + c], kxs[k])) : make_float2(0.f, 0.f);
-    });
-    fft2<OB, OA, true, TR>(w, z, s, twi, exi);
-    store_z(S1);
+    auto times_ikx = [&]() {
+      static_for<0, OB>([&](auto bi) {
+        constexpr int b = decltype(bi)::value;
+        const int k = (s < OA) ? s + OA * b : 0;
+        w[b] = (s < OA) ? c_muli(c_scale(qs[(s + OA * b) * XP + c], kxs[k])) : make_float2(0.f, 0.f);
+      });
+    };
+    if constexpr (XT<N>::LOOP) {
+#pragma unroll 1
+      for (int i = 0; i < 2; ++i) {
+        if (i) times_ikx();
+        fft2<OB, OA, true, TR>(w, z, s, twi, exi);
+        store_z(i ? S1 : S2);
+      }
+    } else {
+      fft2<OB, OA, true, TR>(w, z, s, twi, exi);
+      store_z(S2);
+      times_ikx();
+      fft2<OB, OA, true, TR>(w, z, s, twi, exi);
+      store_z(S1);
+    }
   } else {
     // X_DIV: S0 <- IFFT(kappa/N (FFT(S0) + i kx FFT(S1))); FFT(S1) waits in shared memory
     float2* hs = sm + XB + XT<N>::EX;
