@@ -451,9 +451,13 @@ static size_t smem_xhalf() {
 // y-passes) where 16-thread x-CTAs leave 64 KB of L1 (nx <= 192) and the grid
 // is not so small that waiting CTAs delay the x-pass: with / without, 192x192x256
 // 279 / 282 us, 128x128x160 96 / 100, 96x96x128 54 / 54, 64^3 36 / 33, 240^3
-// 471 / 444, 300^3 1126 / 1114.
-static inline int y_pdl(int mode, const Dims& d) {
-  return d.pdl && (mode == Y_INV || mode == Y_INV_GRAD) && d.nx <= 192 && d.ncell >= (1 << 20);
+// 471 / 444, 300^3 1126 / 1114. On more x planes up to 2^23 cells in all (the
+// three spectra, 100 MB, then fit the L2): 256x256x128 253 / 298, 320x128x128 186 /
+// 200, 400x128x128 238 / 254, 512x128x128 324 / 342; not above: 240x240x180 329 /
+// 317, 256x192x256 387 / 371, 512x160x160 515 / 476.
+static inline int y_pdl(int mode, const Dims& d, int batch) {
+  if (!d.pdl || (mode != Y_INV && mode != Y_INV_GRAD) || d.ncell < (1 << 20)) return 0;
+  return d.nx <= 192 || d.ncell * batch <= (1 << 23);
 }
 
 template <int N>
@@ -462,10 +466,10 @@ bool yx_launch_y(int mode, const Dims& d, const Tables& t, float2* S0, float2* S
   const dim3 grid((unsigned)((d.nx * (long long)d.nzh + YT<N>::YP - 1) / YT<N>::YP), batch);
   const dim3 block(YT<N>::THREADS);
   switch (mode) {
-    case Y_FWD: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_FWD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    case Y_INV: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_INV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    case Y_INV_GRAD: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_INV_GRAD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
-    default: cgf::launch(y_pdl(mode, d), kf_ypass<N, Y_FWD_DIV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_FWD: cgf::launch(y_pdl(mode, d, batch), kf_ypass<N, Y_FWD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_INV: cgf::launch(y_pdl(mode, d, batch), kf_ypass<N, Y_INV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    case Y_INV_GRAD: cgf::launch(y_pdl(mode, d, batch), kf_ypass<N, Y_INV_GRAD>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
+    default: cgf::launch(y_pdl(mode, d, batch), kf_ypass<N, Y_FWD_DIV>, grid, block, smem_y<N>(), st, d, t, S0, S1, S2); break;
   }
   return true;
 }
