@@ -316,11 +316,12 @@ __global__ void __launch_bounds__(XT<N>::THREADS, XT<N>::minb(MODE)) kf_xpass(Di
     static_for<0, A>([&](auto ai) {
       constexpr int a = decltype(ai)::value;
       const float2* g = src + (base + (long long)(s + B * a) * ncol);
-      // in program order: the compiler otherwise starts the divergence pass's
-      // second tile under the first transform and spills (X_GRAD / X_DIV us,
-      // plain against ordered: 192x192x256 41 / 41 -> 39 / 39, 240^3 58 / 70 ->
-      // 55 / 59, 384^3 269 / 304 -> 267 / 282; 20 threads a pencil have the
-      // registers for it: 400^3 309 / 290 -> 309 / 298)
+      // in program order (X_GRAD / X_DIV us, plain against ordered: 192x192x256 41 /
+      // 41 -> 39 / 39, 240^3 58 / 70 -> 55 / 59, 384^3 269 / 304 -> 267 / 282): the
+      // compiler otherwise starts the divergence pass's second tile under the
+      // first transform. It spills either way (X_DIV ordered, 192 / 240 points:
+      // 44 / 92 bytes). 20 threads a pencil do better plain: 400^3 309 / 290 against
+      // 309 / 298
       if constexpr (PSplit<N>::TPP == 20)
         v[a] = (valid && s < B) ? *g : make_float2(0.f, 0.f);
       else

@@ -36,11 +36,11 @@ using cgf::static_for;
 // Smaller factor first on 192, 240 and 320 points, for accuracy: which codelet
 // is next to the field decides how the rounding of the loud part of a field
 // spreads to the quiet part. Error of phasors in a quiet middle of 96x96xN (1e-6
-// of their norm, mean of two fields), larger first / smaller first: 192 18.7 /
-// 12.5, 240 18.7 / 16.1, 320 24.2 / 19.5; but 160 11.7 / 12.5, 180 17.2 / 19.2,
-// 216 11.6 / 15.0, 288 18.0 / 19.2, 384 20.3 / 21.8, 300 14.3 / 13.8. It costs
-// 160x160x192 x 8 1135 -> 1159 us a step, 192x192x320 369 -> 382 (128x128x240 137
-// -> 135).
+// of their norm, mean of three fields), larger first / smaller first: 192 16.2 /
+// 13.5, 240 18.2 / 16.5, 320 24.0 / 20.5; within a tenth elsewhere: 160 12.0 / 12.3,
+// 180 14.3 / 13.7, 216 13.5 / 13.1, 288 18.1 / 17.3, 300 16.2 / 18.0, 360 22.6 /
+// 21.1, 384 21.2 / 22.9. It costs 160x160x192 x 8 1141 -> 1160 us a step,
+// 192x192x320 370 -> 383 (128x128x240 137 -> 135).
 template <int N>
 struct ZSplit {
   using P = cgf::PSplit<N>;
